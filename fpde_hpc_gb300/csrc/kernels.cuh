@@ -92,8 +92,18 @@ struct RichLineArgs {
     double lam = 0, lamR = 0, E = 0, ksat = 0;
     int kform = 1, N = 0, rkind = 0;
     double gN = 0, dLN = 0;              // right end: Dirichlet value, or the flux and last step
+    double *last = nullptr;              // the state before the step (N+1), advanced with U
+    double *Drow = nullptr;              // increment row of the step, `pitch` values
+    float2 *Drowf = nullptr;             // the same as float pairs (split history), may be null
+    int64_t pitch = 0;
+    double *slots = nullptr;             // exchange slots, rich_slot_count(N) values of all-bits-set
+    unsigned long long *seq = nullptr;   // launch sequence counter
+    unsigned *flags = nullptr;
 };
-int launch_rich_line_step(cudaStream_t st, const RichLineArgs &a);
+// Exchange slots of the one-launch step for a line of N intervals (0: the line is too long for it).
+size_t rich_slot_count(int N);
+// U <- the step's new state, last likewise, Drow (and Drowf) <- the increment; *nk += launches.
+int launch_rich_line_step(cudaStream_t st, const RichLineArgs &a, int64_t *nk);
 
 }  // namespace fpde
 

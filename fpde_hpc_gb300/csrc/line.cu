@@ -1074,7 +1074,7 @@ struct fpde_line {
     int rkform = 1;
     double rksat = 0.0;
     double *rZ = nullptr, *rdL = nullptr, *rA = nullptr, *rB = nullptr, *rR = nullptr, *rOm = nullptr,
-           *ral = nullptr, *rbt = nullptr, *last = nullptr, *Sn = nullptr;
+           *ral = nullptr, *rbt = nullptr, *last = nullptr, *Sn = nullptr, *rslots = nullptr;
     std::vector<double> rE;
     // probes: CUDA events around kernels inside the captured graph
     struct Probe { int kind; int64_t n; double bytes, flops; int ev; int steps; };
@@ -1211,7 +1211,8 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     do { if (ev) FPDE_CUDA(record_probe_event((ev)[i], st)); } while (0)
 
 // One Richards step (rich_line.cu): coefficients from the current state, then the solve.
-static int rich_step(fpde_line *L, cudaStream_t st, int64_t n, const double *part, int KS)
+static int rich_step(fpde_line *L, cudaStream_t st, int64_t n, const double *part, int KS, double *Drow, float2 *Drowf,
+                     int64_t *nk)
 {
     RichLineArgs a;
     a.U = L->U; a.Z = L->rZ; a.dL = L->rdL;
@@ -1221,7 +1222,9 @@ static int rich_step(fpde_line *L, cudaStream_t st, int64_t n, const double *par
     a.lam = L->lam; a.lamR = L->lamR; a.ksat = L->rksat; a.kform = L->rkform;
     a.E = L->rE[(size_t)std::min<int64_t>(n, (int64_t)L->rE.size() - 1)];
     a.N = (int)L->N; a.rkind = L->d.right_kind; a.gN = L->d.right_value; a.dLN = L->d.dLN;
-    return launch_rich_line_step(st, a);
+    a.last = L->last; a.Drow = Drow; a.Drowf = Drowf; a.pitch = L->P;
+    a.slots = L->rslots; a.seq = L->seq; a.flags = L->ctx->d_flags;
+    return launch_rich_line_step(st, a, nk);
 }
 
 // Enqueue steps [n0, n0+steps) on st; returns the number of kernels enqueued via *nk.
@@ -1251,9 +1254,8 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
             ev = probe_step ? probe_begin(L, 2, n, 0.0, 0.0) : nullptr;
             PROBE_REC(ev, 0);
             if (L->rich) {                             // coefficients from the solution, then the increment
-                if ((rc = rich_step(L, st, n, L->part, KS))) return rc;
-                if ((rc = launch_append(st, L->U, L->last, L->D + n * L->P, L->N + 1, L->P))) return rc;
-                k += 2;
+                if ((rc = rich_step(L, st, n, L->part, KS, L->D + n * L->P, nullptr, &k))) return rc;
+                --k;                                   // counted below
             } else if ((rc = line_launch_solve(L, st, n, L->part, KS, L->P, L->D + n * L->P, 1))) {
                 return rc;
             }
@@ -1355,11 +1357,9 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
                         KSn = 1;
                         ++k;
                     }
-                    if ((rc = rich_step(L, st, m, L->Sn, KSn))) return rc;
-                    if ((rc = launch_append_ff(st, L->U, L->last, L->ring + (int64_t)q * L->P,
-                                               L->ringf + (int64_t)q * L->P, L->N + 1, L->P)))
+                    if ((rc = rich_step(L, st, m, L->Sn, KSn, L->ring + (int64_t)q * L->P,
+                                        L->ringf + (int64_t)q * L->P, &k)))
                         return rc;
-                    k += 3;
                 }
                 n += nst - 1;
                 continue;
@@ -1431,7 +1431,8 @@ int fpde_line_destroy(fpde_line *L)
     dev_free(L->slots);
     dev_free(L->exps);
     dev_free(L->barrier);
-    for (double *p : {L->rZ, L->rdL, L->rA, L->rB, L->rR, L->rOm, L->ral, L->rbt, L->last, L->Sn}) dev_free(p);
+    for (double *p : {L->rZ, L->rdL, L->rA, L->rB, L->rR, L->rOm, L->ral, L->rbt, L->last, L->Sn, L->rslots})
+        dev_free(p);
     delete L;
     return FPDE_OK;
 }
@@ -1947,7 +1948,9 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
         L->rksat = rich->k_sat;
         L->rE.assign(rich->evaporation, rich->evaporation + std::min(rich->evaporation_rows, d.max_steps));
         const size_t nb1 = (size_t)(N + 1) * sizeof(double);
+        const size_t nslots = rich_slot_count((int)N);
         bool f2 = dev_alloc((void **)&L->rZ, nb1) || dev_alloc((void **)&L->rdL, nb1) ||
+                  (nslots && dev_alloc((void **)&L->rslots, nslots * sizeof(double))) ||
                   dev_alloc((void **)&L->rA, nb1) || dev_alloc((void **)&L->rB, nb1) ||
                   dev_alloc((void **)&L->rR, nb1) || dev_alloc((void **)&L->rOm, nb1) ||
                   dev_alloc((void **)&L->ral, nb1 + sizeof(double)) || dev_alloc((void **)&L->rbt, nb1 + sizeof(double)) ||
@@ -1960,6 +1963,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
         }
         cudaMemcpyAsync(L->rZ, rich->sZ, nb1, cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(L->rdL, rich->dL[0], nb1, cudaMemcpyHostToDevice, st);
+        if (nslots) cudaMemsetAsync(L->rslots, 0xFF, nslots * sizeof(double), st);
         cudaMemsetAsync(L->last, 0, L->P * sizeof(double), st);
         cudaMemcpyAsync(L->last, u0, nb1, cudaMemcpyHostToDevice, st);
     }
