@@ -16,8 +16,10 @@
 // Each pass is a Thomas solve per line with R = Rlap + lam (A_/B/R :3095-3142). For a
 // uniform step the alpha recurrence Al[p+1] = B/(R - A Al[p]) is time-invariant, so it is
 // evaluated once on the host in the reference's order; a pass then needs two first-order
-// recurrences per line (forward y, backward U), swept by four lanes per line in segments
-// (k_lod_pass_seg) or, for lines over 128 interior nodes, by one thread (k_lod_pass).
+// recurrences per line (forward y, backward U), swept by one thread per line with the line's data
+// staged in shared memory (k_lod_pass_st); lines too long for that, or with a requested segment
+// count, by several lanes per line in segments (k_lod_pass_seg), over 512 interior nodes by one
+// thread from global memory (k_lod_pass).
 //
 // HBM layout: the state and every grid input keep the reference's index
 // idx = i + j (sN+2) + k (sN+2)(M+2) (:1181). The per-pass line coefficients (A, g =
@@ -39,6 +41,7 @@
 #include "richards.cuh"
 #include "tc_far.cuh"
 #include "ff.cuh"
+#include "scan.cuh"
 
 namespace fpde {
 
@@ -134,6 +137,349 @@ __global__ void __launch_bounds__(128) k_lod_pass(LodPassArgs p)
         }
     }
     p.U[base] = fma(__ldg(p.al + line), u, g0);                   // Al[1] U[1] + Bt[1]
+}
+
+// Staged pass: one thread per line, 32 lines (a tile) per CTA of four warps. The chain warp runs the two
+// recurrences of its lines and nothing else. The producer warp streams the tile's coefficients into
+// shared memory by bulk copies: they are stored group by group (GN nodes x 32 lines), S groups in a
+// ring, asked into L2 PD groups ahead. Two helper warps take every second group: they load the state
+// (and the K pass's history partials and source) two groups ahead, form the right-hand sides and, on
+// the way back, store the new state. The forward results of the whole line stay in shared memory.
+// A node costs 3 coefficients (gA, g, al) and one state update instead of the segmented pass's 5
+// coefficients (KF, CB), and 3 FP64 operations (K pass 4) instead of 7.
+// What bounds it: a warp gets one FP64 operation per ~68 cycles from its SM quarter, dependent or not,
+// and the SM one per ~19.5. At 128^3 (3.3 tiles per SM) that is 127 nodes x 3 operations x 3.3 x 19.5
+// cycles = 13 us per pass (K pass 17 us), next to 40 bytes per node (13 us at the measured copy
+// rate). Everything that shared the chain's warp held its operations back: forms with one and two
+// warps per tile took 33-37 us per pass with the FP64 pipe 31-35 % busy. Measured at 128^3, per pass:
+// K 32, _M 26, sN 29 us (segmented 66 us each); 61 x 47 x 90: 19, 11, 12 us (25 us each).
+// The sN pass (TRANS) walks along the contiguous axis: a helper's consecutive loads share sectors
+// through L1, and its results go out 4 nodes x 8 lines per store instruction.
+constexpr int GN = 8;                     // nodes per group
+constexpr int ST_KS_MAX = 2;              // history partial rows of a staged K pass
+constexpr int ST_PD = 8;                  // groups asked into L2 ahead of their copy
+
+__device__ __forceinline__ uint32_t st_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool st_try_wait(uint64_t *bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(ok) : "r"(st_smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void st_arrive(uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(st_smem_u32(bar)) : "memory");
+}
+// Bounded wait (2 s); after a timeout (flagged) no wait of this thread waits again.
+__device__ __forceinline__ void st_wait(uint64_t *bar, uint32_t parity, bool &ok, unsigned *flags)
+{
+    if (!ok || st_try_wait(bar, parity)) return;
+    const unsigned long long t0 = gtimer_ns();
+    while (!st_try_wait(bar, parity))
+        if (gtimer_ns() - t0 > 2000000000ull) { ok = false; atomicOr(flags, DEVERR_MBAR_TIMEOUT); return; }
+}
+
+struct LodStageArgs {
+    const double *AG;                     // [tiles][F][2][GN][32]: gA and g (passes without source: g lam)
+    const double *al;                     // [tiles][F][GN][32]
+    unsigned *flags;
+    int wave;                             // CTAs of one resident round over the SMs (role placement)
+};
+
+template <bool TRANS, bool KP, int S>
+__global__ void __launch_bounds__(128, 4) k_lod_pass_st(LodPassArgs p, LodStageArgs sa)
+{
+    extern __shared__ __align__(128) double st_smem[];
+    // full: a group's coefficients have landed; ready: its right-hand sides are in sh; used: the chain
+    // has read the group
+    __shared__ uint64_t full[S], used[S], ready[2];
+    __shared__ int s_done;                              // backward groups whose results are in yb
+    constexpr int YP = TRANS ? 33 : 32;                 // pitch of a node's 32 forward results
+    constexpr int GD = GN * 32;                         // doubles of one array of a group
+    const int lane = threadIdx.x & 31, tile = blockIdx.x, line = tile * 32 + lane;
+    // warp w of a CTA runs on SM quarter w: the roles rotate with the resident CTA, so that an SM's
+    // chains run on different quarters
+    const int role = ((int)(threadIdx.x >> 5) + tile / sa.wave) & 3;      // 0 chain, 1 2 helpers, 3 producer
+    const bool live = line < p.lines;
+    const int ln = live ? line : p.lines - 1;           // idle lanes read the last line and store nothing
+    const int a = ln % p.n1, b = ln / p.n1;
+    const int64_t base = (int64_t)(1 + a) * p.s1 + (int64_t)(1 + b) * p.s2;
+    const int Nl = p.Nl, F = (Nl - 1 + GN - 1) / GN;
+    double *stages = st_smem;                           // [S][2][GN][32]
+    double *sh = st_smem + S * 2 * GD;                  // [2][GN][32]
+    double *yb = sh + 2 * GD;                           // [F GN][YP], row q - 1
+    const double *AL = sa.al + (size_t)tile * F * GD;
+    if (threadIdx.x == 0) {
+        auto init = [](uint64_t *bar) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(st_smem_u32(bar)) : "memory");
+        };
+#pragma unroll
+        for (int s = 0; s < S; ++s) { init(&full[s]); init(&used[s]); }
+        init(&ready[0]);
+        init(&ready[1]);
+        s_done = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    bool ok = true;
+    auto wait_used = [&](int gi) { st_wait(&used[gi % S], (uint32_t)(gi / S) & 1u, ok, sa.flags); };
+    auto wait_full = [&](int gi) { st_wait(&full[gi % S], (uint32_t)(gi / S) & 1u, ok, sa.flags); };
+    // group gi: 0 .. F-1 the forward nodes in order, F .. 2F-1 the backward ones from the far end.
+    // Nodes past the line's end have gA = al = 1, g = 0 and no effect.
+
+    if (role == 3) {                                    // ---- producer
+        if (lane != 0) return;
+        const double *AG = sa.AG + (size_t)tile * F * 2 * GD;
+        auto source = [&](int gi) { return gi < F ? AG + (size_t)gi * 2 * GD : AL + (size_t)(2 * F - 1 - gi) * GD; };
+        auto prefetch = [&](int gi) {
+            if (gi < 2 * F)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(source(gi)),
+                             "r"(gi < F ? 2 * GD * 8 : GD * 8)
+                             : "memory");
+        };
+        for (int gi = 0; gi < 2 * F; ++gi) {
+            if (gi >= S) wait_used(gi - S);
+            const uint32_t bar = st_smem_u32(&full[gi % S]), bytes = gi < F ? 2 * GD * 8 : GD * 8;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             st_smem_u32(stages + (gi % S) * 2 * GD)),
+                         "l"(source(gi)), "r"(bytes), "r"(bar)
+                         : "memory");
+            if (gi == 0)
+                for (int k = S; k < ST_PD; ++k) prefetch(k);
+            prefetch(gi + ST_PD);
+        }
+        for (int gi = max(0, 2 * F - S); gi < 2 * F; ++gi) wait_full(gi);     // own copies in flight
+        return;
+    }
+
+    if (role != 0) {                                    // ---- helpers: groups x, x + 2, ...
+        const int x = role - 1;
+        const double *ptr[4] = {p.U + base + p.st * (1 + x * GN), nullptr, nullptr, nullptr};   // state, partials, source
+        if (KP) {
+            if (p.KS > 0) ptr[1] = p.part + base + p.st * (1 + x * GN);
+            if (p.KS > 1) ptr[2] = ptr[1] + p.pstride;
+            if (p.rp) ptr[3] = p.rp + base + p.st * (1 + x * GN);
+        }
+        double v[KP ? 4 : 1][GN];
+        auto fetch = [&](int gi) {
+            if (gi >= F) return;
+            const bool whole = gi * GN + GN < Nl;
+#pragma unroll
+            for (int k = 0; k < (KP ? 4 : 1); ++k) {
+                const double *q = ptr[k];
+#pragma unroll
+                for (int t = 0; t < GN; ++t) {
+                    v[k][t] = 0.0;
+                    if (q && (whole || gi * GN + t + 1 < Nl)) v[k][t] = (TRANS && k == 0) ? q[t] : __ldcg(q + t * p.st);
+                }
+                if (q) ptr[k] = q + 2 * GN * p.st;
+            }
+        };
+        fetch(x);
+        for (int gi = x; gi < F; gi += 2) {
+            if (gi >= 2) wait_used(gi - 2);             // this half of sh is free
+            wait_full(gi);
+            const double *sg = stages + (gi % S) * 2 * GD + GD + lane;
+            double *ho = sh + x * GD + lane;
+#pragma unroll
+            for (int t = 0; t < GN; ++t) {
+                double mo = v[0][t];
+                if (KP) {                               // -Om = lam U - Rp - S (Om1 :4191, :4267)
+                    double s = v[KP ? 1 : 0][t];
+                    if (p.KS > 1) s += v[KP ? 2 : 0][t];
+                    if (p.rp) s += v[KP ? 3 : 0][t];
+                    mo = fma(p.lam, mo, -s);
+                }
+                v[0][t] = sg[t * 32] * mo;
+            }
+#pragma unroll
+            for (int t = 0; t < GN; ++t) ho[t * 32] = v[0][t];
+            __syncwarp();
+            if (lane == 0) st_arrive(&ready[x]);
+            fetch(gi + 2);
+        }
+        int64_t ob[TRANS ? 4 : 1];                      // sN pass: the lines this lane stores nodes of
+        if (TRANS) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) ob[r] = __shfl_sync(0xffffffffu, base, (lane >> 2) + 8 * r);
+        }
+        for (int gi = F + ((F + x) & 1); gi < 2 * F; gi += 2) {     // backward: gi of this helper's parity
+            const unsigned long long t0 = gtimer_ns();
+            while (ok) {
+                int d;
+                asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(d) : "r"(st_smem_u32(&s_done)) : "memory");
+                if (d > gi - F) break;
+                if (gtimer_ns() - t0 > 2000000000ull) { ok = false; atomicOr(sa.flags, DEVERR_MBAR_TIMEOUT); }
+            }
+            const int q0 = 1 + (2 * F - 1 - gi) * GN;
+            if (TRANS) {
+#pragma unroll
+                for (int hf = 0; hf < GN / 4; ++hf) {
+                    const int q = q0 + 4 * hf + (lane & 3);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const int ol = (lane >> 2) + 8 * r;
+                        if (q < Nl && tile * 32 + ol < p.lines) p.U[ob[r] + q] = yb[(q - 1) * YP + ol];
+                    }
+                }
+            } else if (live) {
+                double *o = p.U + base + (int64_t)q0 * p.st;
+#pragma unroll
+                for (int t = 0; t < GN; ++t)
+                    if (q0 + t < Nl) o[t * p.st] = yb[(q0 + t - 1) * YP + lane];
+            }
+        }
+        return;
+    }
+
+    // ---- chain warp. A group's operands are read while the group before it is half done, and its
+    // results are stored once they are complete: a store or load that waits holds the chain back.
+    const double g0 = p.bc ? p.bc[base] : 0.0;
+    const double gN = p.bc ? p.bc[base + (int64_t)Nl * p.st] : 0.0;
+    const bool flux = p.rkind != FPDE_BC_DIRICHLET;
+    const double AlN = flux ? __ldg(AL + (size_t)((Nl - 2) / GN) * GD + ((Nl - 2) % GN) * 32 + lane) : 0.0;
+    const double uold_last = flux ? p.U[base + (int64_t)(Nl - 1) * p.st] : 0.0;   // before any write
+    auto read_f = [&](int gi, double (&A)[GN], double (&H)[GN]) {
+        st_wait(&ready[gi & 1], (uint32_t)(gi >> 1) & 1u, ok, sa.flags);     // implies full
+        const double *sg = stages + (gi % S) * 2 * GD + lane, *hi = sh + (gi & 1) * GD + lane;
+#pragma unroll
+        for (int t = 0; t < GN; ++t) { A[t] = sg[t * 32]; H[t] = hi[t * 32]; }
+    };
+    // Give a group's buffers back. Its operands must be in registers by then: loads that are still
+    // queued behind the helpers' traffic would meet the next bulk copy (seen in the K and sN passes),
+    // so the warp votes on a value formed from all of them.
+    auto release = [&](int gi, const double (&A)[GN], const double (&H)[GN]) {
+        unsigned z = 0;
+#pragma unroll
+        for (int t = 0; t < GN; ++t) z ^= (unsigned)(__double2loint(A[t]) ^ __double2loint(H[t]));
+        asm volatile("{\n\t.reg .pred p, q;\n\t"
+                     "setp.eq.u32 p, %0, 1;\n\t"
+                     "vote.sync.any.pred q, p, 0xffffffff;\n\t}\n" ::"r"(z) : "memory");
+        if (lane == 0) st_arrive(&used[gi % S]);
+    };
+    // forward: y_q = Bt[q+1] = gA y_{q-1} + g (-Om), y_0 = Bt[1] = g0
+    double y = g0, A0[GN], H0[GN], A1[GN], H1[GN], R[GN / 2];
+    auto step_f = [&](int gi, double (&A)[GN], double (&H)[GN], double (&An)[GN], double (&Hn)[GN]) {
+        double *yo = yb + gi * GD * YP / 32 + lane;
+#pragma unroll
+        for (int t = 0; t < GN / 2; ++t) { y = fma(A[t], y, H[t]); H[t] = y; }
+        if (gi + 1 < F) read_f(gi + 1, An, Hn);
+        if (gi > 0) {
+#pragma unroll
+            for (int t = 0; t < GN / 2; ++t) yo[(t - GN / 2) * YP] = R[t];        // the last half of group gi - 1
+        }
+#pragma unroll
+        for (int t = GN / 2; t < GN; ++t) { y = fma(A[t], y, H[t]); R[t - GN / 2] = y; }
+#pragma unroll
+        for (int t = 0; t < GN / 2; ++t) yo[t * YP] = H[t];
+        if (gi + 1 < F) release(gi + 1, An, Hn);
+    };
+    read_f(0, A0, H0);
+    release(0, A0, H0);
+    for (int gi = 0; gi < F; gi += 2) {
+        step_f(gi, A0, H0, A1, H1);
+        if (gi + 1 < F) step_f(gi + 1, A1, H1, A0, H0);
+    }
+    {
+        double *yo = yb + (size_t)(F - 1) * GN * YP + lane;
+#pragma unroll
+        for (int t = 0; t < GN; ++t)
+            if ((F - 1) * GN + t + 1 >= Nl) yo[t * YP] = 0.0;                    // past the line's end
+            else if (t >= GN / 2) yo[t * YP] = R[t >= GN / 2 ? t - GN / 2 : 0];
+    }
+    // right end: Dirichlet value or the flux closure of U1 (:4687-4719) with the old U[Nl-1]
+    double uN;
+    if (!flux) {
+        uN = gN;
+    } else {
+        if (fabs(y) > 1e-15) uN = (fabs(1.0 - AlN) > 1e-15) ? (y + gN * p.dLN) / (1.0 - AlN) : uold_last;
+        else uN = (fabs(1.0 - AlN) > 1e-15) ? 0.0 : uold_last;
+    }
+    double *Uo = p.U + base;
+    if (live) {
+        Uo[(int64_t)Nl * p.st] = uN;
+        Uo[(int64_t)(Nl + 1) * p.st] = uN;              // ghost copy (U1 :4792)
+    }
+    // backward: U_q = al_q U_{q+1} + y_q
+    double u = uN;
+    auto read_b = [&](int gi, double (&A)[GN], double (&H)[GN]) {
+        wait_full(gi);
+        const double *sg = stages + (gi % S) * 2 * GD + lane, *yo = yb + (size_t)(2 * F - 1 - gi) * GN * YP + lane;
+#pragma unroll
+        for (int t = 0; t < GN; ++t) { A[t] = sg[t * 32]; H[t] = yo[t * YP]; }
+    };
+    auto announce = [&](int n) {                        // n backward groups are complete in yb
+        __syncwarp();
+        if (lane == 0)
+            asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(st_smem_u32(&s_done)), "r"(n) : "memory");
+    };
+    auto step_b = [&](int gi, double (&A)[GN], double (&H)[GN], double (&An)[GN], double (&Hn)[GN]) {
+        double *yo = yb + (size_t)(2 * F - 1 - gi) * GN * YP + lane;
+#pragma unroll
+        for (int t = GN - 1; t >= GN / 2; --t) { u = fma(A[t], u, H[t]); H[t] = u; }
+        if (gi + 1 < 2 * F) read_b(gi + 1, An, Hn);
+        if (gi > F) {
+#pragma unroll
+            for (int t = 0; t < GN / 2; ++t) yo[(t + GN) * YP] = R[t];            // the last half of group gi - 1
+        }
+#pragma unroll
+        for (int t = GN / 2 - 1; t >= 0; --t) { u = fma(A[t], u, H[t]); R[t] = u; }
+#pragma unroll
+        for (int t = GN / 2; t < GN; ++t) yo[t * YP] = H[t];
+        if (gi + 1 < 2 * F) release(gi + 1, An, Hn);
+        if (gi > F) announce(gi - F);
+    };
+    read_b(F, A0, H0);
+    release(F, A0, H0);
+    for (int gi = F; gi < 2 * F; gi += 2) {
+        step_b(gi, A0, H0, A1, H1);
+        if (gi + 1 < 2 * F) step_b(gi + 1, A1, H1, A0, H0);
+    }
+#pragma unroll
+    for (int t = 0; t < GN / 2; ++t) yb[t * YP + lane] = R[t];
+    announce(F);
+    if (live) Uo[0] = p.lkind == FPDE_BC_FLUX ? u + g0 : g0;      // Al[1] U[1] + Bt[1], Al[1] = 1 or 0
+}
+
+// Dynamic shared memory of a staged pass.
+static size_t st_smem_bytes(int Nl, bool trans, int S)
+{
+    return ((size_t)(S + 1) * 2 * GN * 32 + (size_t)((Nl - 1 + GN - 1) / GN * GN) * (trans ? 33 : 32)) * sizeof(double);
+}
+constexpr size_t ST_SMEM_MAX = 226 * 1024;
+
+template <int S>
+static cudaError_t st_attrs()
+{
+    cudaError_t e = smem_opt_in((const void *)k_lod_pass_st<false, true, S>, (int)ST_SMEM_MAX);
+    if (e == cudaSuccess) e = smem_opt_in((const void *)k_lod_pass_st<false, false, S>, (int)ST_SMEM_MAX);
+    if (e == cudaSuccess) e = smem_opt_in((const void *)k_lod_pass_st<true, false, S>, (int)ST_SMEM_MAX);
+    return e;
+}
+template <int S>
+static void st_launch(cudaStream_t st, const LodPassArgs &a, const LodStageArgs &sa, int pass)
+{
+    const unsigned blocks = (unsigned)((a.lines + 31) / 32);
+    const size_t smem = st_smem_bytes(a.Nl, pass == 0, S);
+    if (pass == 2) k_lod_pass_st<false, true, S><<<blocks, 128, smem, st>>>(a, sa);
+    else if (pass == 1) k_lod_pass_st<false, false, S><<<blocks, 128, smem, st>>>(a, sa);
+    else k_lod_pass_st<true, false, S><<<blocks, 128, smem, st>>>(a, sa);
+}
+// Groups in the ring: 8 where all of the pass's warps still fit at once (a second wave would repeat
+// the whole recurrence), else 4. 0 where fewer than two of several warps fit on an SM (lines over
+// about 380 intervals): the segmented pass is then no slower.
+static int st_depth(int Nl, int lines, bool trans)
+{
+    const int per_sm = ((lines + 31) / 32 + device_sm_count() - 1) / device_sm_count();
+    for (int S : {8, 4}) {
+        const size_t need = st_smem_bytes(Nl, trans, S) + 1024 + 16 * S + 32;
+        if (need <= ST_SMEM_MAX && need * (S == 4 ? std::min(per_sm, 2) : per_sm) <= 228 * 1024) return S;
+    }
+    return 0;
 }
 
 // Variable steps (the reference's varT): the local term Da kkk0_n / tau_n of R changes every step,
@@ -660,6 +1006,7 @@ struct fpde_lod3d {
     int segs[3] = {0, 0, 0};
     int segcap[3] = {0, 0, 0};                     // the pass kernel's segment capacity (SEGLEN)
     int lines[3] = {0, 0, 0};
+    int sdepth[3] = {0, 0, 0};                     // staged passes (k_lod_pass_st): groups in flight, or 0
     // split path (exact three-slice far history on the tensor cores, FP64 near history)
     bool split = false;
     int64_t rows16 = 0, ld16 = 0, ldp = 0;
@@ -774,6 +1121,12 @@ static int lod_launch_pass(fpde_lod3d *L, cudaStream_t st, int pass, int64_t n, 
             r.nu = L->snu; r.sigma = L->ssig; r.Dc = L->sDc;
         }
         k_lod_pass_rich<<<(unsigned)((a.lines + 127) / 128), 128, 0, st>>>(a, r);
+    } else if (L->sdepth[pass] > 0) {
+        LodStageArgs sa;
+        sa.AG = L->cA[pass]; sa.al = L->cal[pass]; sa.flags = L->ctx->d_flags;
+        sa.wave = device_sm_count();
+        if (L->sdepth[pass] == 8) st_launch<8>(st, a, sa, pass);
+        else st_launch<4>(st, a, sa, pass);
     } else if (L->seglen[pass] > 0) {
         LodSegArgs sg;
         sg.KF = L->cKF[pass]; sg.CB = L->cCB[pass]; sg.PF = L->cPF[pass]; sg.seglen = L->seglen[pass];
@@ -900,6 +1253,7 @@ static int lod_enqueue(fpde_lod3d *L, cudaStream_t st, int64_t n0, int steps, in
             const int64_t t0 = n > L->max_lag ? n - L->max_lag : 0;    // oldest row of the window
             if (n - t0 >= 1) {
                 KS = choose_splits((int)(n - t0), L->P);
+                if (L->sdepth[2] > 0) KS = std::min(KS, ST_KS_MAX);
                 const double *wt = L->vart ? L->wrows + n * L->wld     // variable steps: row n
                                            : L->wrev + (L->max_steps - n);     // wt[t] = w[n - t]
                 if ((rc = launch_l1_partial(st, L->D + t0 * L->P, L->P, (int)(n - t0), wt + t0, L->part, KS)))
@@ -1337,12 +1691,53 @@ int fpde_lod3d_create(fpde_ctx *ctx, const fpde_lod3d_desc *desc, const double *
     }
     // per-pass line coefficients, evaluated in the reference's order (al1 :4002-4027)
     std::vector<double> hA, hg, hal;
+    if (!fail && !rich && !sfd && !vart) {
+        fail = st_attrs<4>() != cudaSuccess || st_attrs<8>() != cudaSuccess;
+        if (fail) set_error(FPDE_ERR_CUDA, "lod3d: shared memory attributes");
+    }
     for (int pass = 0; pass < 3 && !fail && !rich && !sfd && !vart; ++pass) {
         int Nl, n1, n2;
         int64_t s1, s2, stp;
         pass_geometry(L, pass, &Nl, &n1, &n2, &s1, &s2, &stp);
         const int lines = n1 * n2;
         L->lines[pass] = lines;
+        // staged unless segments are asked for or the line is too long for it
+        if (d.segments[pass] == 0 && lines > 0) L->sdepth[pass] = st_depth(Nl, lines, pass == 0);
+        if (L->sdepth[pass] > 0) {
+            // tile-major: [tile][group][gA, g][GN][32] and [tile][group][GN][32]; g lam where the
+            // right-hand side is -lam U alone
+            const int F = (Nl - 1 + GN - 1) / GN, tiles = (lines + 31) / 32;
+            const double gscale = pass == 2 ? 1.0 : L->lam;
+            const double *cA = coefA + (int64_t)pass * L->G, *cB = coefB + (int64_t)pass * L->G,
+                         *cR = coefRlap + (int64_t)pass * L->G;
+            hA.assign((size_t)tiles * F * 2 * GN * 32, 0.0);      // padding: gA = al = 1, g = 0
+            hal.assign((size_t)tiles * F * GN * 32, 1.0);
+            for (size_t o = 0; o < hA.size(); ++o)
+                if (o / (GN * 32) % 2 == 0) hA[o] = 1.0;
+            for (int line = 0; line < lines; ++line) {
+                const int64_t base = (int64_t)(1 + line % n1) * s1 + (int64_t)(1 + line / n1) * s2;
+                const size_t at = (size_t)(line / 32) * F * GN * 32 + line % 32;
+                double Al = d.left_kind[pass] == FPDE_BC_FLUX ? 1.0 : 0.0;        // Al[1]
+                for (int q = 1; q < Nl; ++q) {
+                    const int64_t id = base + (int64_t)q * stp;
+                    const double R = cR[id] + L->lamR, Aq = cA[id], Bq = cB[id];
+                    Al = Bq / (R - Aq * Al);                                       // Al[q+1]
+                    const size_t o = at + (size_t)(q - 1) * 32;
+                    const size_t oa = 2 * at - line % 32 + (size_t)((q - 1) / GN) * 2 * GN * 32 + (size_t)((q - 1) % GN) * 32;
+                    hA[oa] = (Al / Bq) * Aq;
+                    hA[oa + GN * 32] = gscale * (Al / Bq);
+                    hal[o] = Al;
+                }
+            }
+            fail = dev_alloc((void **)&L->cA[pass], hA.size() * sizeof(double)) ||
+                   dev_alloc((void **)&L->cal[pass], hal.size() * sizeof(double));
+            if (!fail) {
+                fail = cudaMemcpy(L->cA[pass], hA.data(), hA.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
+                       cudaMemcpy(L->cal[pass], hal.data(), hal.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess;
+                if (fail) set_error(FPDE_ERR_CUDA, "lod3d: coefficient upload failed");
+            }
+            continue;
+        }
         const size_t cnt = (size_t)(Nl + 1) * lines;
         hA.assign(cnt, 0.0);
         hg.assign(cnt, 0.0);
