@@ -248,6 +248,8 @@ class LineWorkload:
         if self.do:
             return fp.autotune_line(ctx, p.N, 0.5, p.tau, 1.0, A, B, R, p.u0, p.steps, precision=prec,
                                     lag_weights=self.weights(p.steps + 1), theta=1.0)
+        if prec == fp.FPDE_PREC_FP64:       # the plain method (a GEMV per step), not the 64-step blocks
+            return fp.LineTuning(gemv_splits=32)
         return fp.autotune_line(ctx, p.N, p.alpha, p.tau, p.Da, A, B, R, p.u0, p.steps, precision=prec)
 
     @property

@@ -1,7 +1,11 @@
 // 1D line problem (fpde_line_*): the plain FP64 path and the split-precision path.
 //
 // Per time step n (fpde_hpc_1d.cpp calc_step / U1 with the history applied every step):
-//   FP64 path (one launch each per step)
+//   FP64 path, blocks of 64 steps (the rule; lines without requested launch parameters)
+//     at n0:  k_far64: the history t < n0 of the block's 64 steps in one FP64 product
+//     steps of the block: k_line_block_spec as on the split path, its near history in FP64 too
+//   FP64 path, one launch each per step (requested launch parameters, lines of over 1,024 nodes
+//   per SM)
 //     1. k_l1_partial : part[ks][i] = sum_t w[n-t] D_t[i]        (FP64 history GEMV)
 //     2. k_line_solve : S = sum_ks part, Om = -lam U + src + S, Thomas solve, U <- U^{n+1},
 //                       D_n = U^{n+1} - U^n
@@ -32,6 +36,7 @@
 #include <vector>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <algorithm>
 
 #include "common.cuh"
@@ -373,6 +378,10 @@ struct LineBlockArgs {
     // speculative kernel with an explicit part: the pre-scaled weights g theta A (on ub at i-1,
     // i > a) and g theta B (on ub at i+1, i < b-1) of the chunk's own zero-carry backward result
     const double *xa, *xb;
+    // FP64 path: a launch that ends inside a block leaves what the next one (j0 > 0) needs to go on
+    // exactly as one launch would: per node the last step's zero-carry backward result and the state
+    // before it, per chunk that step's carries and the right end's values (c_in, u_b, U_N, old U_N)
+    double *cub, *cu, *ccar;
     unsigned *flags;
     double lam, g0, gN, dLN, AlN;
     int64_t n0;                           // global index of step j0
@@ -396,14 +405,54 @@ __device__ __forceinline__ void st_relaxed_f64(double *p, double v)
 
 __device__ __forceinline__ void solver_sync() { asm volatile("bar.sync 1, %0;" ::"n"(LTS) : "memory"); }
 
-// history warps of the block solves: S[node] = far partials of step j + sum_{r < rmax} w[j - r]
-// D_r[node], in float-float arithmetic on the FP32 pipe (one FP64 add per node at the end), from
-// the float-pair copy of the ring and float-pair weights. GB300 issues 2 DFMA/clk/SM, so the FP64 form of these sums (up to 63 rows a step)
-// occupied the FP64 pipe the solver's recurrences wait on.
-// (ah, al) += far partials of steps j .. j+NJ-1 (NJ accumulators; every load issued first).
-template <int SP, int NJ>
-__device__ __forceinline__ void far_fold_ff(const LineBlockArgs &p, int ht, int a, int b, int j, float (&ah)[NJ][SP],
-                                            float (&al)[NJ][SP])
+// History warps of the block solves: S[node] = far partials of step j + sum_{r < rmax} w[j - r]
+// D_r[node]. NearFF (split path): in float-float on the FP32 pipe (one FP64 add per node at the end),
+// from the float-pair copy of the ring and float-pair weights: GB300 issues 2 DFMA/clk/SM, so the
+// FP64 form of these sums (up to 63 rows a step) occupies the FP64 pipe that the solver's recurrences
+// wait on. Near64 (FP64 path): plain FP64 multiply-adds from the FP64 rows.
+struct NearFF {
+    using Row = float2;                                  // an increment in the row rings
+    using W = float2;
+    float h = 0.f, l = 0.f;
+    static __device__ __forceinline__ Row row(double d) { return d2ff(d); }
+    static __device__ __forceinline__ Row zero() { return make_float2(0.f, 0.f); }
+    __device__ __forceinline__ void add(double slot, bool pairs)
+    {
+        const float2 f = pairs ? *reinterpret_cast<const float2 *>(&slot) : d2ff(slot);
+        ff_add(h, l, f.x, f.y);
+    }
+    __device__ __forceinline__ void mac(W w, Row d) { ff_fma(h, l, w, d); }
+    __device__ __forceinline__ void renorm() { ff_renorm(h, l); }
+    __device__ __forceinline__ double scaled(W s) const  // (h + l) s: float-float, one FP64 add
+    {
+        const float ph = __fmul_rn(h, s.x);
+        float pe = __fmaf_rn(h, s.x, -ph);
+        pe = __fmaf_rn(h, s.y, pe);
+        pe = __fmaf_rn(l, s.x, pe);
+        return f2d_bits(ph) + f2d_bits(pe);
+    }
+    static __device__ __forceinline__ Row *rows(const LineBlockArgs &p) { return p.ringf; }
+    static __device__ __forceinline__ const W *weights(const LineBlockArgs &p) { return p.wff; }
+    static __device__ __forceinline__ const W *scale(const LineBlockArgs &p) { return p.ngf; }
+};
+struct Near64 {
+    using Row = double;
+    using W = double;
+    double s = 0.0;
+    static __device__ __forceinline__ Row row(double d) { return d; }
+    static __device__ __forceinline__ Row zero() { return 0.0; }
+    __device__ __forceinline__ void add(double slot, bool) { s += slot; }
+    __device__ __forceinline__ void mac(W w, Row d) { s = fma(w, d, s); }
+    __device__ __forceinline__ void renorm() {}
+    __device__ __forceinline__ double scaled(W g) const { return s * g; }
+    static __device__ __forceinline__ Row *rows(const LineBlockArgs &p) { return p.ring; }
+    static __device__ __forceinline__ const W *weights(const LineBlockArgs &p) { return p.wlag; }
+    static __device__ __forceinline__ const W *scale(const LineBlockArgs &p) { return p.ng; }
+};
+
+// acc += far partials of steps j .. j+NJ-1 (NJ accumulators; every load issued first).
+template <class H, int SP, int NJ>
+__device__ __forceinline__ void far_fold(const LineBlockArgs &p, int ht, int a, int b, int j, H (&acc)[NJ][SP])
 {
     double v[NJ][FAR_MAX_SPLITS][SP];
 #pragma unroll
@@ -422,40 +471,37 @@ __device__ __forceinline__ void far_fold_ff(const LineBlockArgs &p, int ht, int 
 #pragma unroll
         for (int k = 0; k < FAR_MAX_SPLITS; ++k)
 #pragma unroll
-            for (int q = 0; q < SP; ++q) {
-                const float2 f = p.far_pairs ? *reinterpret_cast<const float2 *>(&v[m][k][q]) : d2ff(v[m][k][q]);
-                ff_add(ah[m][q], al[m][q], f.x, f.y);
-            }
+            for (int q = 0; q < SP; ++q) acc[m][q].add(v[m][k][q], p.far_pairs);
 }
 
-// (ah, al) += sum_{r < rmax} w[j - r] D_r for this thread's nodes (rows of the float-pair ring,
+// acc += sum_{r < rmax} w[j - r] D_r for this thread's nodes (rows of the row ring in global memory,
 // two batches of rows in flight).
-template <int SP>
-__device__ __forceinline__ void rows_ff(const LineBlockArgs &p, int ht, int a, int b, int j, int rmax, float *ah,
-                                        float *al)
+template <class H, int SP>
+__device__ __forceinline__ void near_rows(const LineBlockArgs &p, int ht, int a, int b, int j, int rmax, H *acc)
 {
+    using Row = typename H::Row;
     constexpr int RB = SP <= 4 ? 8 : 4;                  // rows per batch
     int64_t node[SP];
 #pragma unroll
     for (int q = 0; q < SP; ++q) node[q] = a + ht + LTS * q;
-    float2 va[RB][SP], vb[RB][SP];
-    auto load = [&](float2 (&v)[RB][SP], int r0) {
+    Row va[RB][SP], vb[RB][SP];
+    auto load = [&](Row (&v)[RB][SP], int r0) {
 #pragma unroll
         for (int u = 0; u < RB; ++u) {
-            const float2 *row = p.ringf + (int64_t)(r0 + u) * p.P;
+            const Row *row = H::rows(p) + (int64_t)(r0 + u) * p.P;
 #pragma unroll
-            for (int q = 0; q < SP; ++q) v[u][q] = node[q] < b ? row[node[q]] : make_float2(0.f, 0.f);
+            for (int q = 0; q < SP; ++q) v[u][q] = node[q] < b ? row[node[q]] : H::zero();
         }
     };
-    auto accumulate = [&](const float2 (&v)[RB][SP], int r0) {
+    auto accumulate = [&](const Row (&v)[RB][SP], int r0) {
 #pragma unroll
         for (int u = 0; u < RB; ++u) {
-            const float2 w = __ldg(p.wff + (j - r0 - u));
+            const typename H::W w = __ldg(H::weights(p) + (j - r0 - u));
 #pragma unroll
-            for (int q = 0; q < SP; ++q) ff_fma(ah[q], al[q], w, v[u][q]);
+            for (int q = 0; q < SP; ++q) acc[q].mac(w, v[u][q]);
         }
 #pragma unroll
-        for (int q = 0; q < SP; ++q) ff_renorm(ah[q], al[q]);
+        for (int q = 0; q < SP; ++q) acc[q].renorm();
     };
     int r = 0;
     if (RB <= rmax) load(va, 0);
@@ -472,34 +518,35 @@ __device__ __forceinline__ void rows_ff(const LineBlockArgs &p, int ht, int a, i
         if (!more2) break;
     }
     for (; r < rmax; ++r) {
-        const float2 w = __ldg(p.wff + (j - r));
-        const float2 *row = p.ringf + (int64_t)r * p.P;
+        const typename H::W w = __ldg(H::weights(p) + (j - r));
+        const Row *row = H::rows(p) + (int64_t)r * p.P;
 #pragma unroll
         for (int q = 0; q < SP; ++q)
-            if (node[q] < b) ff_fma(ah[q], al[q], w, row[node[q]]);
+            if (node[q] < b) acc[q].mac(w, row[node[q]]);
     }
 }
 
-// The speculative kernel keeps the block's newest NR increment rows (float pairs, this chunk's
-// nodes) in dynamic shared memory, so the per-step history sums read them from shared memory
+// The speculative kernel keeps the block's newest NR increment rows (float pairs or doubles, this
+// chunk's nodes) in dynamic shared memory, so the per-step history sums read them from shared memory
 // instead of re-reading every earlier row of the block from L2 each step; older rows come from
-// the float-pair ring in global memory.
+// the row ring in global memory.
 template <int SP>
 struct SpecRing {
     static constexpr int NR = SP <= 2 ? 64 : (SP == 4 ? 48 : 24);
-    static constexpr size_t bytes = (size_t)NR * LTS * SP * sizeof(float2);
+    static constexpr size_t bytes = (size_t)NR * LTS * SP * sizeof(double);
 };
+static_assert(sizeof(NearFF::Row) == sizeof(double) && sizeof(Near64::Row) == sizeof(double), "row ring slots");
 
-// (ah, al) += sum_{r0 <= r < r1} w[j - r] D_r from the shared-memory row ring (slot r mod NR).
-template <int SP>
-__device__ __forceinline__ void rows_smem_ff(const LineBlockArgs &p, const float2 *sR, int ht, int j, int r0, int r1,
-                                             float *ah, float *al)
+// acc += sum_{r0 <= r < r1} w[j - r] D_r from the shared-memory row ring (slot r mod NR).
+template <class H, int SP>
+__device__ __forceinline__ void near_rows_smem(const LineBlockArgs &p, const typename H::Row *sR, int ht, int j, int r0,
+                                               int r1, H *acc)
 {
     constexpr int NR = SpecRing<SP>::NR;
     int slot = r0 % NR;
     int r = r0;
     for (; r + 8 <= r1; r += 8) {
-        float2 v[8][SP];
+        typename H::Row v[8][SP];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             int sl = slot + u;
@@ -509,32 +556,32 @@ __device__ __forceinline__ void rows_smem_ff(const LineBlockArgs &p, const float
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const float2 w = __ldg(p.wff + (j - r - u));
+            const typename H::W w = __ldg(H::weights(p) + (j - r - u));
 #pragma unroll
-            for (int q = 0; q < SP; ++q) ff_fma(ah[q], al[q], w, v[u][q]);
+            for (int q = 0; q < SP; ++q) acc[q].mac(w, v[u][q]);
         }
 #pragma unroll
-        for (int q = 0; q < SP; ++q) ff_renorm(ah[q], al[q]);
+        for (int q = 0; q < SP; ++q) acc[q].renorm();
         slot += 8;
         if (slot >= NR) slot -= NR;
     }
     for (; r < r1; ++r) {
-        const float2 w = __ldg(p.wff + (j - r));
+        const typename H::W w = __ldg(H::weights(p) + (j - r));
 #pragma unroll
-        for (int q = 0; q < SP; ++q) ff_fma(ah[q], al[q], w, sR[slot * (LTS * SP) + ht + LTS * q]);
+        for (int q = 0; q < SP; ++q) acc[q].mac(w, sR[slot * (LTS * SP) + ht + LTS * q]);
         if (++slot == NR) slot = 0;
     }
 }
 
-// (ah, al) += sum_{r < rmax} w[j - r] D_r: rows below rlo from the global float-pair ring, the
-// rest from the shared-memory row ring.
-template <int SP>
-__device__ __forceinline__ void rows_split_ff(const LineBlockArgs &p, const float2 *sR, int ht, int a, int b, int j,
-                                              int rmax, int rlo, float *ah, float *al)
+// acc += sum_{r < rmax} w[j - r] D_r: rows below rlo from the global row ring, the rest from the
+// shared-memory row ring.
+template <class H, int SP>
+__device__ __forceinline__ void near_rows_split(const LineBlockArgs &p, const typename H::Row *sR, int ht, int a, int b,
+                                                int j, int rmax, int rlo, H *acc)
 {
     const int rg = min(rlo, rmax);
-    if (rg > 0) rows_ff<SP>(p, ht, a, b, j, rg, ah, al);
-    if (rmax > rg) rows_smem_ff<SP>(p, sR, ht, j, rg, rmax, ah, al);
+    if (rg > 0) near_rows<H, SP>(p, ht, a, b, j, rg, acc);
+    if (rmax > rg) near_rows_smem<H, SP>(p, sR, ht, j, rg, rmax, acc);
 }
 
 // v[n - 1] for a register array and a run-time n (1..SP) without indexing it dynamically,
@@ -549,20 +596,14 @@ __device__ __forceinline__ double last_of(const double (&v)[SP], int n)
     return r;
 }
 
-// out = (ah + al) sg for this thread's nodes, sg a per-node float pair: float-float, one FP64 add.
-template <int SP>
-__device__ __forceinline__ void history_store_scaled_ff(int ht, int a, int b, const float *ah, const float *al,
-                                                        const float2 *sg, double *out)
+// out = acc sg for this thread's nodes, sg a per-node scale.
+template <class H, int SP>
+__device__ __forceinline__ void history_store_scaled(int ht, int a, int b, const H *acc, const typename H::W *sg,
+                                                     double *out)
 {
 #pragma unroll
     for (int q = 0; q < SP; ++q)
-        if (a + ht + LTS * q < b) {
-            const float ph = __fmul_rn(ah[q], sg[q].x);
-            float pe = __fmaf_rn(ah[q], sg[q].x, -ph);
-            pe = __fmaf_rn(ah[q], sg[q].y, pe);
-            pe = __fmaf_rn(al[q], sg[q].x, pe);
-            out[ht + LTS * q] = f2d_bits(ph) + f2d_bits(pe);
-        }
+        if (a + ht + LTS * q < b) out[ht + LTS * q] = acc[q].scaled(sg[q]);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -586,9 +627,11 @@ __device__ __forceinline__ void history_store_scaled_ff(int ht, int a, int b, co
 // increments and weights as float pairs; the solver hands each new FP64 row over in shared
 // memory and the history warps convert it), and the four history warps form the four carry
 // dot products side by side.
-template <int SP, bool EXPL>
+template <class H, int SP, bool EXPL>
 __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
 {
+    using Row = typename H::Row;
+    constexpr bool FF = std::is_same<H, NearFF>::value;
     __shared__ double sS[2][LTS * SP];                   // H_t by parity of t
     __shared__ double sUf[EXPL ? LTS : 1], sUl[EXPL ? LTS : 1];   // per solver thread: first, last ub
     __shared__ double sD[2][LTS * SP];                   // D_t (FP64) by parity of t
@@ -596,7 +639,7 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
     __shared__ double sCf[NWS][NWS], sCb[NWS][NWS];
     __shared__ double s_red[4];                          // c_in, Mb.U0, Kb.Y, right end value
     __shared__ int s_abort;
-    extern __shared__ float2 spec_rows[];                // [NR][LTS * SP]: the newest increment rows
+    extern __shared__ double spec_rows[];                // [NR][LTS * SP]: the newest increment rows
     const int tid = threadIdx.x;
     const bool solver = tid < LTS;
     const int c = blockIdx.x, G = p.G, N = p.N;
@@ -684,69 +727,62 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
             }
         };
         constexpr int NR = SpecRing<SP>::NR;
-        float2 *sR = spec_rows;
+        Row *sR = reinterpret_cast<Row *>(spec_rows);
         const int rlo0 = max(0, p.j0 - NR);              // rows of earlier launches into the ring
         for (int r = rlo0; r < p.j0; ++r) {
 #pragma unroll
             for (int q = 0; q < SP; ++q) {
                 const int i = a + ht + LTS * q;
-                if (i < b) sR[(r % NR) * (LTS * SP) + ht + LTS * q] = p.ringf[(int64_t)r * p.P + i];
+                if (i < b) sR[(r % NR) * (LTS * SP) + ht + LTS * q] = H::rows(p)[(int64_t)r * p.P + i];
             }
         }
-        float2 sg[SP];                                   // -g of this thread's nodes
+        typename H::W sg[SP];                            // -g of this thread's nodes
 #pragma unroll
         for (int q = 0; q < SP; ++q) {
             const int i = a + ht + LTS * q;
-            sg[q] = i < b ? __ldg(p.ngf + i) : make_float2(0.f, 0.f);
+            sg[q] = i < b ? __ldg(H::scale(p) + i) : H::zero();
         }
-        float h3[3][SP], l3[3][SP];                      // H_j0, H_j0+1, H_j0+2
-#pragma unroll
-        for (int m = 0; m < 3; ++m)
-#pragma unroll
-            for (int q = 0; q < SP; ++q) { h3[m][q] = 0.f; l3[m][q] = 0.f; }
-        far_fold_ff<SP, 3>(p, ht, a, b, p.j0, h3, l3);
-        rows_split_ff<SP>(p, sR, ht, a, b, p.j0, max(p.j0 - 2, 0), rlo0, h3[0], l3[0]);
-        history_store_scaled_ff<SP>(ht, a, b, h3[0], l3[0], sg, sS[p.j0 & 1]);
-        __syncthreads();                                                    // start: the solver's prologue
+        H h3[3][SP];                                     // H_j0, H_j0+1, H_j0+2
+        far_fold<H, SP, 3>(p, ht, a, b, p.j0, h3);
+        near_rows_split<H, SP>(p, sR, ht, a, b, p.j0, max(p.j0 - 2, 0), rlo0, h3[0]);
+        history_store_scaled<H, SP>(ht, a, b, h3[0], sg, sS[p.j0 & 1]);
+        __syncthreads_or(0);                                                // start: the solver's prologue
         if (p.j0 + 1 < jend) {                                              // runs beside the rest
-            rows_split_ff<SP>(p, sR, ht, a, b, p.j0 + 1, max(p.j0 - 1, 0), rlo0, h3[1], l3[1]);
-            history_store_scaled_ff<SP>(ht, a, b, h3[1], l3[1], sg, sS[(p.j0 + 1) & 1]);
+            near_rows_split<H, SP>(p, sR, ht, a, b, p.j0 + 1, max(p.j0 - 1, 0), rlo0, h3[1]);
+            history_store_scaled<H, SP>(ht, a, b, h3[1], sg, sS[(p.j0 + 1) & 1]);
         }
-        float ah[SP], al[SP];
+        H acc[SP];
 #pragma unroll
-        for (int q = 0; q < SP; ++q) { ah[q] = h3[2][q]; al[q] = l3[2][q]; }
-        if (p.j0 + 2 < jend) rows_split_ff<SP>(p, sR, ht, a, b, p.j0 + 2, p.j0, rlo0, ah, al);   // complete
-        const float2 w3 = __ldg(p.wff + 3);
+        for (int q = 0; q < SP; ++q) acc[q] = h3[2][q];
+        if (p.j0 + 2 < jend) near_rows_split<H, SP>(p, sR, ht, a, b, p.j0 + 2, p.j0, rlo0, acc);   // complete
+        const typename H::W w3 = __ldg(H::weights(p) + 3);
         for (int s = 0; s < p.nsteps; ++s) {
             __syncthreads();                                                // X(s): D_{t-1} is in sD
             if (s_abort) return;
             const int t = p.j0 + s;
-            if (s > 0) {                                                    // row t-1 as float pairs
+            if (s > 0) {                                                    // row t-1 into the rings
                 const double *dd = sD[(t - 1) & 1];
-                float2 *row = p.ringf + (int64_t)(t - 1) * p.P;
-                float2 *srow = sR + ((t - 1) % NR) * (LTS * SP);
+                Row *srow = sR + ((t - 1) % NR) * (LTS * SP);
 #pragma unroll
                 for (int q = 0; q < SP; ++q) {
                     const int i = a + ht + LTS * q;
                     if (i < b) {
-                        const float2 f = d2ff(dd[ht + LTS * q]);
-                        row[i] = f;
+                        const Row f = H::row(dd[ht + LTS * q]);
+                        if (FF) H::rows(p)[(int64_t)(t - 1) * p.P + i] = f;  // (the solver writes the FP64 row)
                         srow[ht + LTS * q] = f;
-                        if (t + 2 < jend) ff_fma(ah[q], al[q], w3, f);
+                        if (t + 2 < jend) acc[q].mac(w3, f);
                     }
                 }
             }
-            if (t + 2 < jend) history_store_scaled_ff<SP>(ht, a, b, ah, al, sg, sS[t & 1]);
+            if (t + 2 < jend) history_store_scaled<H, SP>(ht, a, b, acc, sg, sS[t & 1]);
             carries(s);
             asm volatile("bar.arrive 2, %0;" ::"n"(2 * LTS) : "memory");      // (C): carries of step t
             if (t + 3 < jend) {
-                float fh[1][SP], fl[1][SP];
+                H f[1][SP];
+                far_fold<H, SP, 1>(p, ht, a, b, t + 3, f);
 #pragma unroll
-                for (int q = 0; q < SP; ++q) { fh[0][q] = 0.f; fl[0][q] = 0.f; }
-                far_fold_ff<SP, 1>(p, ht, a, b, t + 3, fh, fl);
-#pragma unroll
-                for (int q = 0; q < SP; ++q) { ah[q] = fh[0][q]; al[q] = fl[0][q]; }
-                rows_split_ff<SP>(p, sR, ht, a, b, t + 3, t, max(0, t - NR), ah, al);
+                for (int q = 0; q < SP; ++q) acc[q] = f[0][q];
+                near_rows_split<H, SP>(p, sR, ht, a, b, t + 3, t, max(0, t - NR), acc);
             }
         }
         return;
@@ -878,9 +914,59 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
         sUf[tid] = cnt > 0 ? u[0] : 0.0;
         sUl[tid] = cnt > 0 ? last_of<SP>(u, cnt) : 0.0;
     }
-    __syncthreads();                                                        // start: H_j0 ready
-    // ---- prologue: step j0 from its full right-hand side
-    {
+    // step t+1's right-hand side on Omega0 (state u^t, ub_t, D_{t-1}; hs holds -g H_{t+1})
+    auto omega0 = [&](int64_t n, const double *hs, const double (&ub)[SP]) {
+        const double *src = src_row(n);
+        if (src) {
+#pragma unroll
+            for (int k = 0; k < SP; ++k) {
+                om[k] = 0.0;
+                if (k < cnt) {
+                    const double h = fma(kng[k], __ldg(src + i0 + k), fma(kc3[k], dm1[k], hs[i0 - a + k]));
+                    om[k] = fma(kc1[k], ub[k], fma(kc2[k], u[k], h));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < SP; ++k) {
+                om[k] = 0.0;
+                if (k < cnt) om[k] = fma(kc1[k], ub[k], fma(kc2[k], u[k], fma(kc3[k], dm1[k], hs[i0 - a + k])));
+            }
+        }
+    };
+    double ubc[SP], ubp[SP], ubprev[SP];                 // ub_t corrected, ub'_{t+1}, ub_{t-1}
+    double ypl = 0.0;                                    // y'_{t+1} at the chunk's last node
+    double cin = 0.0, ubv = 0.0, UNv = 0.0;              // carries and right end of the last gathered step
+    // go on from the launch before, unless the chunk's state is not what that launch left
+    bool changed = FF || p.j0 == 0;
+    if (!changed) {
+        cin = p.ccar[4 * c];
+        ubv = p.ccar[4 * c + 1];
+        UNv = p.ccar[4 * c + 2];
+#pragma unroll
+        for (int k = 0; k < SP; ++k) {
+            ubprev[k] = k < cnt ? p.cub[i0 + k] : 0.0;
+            if (k < cnt)
+                changed |= __double_as_longlong(fma(kCB[k], ubv, fma(kGG[k], cin, ubprev[k]))) != __double_as_longlong(u[k]);
+        }
+        if (ownsN) changed |= __double_as_longlong(UNv) != __double_as_longlong(uNv);
+    }
+    const bool cont = !__syncthreads_or(changed);                           // start: H_j0 ready
+    if (cont) {
+        // ---- step j0 on Omega0, as the launch that ran step j0 - 1 would have
+#pragma unroll
+        for (int k = 0; k < SP; ++k) {
+            u[k] = k < cnt ? p.cu[i0 + k] : 0.0;
+            dm1[k] = dm2[k];
+        }
+        omega0(p.n0, sS[p.j0 & 1], ubprev);
+        sweeps();
+        ypl = last ? last_of<SP>(yv, cnt) : 0.0;
+#pragma unroll
+        for (int k = 0; k < SP; ++k) ubp[k] = ubw[k];
+        if (ownsN) uNv = p.ccar[4 * c + 3];
+    } else {
+        // ---- prologue: step j0 from its full right-hand side
         const double *src = src_row(p.n0);
         const double *hs = sS[p.j0 & 1];                 // -g H_j0
         double ul = 0.0, hr = 0.0;                       // explicit part: the neighbours of the segment
@@ -912,15 +998,12 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
         if (ownsN && flux) st_relaxed_f64(agg + 2 * G, last_of<SP>(u, cnt));
         if (last) st_relaxed_f64(agg + 2 * c, last_of<SP>(yv, cnt));
         if (tid == 0) st_relaxed_f64(agg + 2 * c + 1, ubw[0]);
-    }
-    double ubc[SP], ubp[SP], ubprev[SP];                 // ub_t corrected, ub'_{t+1}, ub_{t-1}
 #pragma unroll
-    for (int k = 0; k < SP; ++k) { ubc[k] = ubw[k]; ubp[k] = 0.0; ubprev[k] = 0.0; }
-    double ypl = 0.0;                                    // y'_{t+1} at the chunk's last node
-    double cin = 0.0, ubv = 0.0;                         // carries of the last gathered step
+        for (int k = 0; k < SP; ++k) { ubc[k] = ubw[k]; ubp[k] = 0.0; ubprev[k] = 0.0; }
+    }
     for (int s = 0; s < p.nsteps; ++s) {
         const int t = p.j0 + s;
-        if (s > 0) {
+        if (s > 0 || cont) {
             // ---- carries of step t-1: first step t's corrected aggregates (the chunk's last y,
             // first u; at a flux end the new U[N-1]) go out, then state u^t, increment D_{t-1}
             // and the corrected backward results
@@ -944,9 +1027,8 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
                 }
             }
             if (ownsN) {
-                const double UN = s_red[3];
-                p.ring[(int64_t)(t - 1) * p.P + N] = UN - uNv;
-                uNv = UN;
+                p.ring[(int64_t)(t - 1) * p.P + N] = UNv - uNv;
+                uNv = UNv;
             }
         }
         if constexpr (EXPL) {                            // the segment's first and last ub_t
@@ -956,24 +1038,7 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
         __syncthreads();                                                    // X(s)
         if (t + 1 < jend) {
             // ---- step t+1 on Omega0, while the aggregates of step t are exchanged
-            const double *src = src_row(p.n0 + s + 1);
-            const double *hs = sS[(t + 1) & 1];          // -g H_{t+1}
-            if (src) {
-#pragma unroll
-                for (int k = 0; k < SP; ++k) {
-                    om[k] = 0.0;
-                    if (k < cnt) {
-                        const double h = fma(kng[k], __ldg(src + i0 + k), fma(kc3[k], dm1[k], hs[i0 - a + k]));
-                        om[k] = fma(kc1[k], ubc[k], fma(kc2[k], u[k], h));
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < SP; ++k) {
-                    om[k] = 0.0;
-                    if (k < cnt) om[k] = fma(kc1[k], ubc[k], fma(kc2[k], u[k], fma(kc3[k], dm1[k], hs[i0 - a + k])));
-                }
-            }
+            omega0(p.n0 + s + 1, sS[(t + 1) & 1], ubc);
             if constexpr (EXPL) {                        // neighbours' ub_t inside the chunk
                 const double xl = (cnt > 0 && tid > 0) ? sUl[tid - 1] : 0.0;
                 const double xr = (cnt > 0 && i1 < b) ? sUf[tid + 1] : 0.0;
@@ -997,11 +1062,22 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
             return;
         }
         cin = s_red[0];
-        ubv = fma(mbc, s_red[3], s_red[1] + s_red[2]);
+        UNv = s_red[3];
+        ubv = fma(mbc, UNv, s_red[1] + s_red[2]);
 #pragma unroll
         for (int k = 0; k < SP; ++k) ubprev[k] = ubc[k];
     }
     // ---- carries of the last step: the final state and increment (FP64 ring and float pairs)
+    if (!FF && jend < BLK) {                             // for a launch that goes on from here
+#pragma unroll
+        for (int k = 0; k < SP; ++k)
+            if (k < cnt) {
+                p.cu[i0 + k] = u[k];
+                p.cub[i0 + k] = ubprev[k];
+            }
+        if (tid == 0) { p.ccar[4 * c] = cin; p.ccar[4 * c + 1] = ubv; p.ccar[4 * c + 2] = UNv; }
+        if (ownsN) p.ccar[4 * c + 3] = uNv;
+    }
     {
         const int64_t row = (int64_t)(jend - 1) * p.P;
 #pragma unroll
@@ -1010,16 +1086,74 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
                 const double un = fma(kCB[k], ubv, fma(kGG[k], cin, ubprev[k]));
                 const double d = un - u[k];
                 p.ring[row + i0 + k] = d;
-                p.ringf[row + i0 + k] = d2ff(d);
+                if (FF) p.ringf[row + i0 + k] = d2ff(d);
                 p.U[i0 + k] = un;
             }
         }
         if (ownsN) {
-            const double UN = s_red[3];
-            p.ring[row + N] = UN - uNv;
-            p.U[N] = UN;
+            p.ring[row + N] = UNv - uNv;
+            p.U[N] = UNv;
         }
     }
+}
+
+// Far history of a block in FP64: C[j][i] = sum_{t0 <= t < nb0} w[nb0 + j - t] D_t[i] for the block's 64
+// steps at once, so that a row is read 4 times per 64 steps (once per FJ steps) instead of once per
+// step. CTA: 32 nodes (lanes) x FJ steps; its FW warps take consecutive slices of the rows and their
+// sums are added in order. A thread slides the FJ weights through registers (the next row needs
+// one new weight). Bound by the FP64 pipe: one multiply-add per row, step and node; the row
+// slices give a short line (1,000 nodes: 32 x 4 CTAs) 8 warps per SM, enough to fill it.
+constexpr int FJ = 16, FW = 8;
+
+__global__ void __launch_bounds__(32 * FW) k_far64(const double *__restrict__ D, int64_t P, int N, int t0, int nb0,
+                                                   const double *__restrict__ wlag, double *__restrict__ C)
+{
+    __shared__ double red[FW][FJ][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+    const int j0 = blockIdx.y * FJ;
+    const int per = (nb0 - t0 + FW - 1) / FW;
+    const int ta = t0 + warp * per, tb = min(ta + per, nb0);
+    const double *col = D + (i < N ? i : N - 1);
+    double acc[FJ], w[FJ];
+#pragma unroll
+    for (int j = 0; j < FJ; ++j) acc[j] = 0.0;
+    // w[(j - u) mod FJ] = weight of step j at row ta + u, u counted within FJ rows
+#pragma unroll
+    for (int j = 0; j < FJ; ++j) w[j] = __ldg(wlag + (nb0 + j0 + j - min(ta, nb0)));
+    for (int t = ta; t < tb; t += FJ) {
+        double d[FJ], wn[FJ];
+#pragma unroll
+        for (int u = 0; u < FJ; ++u) {
+            d[u] = t + u < tb ? __ldcg(col + (int64_t)(t + u) * P) : 0.0;
+            wn[u] = __ldg(wlag + max(nb0 + j0 - (t + u) - 1, 0));     // enters for row t + u + 1
+        }
+#pragma unroll
+        for (int u = 0; u < FJ; ++u) {
+#pragma unroll
+            for (int j = 0; j < FJ; ++j) acc[j] = fma(w[(j - u) & (FJ - 1)], d[u], acc[j]);
+            w[(FJ - 1 - u) & (FJ - 1)] = wn[u];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < FJ; ++j) red[warp][j][lane] = acc[j];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < FJ / FW; ++q) {
+        const int j = warp + q * FW;
+        double s = red[0][j][lane];
+#pragma unroll
+        for (int v = 1; v < FW; ++v) s += red[v][j][lane];
+        if (i < N) C[(int64_t)(j0 + j) * P + i] = s;
+    }
+}
+
+static int launch_far64(cudaStream_t st, const double *D, int64_t P, int64_t N, int64_t t0, int64_t nb0,
+                        const double *wlag, double *C)
+{
+    k_far64<<<dim3((unsigned)((N + 31) / 32), BLK / FJ), 32 * FW, 0, st>>>(D, P, (int)N, (int)t0, (int)nb0, wlag, C);
+    FPDE_LAUNCHED(1);
+    return FPDE_OK;
 }
 
 }  // namespace fpde
@@ -1035,6 +1169,7 @@ struct fpde_line {
     int sbk = 4;                              // blocks per far super-block (three-slice path)
     int max_lag = INT_MAX;                    // restricted summing: lags above are dropped
     bool split = false;
+    bool b64 = false;                         // FP64 in 64-step blocks (k_far64, k_line_block_spec<Near64>)
     double lam = 0, lamR = 0, kkk0 = 0, AlN = 0;
     double *A = nullptr, *g = nullptr, *al = nullptr, *cf = nullptr, *cb = nullptr;
     double *CF = nullptr, *CB = nullptr, *GG = nullptr;
@@ -1044,6 +1179,7 @@ struct fpde_line {
     double *sga = nullptr, *sng = nullptr, *sc1 = nullptr, *sc2 = nullptr, *sc3 = nullptr;  // -g pre-scaling
     float2 *sngf = nullptr;
     double *sxa = nullptr, *sxb = nullptr;    // pre-scaled neighbour weights (explicit part)
+    double *cub = nullptr, *cu = nullptr, *ccar = nullptr;   // block solve's state at a cut (FP64 path)
     double *Lf = nullptr, *Mb = nullptr, *Kb = nullptr, *mb = nullptr;
     unsigned long long *cflag = nullptr, *seq = nullptr;
     double *sclane = nullptr, *scwarp = nullptr;
@@ -1144,14 +1280,19 @@ static cudaError_t spec_smem_attrs()
     auto opt = [&e](const void *fn, size_t bytes) {
         if (e == cudaSuccess) e = smem_opt_in(fn, (int)bytes);
     };
-    opt((const void *)k_line_block_spec<1, false>, SpecRing<1>::bytes);
-    opt((const void *)k_line_block_spec<2, false>, SpecRing<2>::bytes);
-    opt((const void *)k_line_block_spec<4, false>, SpecRing<4>::bytes);
-    opt((const void *)k_line_block_spec<8, false>, SpecRing<8>::bytes);
-    opt((const void *)k_line_block_spec<1, true>, SpecRing<1>::bytes);
-    opt((const void *)k_line_block_spec<2, true>, SpecRing<2>::bytes);
-    opt((const void *)k_line_block_spec<4, true>, SpecRing<4>::bytes);
-    opt((const void *)k_line_block_spec<8, true>, SpecRing<8>::bytes);
+    auto both = [&](auto h) {
+        using H = decltype(h);
+        opt((const void *)k_line_block_spec<H, 1, false>, SpecRing<1>::bytes);
+        opt((const void *)k_line_block_spec<H, 2, false>, SpecRing<2>::bytes);
+        opt((const void *)k_line_block_spec<H, 4, false>, SpecRing<4>::bytes);
+        opt((const void *)k_line_block_spec<H, 8, false>, SpecRing<8>::bytes);
+    };
+    both(NearFF());
+    both(Near64());
+    opt((const void *)k_line_block_spec<NearFF, 1, true>, SpecRing<1>::bytes);
+    opt((const void *)k_line_block_spec<NearFF, 2, true>, SpecRing<2>::bytes);
+    opt((const void *)k_line_block_spec<NearFF, 4, true>, SpecRing<4>::bytes);
+    opt((const void *)k_line_block_spec<NearFF, 8, true>, SpecRing<8>::bytes);
     return e;
 }
 
@@ -1159,8 +1300,9 @@ template <int SP>
 static cudaError_t launch_block_sp(cudaLaunchConfig_t cfg, const LineBlockArgs &a)
 {
     cfg.dynamicSmemBytes = SpecRing<SP>::bytes;     // both keep the newest rows in shared memory
-    return a.xa ? cudaLaunchKernelEx(&cfg, k_line_block_spec<SP, true>, a)
-                : cudaLaunchKernelEx(&cfg, k_line_block_spec<SP, false>, a);
+    if (!a.ringf) return cudaLaunchKernelEx(&cfg, k_line_block_spec<Near64, SP, false>, a);   // FP64 path
+    return a.xa ? cudaLaunchKernelEx(&cfg, k_line_block_spec<NearFF, SP, true>, a)
+                : cudaLaunchKernelEx(&cfg, k_line_block_spec<NearFF, SP, false>, a);
 }
 
 // Steps j0 .. j0+nsteps-1 of the block starting at nb0 in one persistent launch.
@@ -1171,7 +1313,7 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     a.A = L->A; a.g = L->g; a.al = L->al; a.cf = L->cf; a.cb = L->cb; a.CB = L->CB; a.GG = L->GG;
     a.lamv = L->lamv; a.eA = L->eA; a.eB = L->eB;
     a.src = L->srcd; a.src_rows = L->src_rows;
-    a.U = L->U; a.ring = L->ring; a.cfar = L->cfar; a.KS = KS; a.P = L->P; a.wlag = L->wlag;
+    a.U = L->U; a.ring = L->b64 ? L->D + nb0 * L->P : L->ring; a.cfar = L->cfar; a.KS = KS; a.P = L->P; a.wlag = L->wlag;
     a.far_ld = far_ld; a.far_row0 = far_row0;
     a.far_pairs = L->x3 ? 1 : 0;
     a.agg = L->agg; a.cflag = L->cflag; a.seq = L->seq;
@@ -1181,6 +1323,7 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     a.ringf = L->ringf; a.wff = L->wff;
     a.ga = L->sga; a.ng = L->sng; a.c1 = L->sc1; a.c2 = L->sc2; a.c3 = L->sc3; a.ngf = L->sngf;
     a.xa = L->sxa; a.xb = L->sxb;
+    a.cub = L->cub; a.cu = L->cu; a.ccar = L->ccar;
     a.lam = L->lam; a.g0 = L->d.left_value; a.gN = L->d.right_value; a.dLN = L->d.dLN; a.AlN = L->AlN;
     a.n0 = nb0 + j0; a.j0 = j0; a.nsteps = nsteps; a.N = (int)L->N; a.G = L->G; a.rkind = L->d.right_kind;
     a.chunk = L->chunk;
@@ -1205,6 +1348,25 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     if (e != cudaSuccess) return set_error(FPDE_ERR_CUDA, "line block launch: %s", cudaGetErrorString(e));
     count_launches(1);
     return FPDE_OK;
+}
+
+// Whether an FP64 line runs in 64-step blocks: every one but
+//   - the Richards problem (its coefficients change with the state);
+//   - lines with an explicit part, whose speculative form rounds 3 to 6 times worse than the
+//     per-step form (20,000 intervals: 1.1e-9 against 1.9e-10);
+//   - a requested number of row splits of the per-step history sum, or a requested partition that
+//     only fits the per-step form's wider CTAs;
+//   - lines of over 1,024 nodes per SM.
+// N = 1,000, 1,000 steps: 24.3 ms per step by step (two launches a step), 4.6 ms in blocks; N = 65,536, 2,048
+// steps: 270 ms (the row sums' FP64 multiply-adds) against 245 ms.
+static bool line_blocked64(const fpde_ctx *ctx, const fpde_line_desc &d, const fpde_line_tuning *tu)
+{
+    if (d.richards || d.theta != 0.0 || d.N > (int64_t)ctx->sm_count * LTS * LSEG) return false;
+    if (!tu) return true;
+    if (tu->gemv_splits > 0) return false;
+    if (tu->solve_sp <= 0 && tu->chunks <= 0) return true;
+    const int64_t per = (int64_t)LTS * (tu->solve_sp > 0 ? tu->solve_sp : LSEG);
+    return (d.N + per - 1) / per <= (tu->chunks > 0 ? tu->chunks : ctx->sm_count);
 }
 
 #define PROBE_REC(ev, i) \
@@ -1237,7 +1399,21 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
     for (int64_t n = n0; n < n0 + steps; ++n) {
         const bool probe_step = L->probe_every > 0 && n >= 1 && (n % L->probe_every) == L->probe_every - 1;
         cudaEvent_t *ev;
-        if (!L->split) {
+        if (L->b64) {
+            const int64_t nb0 = n - n % BLK, t0 = nb0 > L->max_lag ? nb0 - L->max_lag : 0;
+            const int j = (int)(n - nb0);
+            if (j == 0 && nb0 > t0) {
+                if ((rc = launch_far64(st, L->D, L->P, L->N, t0, nb0, L->wlag, L->cfar))) return rc;
+                ++k;
+            }
+            const int nst = (int)std::min<int64_t>(BLK - j, n0 + steps - n);
+            ev = L->probe_every > 0 ? probe_begin(L, 2, n, 0.0, 0.0, nst) : nullptr;
+            PROBE_REC(ev, 0);
+            if ((rc = line_launch_block(L, st, nb0, j, nst, nb0 > t0 ? 1 : 0, BLK, 0))) return rc;
+            PROBE_REC(ev, 1);
+            ++k;
+            n += nst - 1;
+        } else if (!L->split) {
             int KS = 0;
             const int64_t t0 = n > L->max_lag ? n - L->max_lag : 0;   // oldest row of the window
             const int64_t nr = n - t0;
@@ -1421,6 +1597,7 @@ int fpde_line_destroy(fpde_line *L)
     dev_free(L->wff);
     for (double *q : {L->sga, L->sng, L->sc1, L->sc2, L->sc3}) dev_free(q);
     dev_free(L->sngf);
+    for (double *q : {L->cub, L->cu, L->ccar}) dev_free(q);
     dev_free(L->sxa);
     dev_free(L->sxb);
     for (uint16_t *p : {L->h_hi, L->h_lo, L->w_hi, L->w_lo, L->h3[0], L->h3[1], L->h3[2], L->w3[0], L->w3[1],
@@ -1489,8 +1666,10 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     // path): one CTA when the line fits in 8 nodes per thread, otherwise the smallest sp that
     // keeps G within the SM count
     const bool split = d.precision != FPDE_PREC_FP64;
-    const int lt = split ? LTS : LT;
     const fpde_line_tuning *tu = d.tuning;
+    const bool b64 = !split && line_blocked64(ctx, d, tu);
+    const bool spec = split || b64;            // the persistent block solve
+    const int lt = spec ? LTS : LT;
     int sp = 1, G = 1;
     int64_t chunk;
     if (tu && (tu->solve_sp > 0 || tu->chunks > 0)) {
@@ -1504,7 +1683,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
         chunk = (chunk + sp - 1) / sp * sp;
         G = (int)((N + chunk - 1) / chunk);
     } else {
-        if (N <= (int64_t)lt * LSEG) {
+        if (N <= (int64_t)lt * LSEG && !b64) {
             while ((int64_t)lt * sp < N) sp <<= 1;
         } else {
             while (sp <= LSEG && (N + (int64_t)lt * sp - 1) / ((int64_t)lt * sp) > ctx->sm_count) sp <<= 1;
@@ -1523,14 +1702,15 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     }
     if (G > 160) return set_error(FPDE_ERR_UNSUPPORTED, "line solve: at most 160 chunks");
     int per_sm = 0;
-    if (split) {
-        int per_sm2 = 0;
+    if (spec) {
         FPDE_CUDA(spec_smem_attrs());
-        FPDE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_line_block_spec<LSEG, false>, 2 * LTS,
-                                                                SpecRing<LSEG>::bytes));
-        FPDE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_line_block_spec<LSEG, true>, 2 * LTS,
-                                                                SpecRing<LSEG>::bytes));
-        per_sm = std::min(per_sm, per_sm2);
+        per_sm = INT_MAX;
+        for (auto fn : {k_line_block_spec<NearFF, LSEG, false>, k_line_block_spec<NearFF, LSEG, true>,
+                        k_line_block_spec<Near64, LSEG, false>}) {
+            int n_sm = 0;
+            FPDE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n_sm, fn, 2 * LTS, SpecRing<LSEG>::bytes));
+            per_sm = std::min(per_sm, n_sm);
+        }
     }
     else FPDE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_line_solve<LSEG>, LT, 0));
     if (G > 1 && G > per_sm * ctx->sm_count)
@@ -1553,6 +1733,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     if (rich) L->sbk = 1;                      // per-block far history; the near history per step
     L->max_steps = d.max_steps;
     L->split = split;
+    L->b64 = b64;
     L->x3 = d.precision == FPDE_PREC_SPLIT_BF16X3;
     // local weight kkk0 = tau^{1-alpha}/(1-alpha); lam as in Om1 (:4191), lamR as in R (:3120);
     // or the caller's lag weights (distributed order: w[0] = b0/tau of eq_init, fr_do.cpp:688-694)
@@ -1626,7 +1807,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     // CTA the cross-warp coefficients of the solver warps.
     const int64_t GT = (int64_t)G * LTS;
     std::vector<double> hsl, hsw;
-    if (split) {
+    if (spec) {
         hsl.assign((size_t)12 * GT, 1.0);
         hsw.assign((size_t)G * 2 * NWS * NWS, 0.0);
         for (int cc = 0; cc < G; ++cc) {
@@ -1708,7 +1889,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
             hwff[j] = make_float2(hi, (float)(wlag[j] - (double)hi));
         }
     }
-    if (split) {
+    if (spec) {
         // E1, E2: Omega0's coefficients on the carries (c_in, u_b) of the step before. With an
         // explicit part (theta != 0) the new state at the neighbours enters too: inside the
         // chunk u = ub + c_in GG + u_b CB; before it u_{a-1} = al_{a-1} u_a + c_in (the backward
@@ -1775,12 +1956,15 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
                 dev_alloc((void **)&L->U, L->P * sizeof(double)) ||
                 dev_alloc((void **)&L->wrev, wrev.size() * sizeof(double)) ||
                 dev_alloc((void **)&L->agg, (size_t)BLK * (2 * G + 2) * sizeof(double)) ||
-                (split && (dev_alloc((void **)&L->sclane, hsl.size() * sizeof(double)) ||
+                (spec && (dev_alloc((void **)&L->sclane, hsl.size() * sizeof(double)) ||
                            dev_alloc((void **)&L->scwarp, hsw.size() * sizeof(double)))) ||
                 dev_alloc((void **)&L->barrier, 2 * sizeof(unsigned));
     if (!fail && !L->split) {
         fail = dev_alloc((void **)&L->D, (size_t)L->max_steps * L->P * sizeof(double)) ||
-               dev_alloc((void **)&L->part, (size_t)KS_MAX * L->P * sizeof(double));
+               (b64 ? dev_alloc((void **)&L->cfar, (size_t)BLK * L->P * sizeof(double)) ||
+                          dev_alloc((void **)&L->wlag, LW * sizeof(double)) || dev_alloc((void **)&L->cub, nb) ||
+                          dev_alloc((void **)&L->cu, nb) || dev_alloc((void **)&L->ccar, 4 * gb)
+                    : dev_alloc((void **)&L->part, (size_t)KS_MAX * L->P * sizeof(double)));
     }
     if (!fail && L->x3) {
         L->rows16 = (N + 1 + 127) / 128 * 128;
@@ -1836,12 +2020,12 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     if (!fail && split)
         fail = dev_alloc((void **)&L->ringf, (size_t)BLK * L->P * sizeof(float2)) ||
                dev_alloc((void **)&L->wff, (size_t)LW * sizeof(float2));
-    if (!fail && split)
+    if (!fail && spec)
         fail = dev_alloc((void **)&L->RB1, nb) || dev_alloc((void **)&L->RB2, nb) || dev_alloc((void **)&L->RY1, nb) ||
                dev_alloc((void **)&L->RY2, nb) || dev_alloc((void **)&L->sga, nb) ||
                dev_alloc((void **)&L->sng, nb) || dev_alloc((void **)&L->sc1, nb) || dev_alloc((void **)&L->sc2, nb) ||
                dev_alloc((void **)&L->sc3, nb) || dev_alloc((void **)&L->sngf, (size_t)N * sizeof(float2));
-    if (!fail && split && d.theta != 0.0)
+    if (!fail && spec && d.theta != 0.0)
         fail = dev_alloc((void **)&L->sxa, nb) || dev_alloc((void **)&L->sxb, nb);
     if (fail) {
         std::string keep = fpde_last_error_string();
@@ -1867,7 +2051,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
         cudaMemcpyAsync(L->wff, hwff.data(), (size_t)LW * sizeof(float2), cudaMemcpyHostToDevice, st);
         cudaMemsetAsync(L->ringf, 0, (size_t)BLK * L->P * sizeof(float2), st);
     }
-    if (split) {
+    if (spec) {
         cudaMemcpyAsync(L->RB1, hRB1.data(), nb, cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(L->RB2, hRB2.data(), nb, cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(L->RY1, hRY1.data(), nb, cudaMemcpyHostToDevice, st);
@@ -1912,7 +2096,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     cudaMemcpyAsync(L->Kb, hKb.data(), hKb.size() * sizeof(double), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(L->mb, hmb.data(), gb, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(L->cflag, 0, (size_t)G * sizeof(unsigned long long), st);
-    if (split) {
+    if (spec) {
         cudaMemcpyAsync(L->sclane, hsl.data(), hsl.size() * sizeof(double), cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(L->scwarp, hsw.data(), hsw.size() * sizeof(double), cudaMemcpyHostToDevice, st);
     }
@@ -1923,6 +2107,10 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     cudaMemsetAsync(L->barrier, 0, 2 * sizeof(unsigned), st);
     if (!L->split) {
         cudaMemsetAsync(L->D, 0, (size_t)L->max_steps * L->P * sizeof(double), st);
+        if (b64) {
+            cudaMemsetAsync(L->cfar, 0, (size_t)BLK * L->P * sizeof(double), st);
+            cudaMemcpyAsync(L->wlag, wlag.data(), LW * sizeof(double), cudaMemcpyHostToDevice, st);
+        }
     } else if (L->x3) {
         for (int q = 0; q < 3; ++q) {
             cudaMemsetAsync(L->h3[q], 0, (size_t)L->rows16 * L->ld16 * 2, st);
@@ -2171,8 +2359,8 @@ extern "C" int fpde_line_autotune(fpde_ctx *ctx, const fpde_line_desc *desc, con
     int rc = ctx_enter(ctx);
     if (rc) return rc;
     const fpde_line_desc &d = *desc;
-    const bool split = d.precision != FPDE_PREC_FP64;
-    const int lt = split ? LTS : LT;
+    const bool split = d.precision != FPDE_PREC_FP64, b64 = !split && line_blocked64(ctx, d, nullptr);
+    const int lt = split || b64 ? LTS : LT;
     const int64_t N = d.N;
     cudaStream_t st = ctx->stream;
     fpde_line_tuning best{};
@@ -2283,8 +2471,8 @@ extern "C" int fpde_line_autotune(fpde_ctx *ctx, const fpde_line_desc *desc, con
         dev_free(C);
         clear_error();
     }
-    if (!split) {
-        // 3. row splits of the FP64 history sum at min(max_steps, 2048) rows (zero data)
+    if (!split && !b64) {
+        // 3. row splits of the per-step FP64 history sum at min(max_steps, 2048) rows (zero data)
         const int64_t P = (N + 1 + 511) / 512 * 512;
         const int nrow = std::min(d.max_steps, 2048);
         double *D = nullptr, *part = nullptr, *w = nullptr;

@@ -307,7 +307,8 @@ typedef struct fpde_line_tuning {
     int chunks;         /* CTAs the line is split into for the solve (at most the SM count) */
     int far_splits;     /* K splits of the tensor-core far contraction: 1..4 (split paths; the
                            three-slice path keeps one slot for its super-block partial: 1..3) */
-    int gemv_splits;    /* row splits of the FP64 history sum: 1..64 (FP64 path) */
+    int gemv_splits;    /* row splits of the FP64 history sum: 1..64; asking for them selects the plain
+                           per-step form of the FP64 path (0: 64-step blocks where they apply) */
     int far_super;      /* three-slice path: 64-step blocks per far super-block, 1..4 (the history
                            older than a super-block is contracted once for all its steps) */
     double ms_per_step; /* output of fpde_line_autotune: measured time per step of the choice */
