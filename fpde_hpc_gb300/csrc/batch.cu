@@ -1,5 +1,5 @@
 // Ensemble of independent 1D Caputo columns (fpde_batch_*): many lines of different length,
-// order and coefficients advanced together, two kernels per time step for the whole ensemble.
+// order and coefficients advanced together, three kernels per time step for the whole ensemble.
 //
 // Layout in HBM: the columns' nodes are concatenated, column c occupying
 // [off_c, off_c + P_c) with P_c = N_c + 1 rounded up to 512, so that every CTA of the
@@ -9,10 +9,11 @@
 // Per time step n:
 //   1. k_batch_partial : part[ks][q] = sum_t w_c[n-t] D_t[q], the column's lag weights picked
 //                        per CTA (one flat grid over all nodes: balanced by construction)
-//   2. k_batch_solve   : one persistent launch fed by a device work queue: each CTA takes the
-//                        next column (largest first) from an atomic counter of the step and runs
-//                        Thomas on it (fpde_hpc_1d.cpp al1/bt1/U1 :4002-4027, :4585-4590,
-//                        :4683-4724) as segment sweeps joined by a CTA scan, then writes U and D_n.
+//   2. k_batch_sweep   : Thomas (fpde_hpc_1d.cpp al1/bt1/U1 :4002-4027, :4585-4590, :4683-4724) inside
+//                        every chunk of up to 1,024 nodes of a column from zero carries: the chunk's
+//                        solution, its last y and first u; the column's last chunk to finish solves
+//                        the column's chunk-level recurrences for every chunk's carries
+//   3. k_batch_join    : u = u^chunk + c_in KF + c_out CB, writing U and D_n
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
 // three-slice tensor-core contraction of all history before the block with one weight tile
 // per column (tc_far.cu; each 128-row tile picks its column's tile), and per step the near
@@ -22,7 +23,6 @@
 #include <algorithm>
 #include <cmath>
 #include <map>
-#include <numeric>
 #include <string>
 #include <vector>
 
@@ -35,19 +35,17 @@
 
 namespace fpde {
 
-#ifndef FPDE_BATCH_THREADS
-#define FPDE_BATCH_THREADS 512
-#endif
-constexpr int BT = FPDE_BATCH_THREADS;   // threads per column CTA (halves the sequential segment of the longest
-                                         // columns, which set the step time of a skewed ensemble)
-constexpr int BW = BT / 32;
-
 struct ColInfo {
     int64_t off;              // first node of the column in the concatenated node space
-    int N;                    // intervals (nodes 0..N)
-    int seg;                  // nodes per thread segment (nodes 0..N-1 are swept)
+    int N;                    // intervals (nodes 0..N; nodes 0..N-1 are swept)
+    int chunk0, nchunk;       // the column's chunks
     double lam, g0, gN, dLN, AlN;
     int rkind;
+    int pad;
+};
+struct ChunkInfo {
+    int64_t off;              // first node in the concatenated node space (a multiple of 512)
+    int n, col, idx;          // nodes, column, position in the column
     int pad;
 };
 
@@ -86,166 +84,227 @@ __global__ void __launch_bounds__(256) k_batch_partial(const double2 *__restrict
     part[(int64_t)ks * P2 + i] = make_double2(ax, ay);
 }
 
-// Exclusive CTA scan of (P, X) pairs in thread order (up) or reverse order (down).
-template <bool UP>
-__device__ __forceinline__ void cta_scan_excl(double &P, double &X, double *wP, double *wX, int lane, int warp)
+// One step of every column, cut into chunks of CN nodes so that the work per CTA is even whatever the
+// columns' lengths (one CTA per column left most SMs idle behind the longest columns: 153 us per step
+// for 512 columns of 2.1 M nodes, and its segments were read with strides of up to 256 bytes). Bound
+// by the FP64 pipe: 6 operations per node for the sweeps, about 1.5 for the scans, 3 to finish.
+// Measured on that ensemble: sweep 56 us (FP64 pipe 59 % busy; six CTAs per SM, four took 60 us),
+// join 18 us.
+constexpr int CT = 128, CW = CT / 32;    // threads of a chunk
+constexpr int CQ = 8;                    // nodes per thread
+constexpr int CN = CT * CQ;              // nodes per chunk
+
+// 8 consecutive doubles at a 16-byte aligned address
+__device__ __forceinline__ void load8(const double *p, double (&v)[CQ])
 {
-    if (UP) warp_scan_up(P, X, lane);
-    else warp_scan_down(P, X, lane);
-    double Pe = UP ? __shfl_up_sync(FULL, P, 1) : __shfl_down_sync(FULL, P, 1);
-    double Xe = UP ? __shfl_up_sync(FULL, X, 1) : __shfl_down_sync(FULL, X, 1);
-    if (lane == (UP ? 0 : 31)) { Pe = 1.0; Xe = 0.0; }
-    if (lane == (UP ? 31 : 0)) { wP[warp] = P; wX[warp] = X; }
-    __syncthreads();
-    if (warp == 0) {
-        double Pw = lane < BW ? wP[lane] : 1.0, Xw = lane < BW ? wX[lane] : 0.0;
-        if (UP) warp_scan_up(Pw, Xw, lane);
-        else warp_scan_down(Pw, Xw, lane);
-        double Pwe = UP ? __shfl_up_sync(FULL, Pw, 1) : __shfl_down_sync(FULL, Pw, 1);
-        double Xwe = UP ? __shfl_up_sync(FULL, Xw, 1) : __shfl_down_sync(FULL, Xw, 1);
-        if (UP ? lane == 0 : lane >= BW - 1) { Pwe = 1.0; Xwe = 0.0; }
-        __syncwarp();
-        if (lane < BW) { wP[lane] = Pwe; wX[lane] = Xwe; }
+#pragma unroll
+    for (int k = 0; k < CQ; k += 2) {
+        const double2 x = __ldcg(reinterpret_cast<const double2 *>(p + k));
+        v[k] = x.x;
+        v[k + 1] = x.y;
     }
-    __syncthreads();
-    // compose: the warps before this one (wP, wX of this warp), then this warp's earlier lanes
-    X = fma(Pe, wX[warp], Xe);
-    P = Pe * wP[warp];
-    __syncthreads();                                                // wP/wX reused by the caller
 }
 
-__global__ void __launch_bounds__(BT) k_batch_solve(const ColInfo *__restrict__ cols, const int *__restrict__ order,
-                                                    int n_cols, unsigned *__restrict__ queue,
-                                                    const double *__restrict__ A, const double *__restrict__ g,
-                                                    const double *__restrict__ al, const double *__restrict__ segP,
-                                                    const double *__restrict__ segQ, const double *__restrict__ KF,
-                                                    const double *__restrict__ CB, const double *__restrict__ part,
-                                                    int KS, int64_t pstride, double *__restrict__ U,
-                                                    double *__restrict__ Y, double *__restrict__ Drow,
-                                                    float2 *__restrict__ Drowf)
+struct BatchSweepArgs {
+    const ColInfo *cols;
+    const ChunkInfo *chunks;
+    const double *ga, *g, *al;           // gA, g, Al per node (0, 0, Al[1] at a column's first node)
+    const double *lane;                  // [12][chunks CT]: 5 forward level products, prefix, 5 backward, suffix
+    const double *warp;                  // [chunks][2][CW]: the warps' forward and backward products
+    int64_t nlane;                       // chunks CT
+    const double *part;
+    int KS;
+    int64_t pstride;
+    const double *U;
+    double *Y;                           // the chunk's zero-carry solution
+    double *agg;                         // [chunks][2]: last y, first u; then the chunk's carries c_in, c_out
+    const double *cmap;                  // [chunks][3]: product of gA, and KF, CB at the chunk's first node
+    double *uN;                          // per column: U[N-1] before the step, then U[N] after it
+    unsigned *count;                     // per column: chunks done in this step
+};
+
+// One warp: the chunk-level recurrences of a column (at most 17 chunks up to 16,384 intervals, one per
+// lane). agg[k] (last y, first u of chunk k from zero carries) becomes chunk k's carries.
+__device__ void batch_carries(const ColInfo &c, int col, const BatchSweepArgs &p, int lane)
 {
-    __shared__ double wP[BW], wX[BW];
-    __shared__ double s_y, s_uN;
-    __shared__ int s_item;
-    while (true) {
-    if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= n_cols) return;
-    const int col = order[item];
-    const ColInfo c = cols[col];
+    const int nch = c.nchunk, per = (nch + 31) / 32;
+    const int a = min(lane * per, nch), b = min(a + per, nch);
+    double *ag = p.agg + 2 * (int64_t)c.chunk0;
+    const double *cm = p.cmap + 3 * (int64_t)c.chunk0;
+    double P = 1.0, X = 0.0;                             // y after this lane's chunks = P y_before + X
+    for (int k = a; k < b; ++k) {
+        const double pk = __ldg(cm + 3 * k);
+        X = fma(pk, X, __ldcg(ag + 2 * k));
+        P *= pk;
+    }
+    warp_scan_up(P, X, lane);
+    const double yN = __shfl_sync(FULL, X, 31);          // Bt[N]
+    double y = __shfl_up_sync(FULL, X, 1);
+    if (lane == 0) y = 0.0;
+    double Q = 1.0, V = 0.0;                             // u at this lane's first chunk = Q u_after + V
+    for (int k = a; k < b; ++k) {
+        const double yl = __ldcg(ag + 2 * k), v = fma(__ldg(cm + 3 * k + 1), y, __ldcg(ag + 2 * k + 1));
+        V = fma(Q, v, V);
+        Q *= __ldg(cm + 3 * k + 2);
+        __stcg(ag + 2 * k, y);                           // c_in
+        __stcg(ag + 2 * k + 1, v);
+        y = fma(__ldg(cm + 3 * k), y, yl);
+    }
+    double uN;                                           // right end (U1 :4685-4719) with the old U[N-1]
+    const double uNm1 = __ldcg(p.uN + col);
+    if (c.rkind == FPDE_BC_DIRICHLET) uN = c.gN;
+    else if (fabs(yN) > 1e-15) uN = (fabs(1.0 - c.AlN) > 1e-15) ? (yN + c.gN * c.dLN) / (1.0 - c.AlN) : uNm1;
+    else uN = (fabs(1.0 - c.AlN) > 1e-15) ? 0.0 : uNm1;
+    warp_scan_down(Q, V, lane);
+    double u = __shfl_down_sync(FULL, fma(Q, uN, V), 1);          // u after this lane's chunks
+    if (lane == 31) u = uN;
+    for (int k = b - 1; k >= a; --k) {
+        const double v = __ldcg(ag + 2 * k + 1);
+        __stcg(ag + 2 * k + 1, u);                       // c_out
+        u = fma(__ldg(cm + 3 * k + 2), u, v);
+    }
+    if (lane == 0) __stcg(p.uN + col, uN);
+}
+
+// The scans' products are time-invariant and come from tables, so a scan level is one shuffle and one
+// multiply-add; carries enter by a second sweep (the same operation count as adding responses,
+// without their loads).
+__global__ void __launch_bounds__(CT, 6) k_batch_sweep(BatchSweepArgs p)
+{
+    __shared__ double sX[2][CW];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t o = c.off;
-    const int i0 = min(tid * c.seg, c.N), i1 = min(i0 + c.seg, c.N);
-    // Segment sweeps from zero carries joined by CTA scans; the carries are applied in one
-    // independent pass, u = ub0 + c_in KF + c_out CB (KF: the segment's backward response to its
-    // forward prefix products, CB: suffix products of al; time-invariant, from the host), so two
-    // dependent FP64 chains per step instead of four. Loads are issued eight nodes at a time.
-    // forward: y0 from a zero carry (y_0 = g0 at the column's first node) into Y
-    double yl = 0.0;
-    for (int ib = i0; ib < i1; ib += 8) {
-        double uu[8], gg[8], aa[8], ss[8];
+    const ChunkInfo ch = p.chunks[blockIdx.x];
+    const ColInfo *c = p.cols + ch.col;
+    const int i0 = tid * CQ, cnt = min(max(ch.n - i0, 0), CQ);
+    const int64_t q = ch.off + (cnt > 0 ? i0 : 0);
+    const int64_t T = (int64_t)blockIdx.x * CT + tid;
+    double h[CQ], ga[CQ], al[CQ];
+    {
+        double u[CQ], g[CQ], s[CQ];
+        load8(p.U + q, u);
+        load8(p.g + q, g);
+        load8(p.ga + q, ga);
+        load8(p.al + q, al);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int i = ib + t;
-            const bool in = i < i1 && i > 0;
-            const int64_t q = o + (in ? i : 0);
-            uu[t] = in ? U[q] : 0.0;
-            gg[t] = in ? __ldg(g + q) : 0.0;
-            aa[t] = in ? __ldg(A + q) : 0.0;
-            double sv = 0.0;
-            for (int k = 0; k < KS; ++k)
-                if (in) sv += __ldcg(part + (int64_t)k * pstride + q);
-            ss[t] = sv;
-        }
+        for (int k = 0; k < CQ; ++k) s[k] = 0.0;
+        if (p.KS > 0) load8(p.part + q, s);
+        for (int r = 1; r < p.KS; ++r) {
+            double v[CQ];
+            load8(p.part + (int64_t)r * p.pstride + q, v);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int i = ib + t;
-            if (i < i1) {
-                if (i == 0) {
-                    yl = c.g0;                                          // Bt[1]
-                } else {
-                    const double om = -(c.lam * uu[t]) + ss[t];
-                    yl = gg[t] * (aa[t] * yl - om);
-                }
-                Y[o + i] = yl;
-            }
+            for (int k = 0; k < CQ; ++k) s[k] += v[k];
         }
+        const double lam = c->lam;
+#pragma unroll
+        for (int k = 0; k < CQ; ++k) h[k] = g[k] * fma(lam, u[k], -s[k]);       // -g Om
+        if (ch.idx == 0 && tid == 0) h[0] = c->g0;                             // Bt[1]
+        if (tid == 0 && ch.idx == c->nchunk - 1) p.uN[ch.col] = __ldcg(p.U + ch.off + ch.n - 1);
     }
-    const double pf = i1 > i0 ? __ldg(segP + (int64_t)col * BT + tid) : 1.0;
-    double P = pf;
-    double X = i1 > i0 ? yl : 0.0;
-    cta_scan_excl<true>(P, X, wP, wX, lane, warp);
-    const double cin = X;                                               // true y before the segment
-    if (i1 == c.N && i1 > i0) s_y = fma(pf, cin, yl);                   // Bt[N]
+    const double *lp = p.lane + T, *wp = p.warp + (int64_t)blockIdx.x * (2 * CW);
+    double pf[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) pf[k] = __ldg(lp + k * p.nlane);
+    // forward: y_i = gA y_{i-1} + h_i
+    double x = 0.0;
+#pragma unroll
+    for (int k = 0; k < CQ; ++k)
+        if (k < cnt) x = fma(ga[k], x, h[k]);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const double xp = __shfl_up_sync(FULL, x, 1 << k);
+        if (lane >= (1 << k)) x = fma(pf[k], xp, x);
+    }
+    double xe = __shfl_up_sync(FULL, x, 1);
+    if (lane == 0) xe = 0.0;
+    if (lane == 31) sX[0][warp] = x;
     __syncthreads();
-    if (tid == 0) {
-        double uN;
-        const double uNm1 = U[o + c.N - 1];
-        if (c.rkind == FPDE_BC_DIRICHLET) uN = c.gN;
-        else if (fabs(s_y) > 1e-15) uN = (fabs(1.0 - c.AlN) > 1e-15) ? (s_y + c.gN * c.dLN) / (1.0 - c.AlN) : uNm1;
-        else uN = (fabs(1.0 - c.AlN) > 1e-15) ? 0.0 : uNm1;
-        s_uN = uN;
+    double cw = 0.0;
+    for (int w = 0; w < warp; ++w) cw = fma(__ldg(wp + w), cw, sX[0][w]);
+    x = fma(pf[5], cw, xe);                                                    // y before this thread's nodes
+#pragma unroll
+    for (int k = 0; k < CQ; ++k)
+        if (k < cnt) h[k] = x = fma(ga[k], x, h[k]);                           // y
+    if (cnt > 0 && i0 + cnt == ch.n) p.agg[2 * (int64_t)blockIdx.x] = x;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) pf[k] = __ldg(lp + (6 + k) * p.nlane);
+    // backward: u_i = Al u_{i+1} + y_i
+    x = 0.0;
+#pragma unroll
+    for (int k = CQ - 1; k >= 0; --k)
+        if (k < cnt) x = fma(al[k], x, h[k]);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const double xn = __shfl_down_sync(FULL, x, 1 << k);
+        if (lane + (1 << k) < 32) x = fma(pf[k], xn, x);
     }
+    xe = __shfl_down_sync(FULL, x, 1);
+    if (lane == 31) xe = 0.0;
+    if (lane == 0) sX[1][warp] = x;
     __syncthreads();
-    const double uN = s_uN;
-    // backward: ub0 from a zero carry over y0, into Y
-    double ul = 0.0;
-    for (int ie = i1 - 1; ie >= i0; ie -= 8) {
-        double yy[8], la[8];
+    cw = 0.0;
+    for (int w = CW - 1; w > warp; --w) cw = fma(__ldg(wp + CW + w), cw, sX[1][w]);
+    x = fma(pf[5], cw, xe);                                                    // u after this thread's nodes
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int i = ie - t;
-            const bool in = i >= i0;
-            const int64_t q = o + (in ? i : i0);
-            yy[t] = in ? Y[q] : 0.0;
-            la[t] = in ? __ldg(al + q) : 0.0;
-        }
+    for (int k = CQ - 1; k >= 0; --k)
+        if (k < cnt) h[k] = x = fma(al[k], x, h[k]);                           // u^chunk
+    if (tid == 0) p.agg[2 * (int64_t)blockIdx.x + 1] = x;
+    if (cnt == CQ) {
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int i = ie - t;
-            if (i >= i0) {
-                ul = fma(la[t], ul, yy[t]);
-                Y[o + i] = ul;
-            }
-        }
+        for (int k = 0; k < CQ; k += 2) *reinterpret_cast<double2 *>(p.Y + q + k) = make_double2(h[k], h[k + 1]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < CQ; ++k)
+            if (k < cnt) p.Y[q + k] = h[k];
     }
-    P = i1 > i0 ? __ldg(segQ + (int64_t)col * BT + tid) : 1.0;
-    X = i1 > i0 ? fma(cin, __ldg(KF + o + i0), ul) : 0.0;              // u at the segment start, c_out = 0
-    cta_scan_excl<false>(P, X, wP, wX, lane, warp);
-    const double cout = fma(P, uN, X);                                  // true u after the segment
-    // carries applied; U and the increment written
-    for (int ib = i0; ib < i1; ib += 8) {
-        double ub[8], kf[8], cb[8], uo[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int i = ib + t;
-            const bool in = i < i1;
-            const int64_t q = o + (in ? i : i0);
-            ub[t] = in ? Y[q] : 0.0;
-            kf[t] = in ? __ldg(KF + q) : 0.0;
-            cb[t] = in ? __ldg(CB + q) : 0.0;
-            uo[t] = in ? U[q] : 0.0;
+    // the column's last chunk to get here joins them
+    __threadfence();
+    __syncthreads();
+    if (warp != 0) return;
+    unsigned done = 0;
+    if (lane == 0) done = atomicAdd(p.count + ch.col, 1u);
+    done = __shfl_sync(FULL, done, 0);
+    if (done != (unsigned)c->nchunk - 1) return;
+    __threadfence();
+    if (lane == 0) p.count[ch.col] = 0;                                        // for the next step
+    batch_carries(*c, ch.col, p, lane);
+}
+
+struct BatchJoinArgs {
+    const ColInfo *cols;
+    const int *cta_col;
+    const double *KF, *CB;               // per node: responses of the chunk's solution to its carries
+    const double *Y, *agg, *uN;
+    double *U, *Drow;
+    float2 *Drowf;                       // split path: the float-pair ring row
+};
+
+// 512 nodes (of one chunk) per CTA, two per thread; bound by memory (56 bytes per node).
+__global__ void __launch_bounds__(256) k_batch_join(BatchJoinArgs p)
+{
+    const int col = p.cta_col[blockIdx.x];
+    const ColInfo *c = p.cols + col;
+    const int64_t q = (int64_t)blockIdx.x * 512 + 2 * threadIdx.x;
+    const int i = (int)(q - c->off), N = c->N;
+    if (i > N) return;
+    const int64_t k = c->chunk0 + min(i / CN, c->nchunk - 1);
+    const double cin = __ldg(p.agg + 2 * k), cout = __ldg(p.agg + 2 * k + 1);
+    const double2 ub = __ldcs(reinterpret_cast<const double2 *>(p.Y + q)), kf = __ldg(reinterpret_cast<const double2 *>(p.KF + q)),
+                  cb = __ldg(reinterpret_cast<const double2 *>(p.CB + q)), uo = *reinterpret_cast<const double2 *>(p.U + q);
+    double2 u = make_double2(fma(cout, cb.x, fma(cin, kf.x, ub.x)), fma(cout, cb.y, fma(cin, kf.y, ub.y)));
+    if (i == N) u.x = p.uN[col];
+    if (i + 1 == N) u.y = p.uN[col];
+    const double dx = u.x - uo.x, dy = u.y - uo.y;
+    if (i < N) {
+        *reinterpret_cast<double2 *>(p.U + q) = u;
+        *reinterpret_cast<double2 *>(p.Drow + q) = make_double2(dx, dy);
+        if (p.Drowf) {
+            const float2 f0 = d2ff(dx), f1 = d2ff(dy);
+            *reinterpret_cast<float4 *>(p.Drowf + q) = make_float4(f0.x, f0.y, f1.x, f1.y);
         }
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int i = ib + t;
-            if (i < i1) {
-                const int64_t q = o + i;
-                const double u = fma(cout, cb[t], fma(cin, kf[t], ub[t]));
-                U[q] = u;
-                Drow[q] = u - uo[t];
-                if (Drowf) Drowf[q] = d2ff(u - uo[t]);          // split path: the float-pair ring row
-            }
-        }
-    }
-    if (tid == 0) {
-        const double uo = U[o + c.N];
-        U[o + c.N] = uN;
-        Drow[o + c.N] = uN - uo;
-        if (Drowf) Drowf[o + c.N] = d2ff(uN - uo);
-    }
-    __syncthreads();                                                // s_item, s_y, s_uN reused
+    } else {
+        p.U[q] = u.x;
+        p.Drow[q] = dx;
+        if (p.Drowf) p.Drowf[q] = d2ff(dx);
     }
 }
 
@@ -259,14 +318,17 @@ struct fpde_batch {
     int64_t Ptot = 0;
     std::vector<int64_t> off;
     std::vector<int> N;
-    double *A = nullptr, *g = nullptr, *al = nullptr, *segP = nullptr, *segQ = nullptr;
-    double *KF = nullptr, *CB = nullptr;      // per node: segment responses KF and suffix products CB
+    double *ga = nullptr, *g = nullptr, *al = nullptr;
+    double *KF = nullptr, *CB = nullptr;      // per node: the chunk's responses to its carries
+    double *lane = nullptr, *warp = nullptr, *cmap = nullptr;   // scan products, chunk-level maps
+    double *agg = nullptr, *uN = nullptr;
+    unsigned *count = nullptr;
+    ChunkInfo *chunks = nullptr;
+    int n_chunks = 0;
     double *U = nullptr, *U0 = nullptr, *Y = nullptr, *D = nullptr, *part = nullptr, *wall = nullptr;
     ColInfo *cols = nullptr;
-    int *order = nullptr, *cta_col = nullptr;
+    int *cta_col = nullptr;
     int *col_lag = nullptr;                   // restricted summing: lags kept per column (null: all)
-    unsigned *queue = nullptr;                // per step: next work item of the solve
-    int solve_grid = 0;
     // split path
     bool split = false;
     int64_t ld16 = 0, ldp = 0, LW = 0;
@@ -288,7 +350,6 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
 {
     int64_t k = 0;
     int rc;
-    FPDE_CUDA(cudaMemsetAsync(b->queue + n0, 0, (size_t)steps * sizeof(unsigned), st));   // work queues of the run
     for (int64_t n = n0; n < n0 + steps; ++n) {
         int KS = 0;
         const double *part = b->part;
@@ -344,11 +405,19 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
             Drow = b->ring + (int64_t)j * b->Ptot;
             Drowf = b->ringf + (int64_t)j * b->Ptot;
         }
-        k_batch_solve<<<b->solve_grid, BT, 0, st>>>(b->cols, b->order, b->n_cols, b->queue + n, b->A, b->g, b->al,
-                                                    b->segP, b->segQ, b->KF, b->CB, part, KS, b->Ptot, b->U, b->Y, Drow,
-                                                    Drowf);
+        BatchSweepArgs sa;
+        sa.cols = b->cols; sa.chunks = b->chunks; sa.ga = b->ga; sa.g = b->g; sa.al = b->al;
+        sa.lane = b->lane; sa.warp = b->warp; sa.nlane = (int64_t)b->n_chunks * CT;
+        sa.part = part; sa.KS = KS; sa.pstride = b->Ptot; sa.U = b->U; sa.Y = b->Y; sa.agg = b->agg; sa.cmap = b->cmap;
+        sa.uN = b->uN; sa.count = b->count;
+        k_batch_sweep<<<b->n_chunks, CT, 0, st>>>(sa);
         FPDE_LAUNCHED(1);
-        ++k;
+        BatchJoinArgs ja;
+        ja.cols = b->cols; ja.cta_col = b->cta_col; ja.KF = b->KF; ja.CB = b->CB;
+        ja.Y = b->Y; ja.agg = b->agg; ja.uN = b->uN; ja.U = b->U; ja.Drow = Drow; ja.Drowf = Drowf;
+        k_batch_join<<<(unsigned)(b->Ptot / 512), 256, 0, st>>>(ja);
+        FPDE_LAUNCHED(1);
+        k += 2;
     }
     *nk = k;
     return FPDE_OK;
@@ -366,8 +435,8 @@ int fpde_batch_destroy(fpde_batch *b)
         cudaStreamSynchronize(b->ctx->stream);
     }
     b->graphs.clear();
-    for (double *p : {b->A, b->g, b->al, b->segP, b->segQ, b->KF, b->CB, b->U, b->U0, b->Y, b->D, b->part, b->wall, b->ring,
-                      b->cfar, b->wlag, b->Sn})
+    for (double *p : {b->ga, b->g, b->al, b->lane, b->warp, b->cmap, b->agg, b->uN, b->KF, b->CB, b->U, b->U0, b->Y, b->D,
+                      b->part, b->wall, b->ring, b->cfar, b->wlag, b->Sn})
         dev_free(p);
     for (int q = 0; q < 3; ++q) {
         dev_free(b->h3[q]);
@@ -379,9 +448,9 @@ int fpde_batch_destroy(fpde_batch *b)
     dev_free(b->pre);
     dev_free(b->wff);
     dev_free(b->wcol);
-    dev_free(b->queue);
     dev_free(b->cols);
-    dev_free(b->order);
+    dev_free(b->chunks);
+    dev_free(b->count);
     dev_free(b->cta_col);
     dev_free(b->col_lag);
     delete b;
@@ -441,9 +510,25 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
         tot += (cols[c].N + 1 + 511) / 512 * 512;
     }
     b->Ptot = tot;
-    std::vector<double> hA(tot, 0.0), hg(tot, 0.0), hal(tot, 0.0), hU(tot, 0.0);
-    std::vector<double> hP((size_t)n_cols * BT, 1.0), hQ((size_t)n_cols * BT, 1.0);
-    std::vector<double> hKF(tot, 0.0), hCB(tot, 0.0);
+    std::vector<double> hga(tot, 0.0), hg(tot, 0.0), hal(tot, 0.0), hU(tot, 0.0);
+    std::vector<double> hKF(tot, 0.0), hCB(tot, 0.0), hlane, hwarp, hmap;
+    std::vector<ChunkInfo> hch;
+    for (int c = 0; c < n_cols; ++c)
+        for (int64_t a = 0; a < cols[c].N; a += CN) {
+            ChunkInfo ci;
+            ci.off = b->off[c] + a;
+            ci.n = (int)std::min<int64_t>(CN, cols[c].N - a);
+            ci.col = c;
+            ci.idx = (int)(a / CN);
+            ci.pad = 0;
+            hch.push_back(ci);
+        }
+    b->n_chunks = (int)hch.size();
+    const int64_t nlane = (int64_t)hch.size() * CT;
+    hlane.assign((size_t)12 * nlane, 1.0);
+    hwarp.assign(hch.size() * 2 * CW, 1.0);
+    hmap.assign(hch.size() * 3, 1.0);
+    int chunk0 = 0;
     std::vector<double> hw((size_t)n_cols * (max_steps + 1), 0.0);
     std::vector<ColInfo> hc(n_cols);
     std::vector<int> cta_col(tot / 512);
@@ -464,13 +549,14 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
             Al = d.B[i] / ((d.Rlap[i] + lamR) - d.A[i] * Al);        // Al[i+1]
             hal[o + i] = Al;
             hg[o + i] = Al / d.B[i];
-            hA[o + i] = d.A[i];
+            hga[o + i] = hg[o + i] * d.A[i];
         }
         for (int64_t i = 0; i <= N; ++i) hU[o + i] = d.u0[i];
         ColInfo &ci = hc[c];
         ci.off = o;
         ci.N = (int)N;
-        ci.seg = (int)((N + BT - 1) / BT);
+        ci.chunk0 = chunk0;
+        ci.nchunk = (int)((N + CN - 1) / CN);
         ci.lam = lam;
         ci.g0 = d.left_value;
         ci.gN = d.right_value;
@@ -478,22 +564,50 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
         ci.AlN = Al;
         ci.rkind = d.right_kind;
         ci.pad = 0;
-        for (int t = 0; t < BT; ++t) {                              // segment products (time-invariant)
-            const int64_t i0 = std::min<int64_t>((int64_t)t * ci.seg, N), i1 = std::min<int64_t>(i0 + ci.seg, N);
-            double pf = 1.0, pb = 1.0;
-            for (int64_t i = i0; i < i1; ++i) {
-                pf *= hg[o + i] * hA[o + i];
-                hKF[o + i] = pf;                                       // forward prefix product (CF)
-                pb *= hal[o + i];
+        for (int k = 0; k < ci.nchunk; ++k, ++chunk0) {              // time-invariant products of the chunk
+            const int64_t a0 = o + (int64_t)k * CN, b0 = a0 + hch[chunk0].n;
+            double pr = 1.0;
+            for (int64_t i = a0; i < b0; ++i) { pr *= hga[i]; hKF[i] = pr; }
+            hmap[(size_t)chunk0 * 3] = pr;
+            double kf = 0.0, cb = 1.0;                                  // backward sweep of the prefix products, suffix of al
+            for (int64_t i = b0 - 1; i >= a0; --i) {
+                kf = hal[i] * kf + hKF[i];
+                cb = hal[i] * cb;
+                hKF[i] = kf;
+                hCB[i] = cb;
             }
-            hP[(size_t)c * BT + t] = pf;
-            hQ[(size_t)c * BT + t] = pb;
-            double kf = 0.0, cb = 1.0;                                  // backward sweep of CF, suffix of al
-            for (int64_t i = i1 - 1; i >= i0; --i) {
-                kf = hal[o + i] * kf + hKF[o + i];
-                cb = hal[o + i] * cb;
-                hKF[o + i] = kf;
-                hCB[o + i] = cb;
+            hmap[(size_t)chunk0 * 3 + 1] = kf;
+            hmap[(size_t)chunk0 * 3 + 2] = cb;
+            double Pt[CT], Qt[CT];
+            for (int t = 0; t < CT; ++t) {
+                Pt[t] = Qt[t] = 1.0;
+                for (int64_t i = a0 + (int64_t)t * CQ; i < std::min(a0 + (int64_t)(t + 1) * CQ, b0); ++i) {
+                    Pt[t] *= hga[i];
+                    Qt[t] *= hal[i];
+                }
+            }
+            for (int w = 0; w < CW; ++w) {
+                const double *pw = Pt + 32 * w, *qw = Qt + 32 * w;
+                double F[32], B[32];                                   // running level products
+                for (int l = 0; l < 32; ++l) { F[l] = pw[l]; B[l] = qw[l]; }
+                const int64_t T0 = (int64_t)chunk0 * CT + 32 * w;
+                for (int s = 0; s < 5; ++s) {
+                    for (int l = 0; l < 32; ++l) {
+                        hlane[(size_t)s * nlane + T0 + l] = F[l];
+                        hlane[(size_t)(6 + s) * nlane + T0 + l] = B[l];
+                    }
+                    for (int l = 31; l >= (1 << s); --l) F[l] *= F[l - (1 << s)];
+                    for (int l = 0; l + (1 << s) < 32; ++l) B[l] *= B[l + (1 << s)];
+                }
+                double pe = 1.0, qe = 1.0;
+                for (int l = 0; l < 32; ++l) {
+                    hlane[(size_t)5 * nlane + T0 + l] = pe;
+                    pe *= pw[l];
+                    hlane[(size_t)11 * nlane + T0 + 31 - l] = qe;
+                    qe *= qw[31 - l];
+                }
+                hwarp[(size_t)chunk0 * 2 * CW + w] = pe;
+                hwarp[(size_t)chunk0 * 2 * CW + CW + w] = qe;
             }
         }
         double *w = hw.data() + (size_t)c * (max_steps + 1);          // w[m] = w_c[max_steps - m]
@@ -523,20 +637,20 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
             for (int64_t q = o / 128; q < (o + Pc) / 128; ++q) hwcol[q] = c;
         }
     }
-    std::vector<int> order(n_cols);                                    // largest columns first
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->N[x] > b->N[y]; });
     const size_t tb = (size_t)tot * sizeof(double);
-    bool fail = dev_alloc((void **)&b->A, tb) || dev_alloc((void **)&b->g, tb) || dev_alloc((void **)&b->al, tb) ||
-                dev_alloc((void **)&b->segP, hP.size() * sizeof(double)) ||
-                dev_alloc((void **)&b->segQ, hQ.size() * sizeof(double)) || dev_alloc((void **)&b->U, tb) ||
+    bool fail = dev_alloc((void **)&b->ga, tb) || dev_alloc((void **)&b->g, tb) || dev_alloc((void **)&b->al, tb) ||
+                dev_alloc((void **)&b->lane, hlane.size() * sizeof(double)) ||
+                dev_alloc((void **)&b->warp, hwarp.size() * sizeof(double)) ||
+                dev_alloc((void **)&b->cmap, hmap.size() * sizeof(double)) ||
+                dev_alloc((void **)&b->agg, hch.size() * 2 * sizeof(double)) ||
+                dev_alloc((void **)&b->uN, (size_t)n_cols * sizeof(double)) ||
+                dev_alloc((void **)&b->count, (size_t)n_cols * sizeof(unsigned)) ||
+                dev_alloc((void **)&b->chunks, hch.size() * sizeof(ChunkInfo)) || dev_alloc((void **)&b->U, tb) ||
                 dev_alloc((void **)&b->KF, tb) || dev_alloc((void **)&b->CB, tb) ||
                 dev_alloc((void **)&b->U0, tb) || dev_alloc((void **)&b->Y, tb) ||
                 dev_alloc((void **)&b->cols, hc.size() * sizeof(ColInfo)) ||
-                dev_alloc((void **)&b->order, order.size() * sizeof(int)) ||
                 dev_alloc((void **)&b->cta_col, cta_col.size() * sizeof(int)) ||
-                (any_restrict && dev_alloc((void **)&b->col_lag, (size_t)n_cols * sizeof(int))) ||
-                dev_alloc((void **)&b->queue, (size_t)max_steps * sizeof(unsigned));
+                (any_restrict && dev_alloc((void **)&b->col_lag, (size_t)n_cols * sizeof(int)));
     if (!fail && !split) {
         fail = dev_alloc((void **)&b->D, (size_t)max_steps * tb) || dev_alloc((void **)&b->part, (size_t)KS_MAX * tb) ||
                dev_alloc((void **)&b->wall, hw.size() * sizeof(double));
@@ -571,17 +685,19 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
         return set_error(FPDE_ERR_NOMEM, "%s", keep.c_str());
     }
     cudaStream_t st = ctx->stream;
-    cudaMemcpyAsync(b->A, hA.data(), tb, cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(b->ga, hga.data(), tb, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->g, hg.data(), tb, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->al, hal.data(), tb, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(b->segP, hP.data(), hP.size() * sizeof(double), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(b->segQ, hQ.data(), hQ.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(b->lane, hlane.data(), hlane.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(b->warp, hwarp.data(), hwarp.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(b->cmap, hmap.data(), hmap.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(b->chunks, hch.data(), hch.size() * sizeof(ChunkInfo), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->KF, hKF.data(), tb, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->CB, hCB.data(), tb, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->U, hU.data(), tb, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->U0, hU.data(), tb, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(b->Y, 0, tb, st);
-    cudaMemsetAsync(b->queue, 0, (size_t)max_steps * sizeof(unsigned), st);
+    cudaMemsetAsync(b->count, 0, (size_t)n_cols * sizeof(unsigned), st);
     if (!split) {
         cudaMemsetAsync(b->D, 0, (size_t)max_steps * tb, st);
         cudaMemcpyAsync(b->wall, hw.data(), hw.size() * sizeof(double), cudaMemcpyHostToDevice, st);
@@ -605,13 +721,7 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
         cudaMemsetAsync(b->ringf, 0, (size_t)64 * tot * sizeof(float2), st);
         cudaMemcpyAsync(b->wcol, hwcol.data(), hwcol.size() * sizeof(int), cudaMemcpyHostToDevice, st);
     }
-    {                                                                  // persistent solve grid
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_solve, BT, 0);
-        b->solve_grid = std::max(1, std::min(n_cols, std::max(1, per_sm) * ctx->sm_count));
-    }
     cudaMemcpyAsync(b->cols, hc.data(), hc.size() * sizeof(ColInfo), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(b->order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(b->cta_col, cta_col.data(), cta_col.size() * sizeof(int), cudaMemcpyHostToDevice, st);
     if (b->col_lag) cudaMemcpyAsync(b->col_lag, lag_keep.data(), (size_t)n_cols * sizeof(int), cudaMemcpyHostToDevice, st);
     cudaError_t e = cudaStreamSynchronize(st);
