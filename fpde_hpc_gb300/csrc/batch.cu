@@ -329,6 +329,10 @@ struct fpde_batch {
     ColInfo *cols = nullptr;
     int *cta_col = nullptr;
     int *col_lag = nullptr;                   // restricted summing: lags kept per column (null: all)
+    // FP64 with the far history of every 64-step block in seven bf16 slices (else the rows of D)
+    bool x7 = false;
+    Hist7 h7;
+    FarPlan7 plan7;
     // split path
     bool split = false;
     int64_t ld16 = 0, ldp = 0, LW = 0;
@@ -355,7 +359,25 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
         const double *part = b->part;
         double *Drow;
         float2 *Drowf = nullptr;                                     // split: the float-pair ring row
-        if (!b->split) {
+        if (b->x7) {
+            const int64_t nb0 = n - n % 64;
+            const int j = (int)(n - nb0);
+            if (j == 0 && nb0 > 0) {
+                if ((rc = hist7_convert(st, b->h7, b->ring, b->Ptot, b->Ptot, nb0))) return rc;
+                if ((rc = far7_launch(st, &b->plan7, b->h7, 0, (int)nb0, b->cfar, (int64_t)64 * b->Ptot, b->Ptot, 1,
+                                      b->ctx->d_flags, b->wcol)))
+                    return rc;
+                k += 2;
+            }
+            if (n >= 1) {                                            // far sums + the block's earlier rows
+                if ((rc = launch_near64(st, b->ring, b->Ptot, 0, j, b->wlag, nb0 > 0 ? b->cfar + (int64_t)j * b->Ptot : nullptr,
+                                        b->part, b->cta_col, b->col_lag, b->LW)))
+                    return rc;
+                ++k;
+                KS = 1;
+            }
+            Drow = b->ring + (int64_t)j * b->Ptot;
+        } else if (!b->split) {
             if (n >= 1) {
                 KS = choose_splits((int)n, b->Ptot);
                 dim3 grid((unsigned)(b->Ptot / 512), (unsigned)KS);
@@ -442,6 +464,7 @@ int fpde_batch_destroy(fpde_batch *b)
         dev_free(b->h3[q]);
         dev_free(b->w3[q]);
     }
+    hist7_free(&b->h7);
     dev_free(b->pA);
     dev_free(b->pW);
     dev_free(b->ringf);
@@ -622,8 +645,11 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
     b->split = split;
     b->LW = (int64_t)max_steps + 64 + 1;
     std::vector<double> hwl;                                           // split: w_c[lag], lag < LW
-    std::vector<int> hwcol;                                            // split: column of each 128-row tile
-    if (split) {
+    std::vector<int> hwcol;                                            // column of each 128-row tile
+    // FP64 runs of more than a block also take the tables (up to 4 GB of weight tiles, 56 KB per column
+    // and distance)
+    const bool want7 = !split && max_steps > 64 && (int64_t)n_cols * ((max_steps - 1) / 64) * 57344 <= (4ll << 30);
+    if (split || want7) {
         hwl.assign((size_t)n_cols * b->LW, 0.0);
         hwcol.assign(tot / 128, 0);
         for (int c = 0; c < n_cols; ++c) {
@@ -651,7 +677,15 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
                 dev_alloc((void **)&b->cols, hc.size() * sizeof(ColInfo)) ||
                 dev_alloc((void **)&b->cta_col, cta_col.size() * sizeof(int)) ||
                 (any_restrict && dev_alloc((void **)&b->col_lag, (size_t)n_cols * sizeof(int)));
-    if (!fail && !split) {
+    if (!fail && want7) {
+        b->x7 = hist7_alloc(&b->h7, &b->plan7, tot, max_steps, n_cols) == FPDE_OK;
+        if (!b->x7) clear_error();                                     // FP64 rows instead (8 bytes against 14)
+    }
+    if (!fail && b->x7) {
+        fail = dev_alloc((void **)&b->ring, (size_t)64 * tb) || dev_alloc((void **)&b->cfar, (size_t)64 * tb) ||
+               dev_alloc((void **)&b->part, tb) || dev_alloc((void **)&b->wlag, hwl.size() * sizeof(double)) ||
+               dev_alloc((void **)&b->wcol, hwcol.size() * sizeof(int));
+    } else if (!fail && !split) {
         fail = dev_alloc((void **)&b->D, (size_t)max_steps * tb) || dev_alloc((void **)&b->part, (size_t)KS_MAX * tb) ||
                dev_alloc((void **)&b->wall, hw.size() * sizeof(double));
     } else if (!fail) {
@@ -698,7 +732,17 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
     cudaMemcpyAsync(b->U0, hU.data(), tb, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(b->Y, 0, tb, st);
     cudaMemsetAsync(b->count, 0, (size_t)n_cols * sizeof(unsigned), st);
-    if (!split) {
+    if (b->x7) {
+        cudaMemsetAsync(b->ring, 0, (size_t)64 * tb, st);
+        cudaMemcpyAsync(b->wlag, hwl.data(), hwl.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(b->wcol, hwcol.data(), hwcol.size() * sizeof(int), cudaMemcpyHostToDevice, st);
+        if ((rc = hist7_weights(st, b->h7, b->wlag, b->LW))) {
+            cudaStreamSynchronize(st);
+            std::string keep = fpde_last_error_string();
+            fpde_batch_destroy(b);
+            return set_error(rc, "%s", keep.c_str());
+        }
+    } else if (!split) {
         cudaMemsetAsync(b->D, 0, (size_t)max_steps * tb, st);
         cudaMemcpyAsync(b->wall, hw.data(), hw.size() * sizeof(double), cudaMemcpyHostToDevice, st);
     } else {

@@ -1169,7 +1169,10 @@ struct fpde_line {
     int sbk = 4;                              // blocks per far super-block (three-slice path)
     int max_lag = INT_MAX;                    // restricted summing: lags above are dropped
     bool split = false;
-    bool b64 = false;                         // FP64 in 64-step blocks (k_far64, k_line_block_spec<Near64>)
+    bool b64 = false;                         // FP64 in 64-step blocks (k_line_block_spec<Near64>)
+    bool x7 = false;                          // ... with the far history in seven bf16 slices (else k_far64 on D)
+    Hist7 h7;
+    FarPlan7 plan7;
     double lam = 0, lamR = 0, kkk0 = 0, AlN = 0;
     double *A = nullptr, *g = nullptr, *al = nullptr, *cf = nullptr, *cb = nullptr;
     double *CF = nullptr, *CB = nullptr, *GG = nullptr;
@@ -1313,7 +1316,7 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     a.A = L->A; a.g = L->g; a.al = L->al; a.cf = L->cf; a.cb = L->cb; a.CB = L->CB; a.GG = L->GG;
     a.lamv = L->lamv; a.eA = L->eA; a.eB = L->eB;
     a.src = L->srcd; a.src_rows = L->src_rows;
-    a.U = L->U; a.ring = L->b64 ? L->D + nb0 * L->P : L->ring; a.cfar = L->cfar; a.KS = KS; a.P = L->P; a.wlag = L->wlag;
+    a.U = L->U; a.ring = L->b64 && !L->x7 ? L->D + nb0 * L->P : L->ring; a.cfar = L->cfar; a.KS = KS; a.P = L->P; a.wlag = L->wlag;
     a.far_ld = far_ld; a.far_row0 = far_row0;
     a.far_pairs = L->x3 ? 1 : 0;
     a.agg = L->agg; a.cflag = L->cflag; a.seq = L->seq;
@@ -1402,14 +1405,26 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
         if (L->b64) {
             const int64_t nb0 = n - n % BLK, t0 = nb0 > L->max_lag ? nb0 - L->max_lag : 0;
             const int j = (int)(n - nb0);
-            if (j == 0 && nb0 > t0) {
-                if ((rc = launch_far64(st, L->D, L->P, L->N, t0, nb0, L->wlag, L->cfar))) return rc;
+            const int64_t kb0 = t0 / BLK * BLK;                      // the oldest 64-step tile in the window
+            const int splits = nb0 == t0 ? 0 : L->x7 ? far_splits((int)((nb0 - kb0) / BLK), L->h7.rows) : 1;
+            if (j == 0 && L->x7 && nb0 > 0) {
+                if ((rc = hist7_convert(st, L->h7, L->ring, L->P, L->N + 1, nb0))) return rc;
+                ++k;
+            }
+            if (j == 0 && splits > 0) {
+                if (L->x7) {
+                    if ((rc = far7_launch(st, &L->plan7, L->h7, (int)kb0, (int)nb0, L->cfar, (int64_t)BLK * L->P, L->P, splits,
+                                          L->ctx->d_flags)))
+                        return rc;
+                } else if ((rc = launch_far64(st, L->D, L->P, L->N, t0, nb0, L->wlag, L->cfar))) {
+                    return rc;
+                }
                 ++k;
             }
             const int nst = (int)std::min<int64_t>(BLK - j, n0 + steps - n);
             ev = L->probe_every > 0 ? probe_begin(L, 2, n, 0.0, 0.0, nst) : nullptr;
             PROBE_REC(ev, 0);
-            if ((rc = line_launch_block(L, st, nb0, j, nst, nb0 > t0 ? 1 : 0, BLK, 0))) return rc;
+            if ((rc = line_launch_block(L, st, nb0, j, nst, splits, BLK, 0))) return rc;
             PROBE_REC(ev, 1);
             ++k;
             n += nst - 1;
@@ -1603,6 +1618,7 @@ int fpde_line_destroy(fpde_line *L)
     for (uint16_t *p : {L->h_hi, L->h_lo, L->w_hi, L->w_lo, L->h3[0], L->h3[1], L->h3[2], L->w3[0], L->w3[1],
                         L->w3[2]})
         dev_free(p);
+    hist7_free(&L->h7);
     dev_free(L->pA);
     dev_free(L->pW);
     dev_free(L->slots);
@@ -1959,9 +1975,16 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
                 (spec && (dev_alloc((void **)&L->sclane, hsl.size() * sizeof(double)) ||
                            dev_alloc((void **)&L->scwarp, hsw.size() * sizeof(double)))) ||
                 dev_alloc((void **)&L->barrier, 2 * sizeof(unsigned));
+    if (!fail && b64 && L->max_steps > BLK) {
+        // the far history in bf16 slices on the tensor cores; where they do not fit (14 bytes per node and
+        // step against 8), FP64 rows and k_far64
+        L->x7 = hist7_alloc(&L->h7, &L->plan7, N + 1, L->max_steps, 1) == FPDE_OK;
+        if (!L->x7) clear_error();
+    }
     if (!fail && !L->split) {
-        fail = dev_alloc((void **)&L->D, (size_t)L->max_steps * L->P * sizeof(double)) ||
-               (b64 ? dev_alloc((void **)&L->cfar, (size_t)BLK * L->P * sizeof(double)) ||
+        fail = (L->x7 ? dev_alloc((void **)&L->ring, (size_t)BLK * L->P * sizeof(double))
+                      : dev_alloc((void **)&L->D, (size_t)L->max_steps * L->P * sizeof(double))) ||
+               (b64 ? dev_alloc((void **)&L->cfar, (size_t)(L->x7 ? FAR_MAX_SPLITS : 1) * BLK * L->P * sizeof(double)) ||
                           dev_alloc((void **)&L->wlag, LW * sizeof(double)) || dev_alloc((void **)&L->cub, nb) ||
                           dev_alloc((void **)&L->cu, nb) || dev_alloc((void **)&L->ccar, 4 * gb)
                     : dev_alloc((void **)&L->part, (size_t)KS_MAX * L->P * sizeof(double)));
@@ -2106,10 +2129,16 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     cudaMemcpyAsync(L->U, u0, (N + 1) * sizeof(double), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(L->barrier, 0, 2 * sizeof(unsigned), st);
     if (!L->split) {
-        cudaMemsetAsync(L->D, 0, (size_t)L->max_steps * L->P * sizeof(double), st);
+        if (L->x7) cudaMemsetAsync(L->ring, 0, (size_t)BLK * L->P * sizeof(double), st);
+        else cudaMemsetAsync(L->D, 0, (size_t)L->max_steps * L->P * sizeof(double), st);
         if (b64) {
-            cudaMemsetAsync(L->cfar, 0, (size_t)BLK * L->P * sizeof(double), st);
+            cudaMemsetAsync(L->cfar, 0, (size_t)(L->x7 ? FAR_MAX_SPLITS : 1) * BLK * L->P * sizeof(double), st);
             cudaMemcpyAsync(L->wlag, wlag.data(), LW * sizeof(double), cudaMemcpyHostToDevice, st);
+        }
+        if (L->x7 && (rc = hist7_weights(st, L->h7, L->wlag, 0))) {
+            std::string keep = fpde_last_error_string();
+            fpde_line_destroy(L);
+            return set_error(rc, "%s", keep.c_str());
         }
     } else if (L->x3) {
         for (int q = 0; q < 3; ++q) {

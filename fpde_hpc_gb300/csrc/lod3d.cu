@@ -1017,6 +1017,10 @@ struct fpde_lod3d {
     float2 *ringf = nullptr, *wff = nullptr;  // the ring and the lag weights as float pairs
     float2 *pre = nullptr;                    // near-history sums of the current 8-step sub-block
     FarPlan3 plan3;
+    // FP64 with the far history of every 64-step block in seven bf16 slices (else the rows of D)
+    bool x7 = false;
+    Hist7 h7;
+    FarPlan7 plan7;
     // Richards problem (desc.richards): coefficients from the solution every step
     bool rich = false;
     int rkform = 0;
@@ -1249,6 +1253,28 @@ static int lod_enqueue(fpde_lod3d *L, cudaStream_t st, int64_t n0, int steps, in
                 KS = 1;
             }
             Drow = L->D + (n & 1) * L->P;
+        } else if (L->x7) {
+            const int64_t nb0 = n - n % 64;
+            const int j = (int)(n - nb0);
+            const int64_t kb0 = nb0 > L->max_lag ? (nb0 - L->max_lag) / 64 * 64 : 0;
+            if (j == 0 && nb0 > 0) {
+                if ((rc = hist7_convert(st, L->h7, L->ring, L->P, L->G, nb0))) return rc;
+                ++k;
+                if (nb0 > kb0) {
+                    if ((rc = far7_launch(st, &L->plan7, L->h7, (int)kb0, (int)nb0, L->cfar, (int64_t)64 * L->P, L->P, 1,
+                                          L->ctx->d_flags)))
+                        return rc;
+                    ++k;
+                }
+            }
+            if (n >= 1) {                                            // far sums + the block's earlier rows
+                const double *far = nb0 > kb0 ? L->cfar + (int64_t)j * L->P : nullptr;
+                const int r0 = std::max<int>(0, (int)std::min<int64_t>(j, j - (int64_t)L->max_lag));
+                if ((rc = launch_near64(st, L->ring, L->P, r0, j, L->wlag, far, L->part))) return rc;
+                ++k;
+                KS = 1;
+            }
+            Drow = L->ring + (int64_t)j * L->P;
         } else if (!L->split) {
             const int64_t t0 = n > L->max_lag ? n - L->max_lag : 0;    // oldest row of the window
             if (n - t0 >= 1) {
@@ -1342,6 +1368,7 @@ int fpde_lod3d_destroy(fpde_lod3d *L)
         cudaStreamSynchronize(L->ctx->stream);
     }
     L->graphs.clear();
+    hist7_free(&L->h7);
     dev_free(L->ringf);
     dev_free(L->wff);
     dev_free(L->pre);
@@ -1497,8 +1524,24 @@ int fpde_lod3d_create(fpde_ctx *ctx, const fpde_lod3d_desc *desc, const double *
         fail = dev_alloc((void **)&L->D, 2 * pbytes) || dev_alloc((void **)&L->part, pbytes) ||
                dev_alloc((void **)&L->H, (size_t)L->series * pbytes);
     } else if (!fail && !L->split) {
-        fail = dev_alloc((void **)&L->D, (size_t)L->max_steps * pbytes) ||
-               dev_alloc((void **)&L->part, (size_t)KS_MAX * pbytes);
+        // blocks of 64 steps, the older history in bf16 slices on the tensor cores, for the passes with
+        // constant coefficients (space-fractional solves stop at a threshold, so their iterates would move
+        // with the sums' rounding); rows of FP64 where the slices do not fit (14 bytes per node and step
+        // against 8)
+        if (!rich && !sfd && !vart && d.max_steps > 64) {
+            L->x7 = hist7_alloc(&L->h7, &L->plan7, L->G, d.max_steps, 1) == FPDE_OK;
+            if (!L->x7) clear_error();
+        }
+        if (L->x7) {
+            const int64_t LW = L->max_steps + 64 + 1;
+            wlag.assign(LW, 0.0);
+            for (int64_t j = 1; j < LW; ++j) wlag[j] = wlag_at(j);
+            fail = dev_alloc((void **)&L->ring, 64 * pbytes) || dev_alloc((void **)&L->cfar, 64 * pbytes) ||
+                   dev_alloc((void **)&L->part, pbytes) || dev_alloc((void **)&L->wlag, LW * sizeof(double));
+        } else {
+            fail = dev_alloc((void **)&L->D, (size_t)L->max_steps * pbytes) ||
+                   dev_alloc((void **)&L->part, (size_t)KS_MAX * pbytes);
+        }
     } else if (!fail) {
         L->rows16 = (L->G + 127) / 128 * 128;
         L->ld16 = ((int64_t)L->max_steps + 63) / 64 * 64;
@@ -1822,6 +1865,14 @@ int fpde_lod3d_create(fpde_ctx *ctx, const fpde_lod3d_desc *desc, const double *
     if (L->series) {
         cudaMemsetAsync(L->D, 0, 2 * pbytes, st);
         cudaMemsetAsync(L->H, 0, (size_t)L->series * pbytes, st);
+    } else if (L->x7) {
+        cudaMemsetAsync(L->ring, 0, 64 * pbytes, st);
+        cudaMemcpyAsync(L->wlag, wlag.data(), wlag.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+        if ((rc = hist7_weights(st, L->h7, L->wlag, 0))) {
+            std::string keep = fpde_last_error_string();
+            fpde_lod3d_destroy(L);
+            return set_error(rc, "%s", keep.c_str());
+        }
     } else if (!L->split) {
         cudaMemsetAsync(L->D, 0, (size_t)L->max_steps * pbytes, st);
     } else {

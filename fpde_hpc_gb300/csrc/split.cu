@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "tc_far.cuh"
 
 namespace fpde {
 
@@ -257,6 +258,235 @@ __global__ void __launch_bounds__(64) k_wgen3(const double *__restrict__ wlag_al
     w0[(int64_t)j * ld + t] = a;
     w1[(int64_t)j * ld + t] = b;
     w2[(int64_t)j * ld + t] = c;
+}
+
+// ---- seven-slice form: x 2^-pe = sum_s a_s 2^-9s, |x| < 2^(pe+8), balanced base-512 digits |a_s| <= 256
+// of the 63-bit integer v = rint(x 2^(54-pe)); each digit is stored as the bf16 value a_s 2^-9s (exact).
+constexpr int PE7_ZERO = -4096;                      // exponent of an all-zero block
+__device__ __forceinline__ int exp7_of_maxbits(unsigned long long mbits)
+{
+    const int ex = (int)((mbits >> 52) & 0x7FF);
+    return ex == 0 ? PE7_ZERO : ex - 1023 + 1 - 8;
+}
+__device__ __forceinline__ void digits7(unsigned long long bits, int pe, uint16_t (&s)[7])
+{
+    const int ex = (int)((bits >> 52) & 0x7FF);
+    long long v = 0;
+    if (ex != 0) {                                   // zero and subnormal values count as 0
+        const long long mant = (long long)((bits & 0xFFFFFFFFFFFFFull) | (1ull << 52));
+        const int r = pe + 1021 - ex;                // >= -9: within 9 binary orders of the largest, exact
+        if (r <= 0) v = mant << min(-r, 9);
+        else if (r < 62) {
+            const long long q = mant >> r, rem = mant & ((1ll << r) - 1), half = 1ll << (r - 1);
+            v = q + ((rem > half || (rem == half && (q & 1))) ? 1 : 0);   // round half to even
+        }
+        if (bits >> 63) v = -v;
+    }
+#pragma unroll
+    for (int k = 6; k >= 1; --k) {
+        const int a = (int)((v + 256) & 511) - 256;
+        v = (v - a) >> 9;
+        s[k] = __bfloat16_as_ushort(__float2bfloat16((float)a * __int_as_float((127 - 9 * k) << 23)));
+    }
+    s[0] = __bfloat16_as_ushort(__float2bfloat16((float)(int)v));
+}
+struct Slices7 { uint16_t *p[7]; };
+
+// Eight adjacent lanes per node, each with 8 of the node's 64 increments (as k_convert3); also the
+// row's largest block exponent so far.
+constexpr int CONV7_LANES = 8, CONV7_ROWS = 64 / CONV7_LANES;
+__global__ void __launch_bounds__(256) k_convert7(const double *__restrict__ rows64, int64_t P, int64_t nvalid, Slices7 out,
+                                                  int64_t ld, int64_t col0, int16_t *__restrict__ pA, int64_t ldp, int blk,
+                                                  int16_t *__restrict__ eA)
+{
+    const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t node = gt / CONV7_LANES;
+    const int part = (int)(gt % CONV7_LANES);
+    const bool live = node < nvalid;
+    const int r0 = part * CONV7_ROWS;
+    unsigned long long v[CONV7_ROWS], mb = 0;
+    const unsigned long long *src = (const unsigned long long *)rows64 + (live ? node : 0);
+#pragma unroll
+    for (int r = 0; r < CONV7_ROWS; ++r) {
+        v[r] = live ? __ldcg(src + (int64_t)(r0 + r) * P) : 0ull;
+        const unsigned long long m0 = v[r] & 0x7FFFFFFFFFFFFFFFull;
+        mb = m0 > mb ? m0 : mb;
+    }
+#pragma unroll
+    for (int o = 1; o < CONV7_LANES; o <<= 1) {
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, mb, o, CONV7_LANES);
+        mb = other > mb ? other : mb;
+    }
+    if (!live) return;
+    const int pe = exp7_of_maxbits(mb);
+    if (part == 0) {
+        pA[node * ldp + blk] = (int16_t)pe;
+        eA[node] = (int16_t)(blk == 0 ? pe : max((int)eA[node], pe));
+    }
+    uint16_t d[CONV7_ROWS][7];
+#pragma unroll
+    for (int k = 0; k < CONV7_ROWS; ++k) digits7(v[k], pe, d[k]);
+    const int64_t o = node * ld + col0 + r0;
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+        uint4 x;
+        x.x = d[0][q] | ((uint32_t)d[1][q] << 16); x.y = d[2][q] | ((uint32_t)d[3][q] << 16);
+        x.z = d[4][q] | ((uint32_t)d[5][q] << 16); x.w = d[6][q] | ((uint32_t)d[7][q] << 16);
+        *(uint4 *)(out.p[q] + o) = x;
+    }
+}
+
+// grid (64 steps j, weight tiles), 64 threads: every distance's tile of step j, two passes (the largest
+// exponent first).
+__global__ void __launch_bounds__(64) k_wgen7(const double *__restrict__ wlag_all, int64_t wstride, Slices7 out, int64_t ldw,
+                                              int n_delta, float *__restrict__ sW, int16_t *__restrict__ eW)
+{
+    __shared__ unsigned long long red[2];
+    const int j = blockIdx.x, c = threadIdx.x;
+    const double *w = wlag_all + (int64_t)blockIdx.y * wstride;
+    auto tile_exp = [&](int d) {
+        unsigned long long m = (unsigned long long)__double_as_longlong(fabs(w[64 * d + j - c]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
+            m = x > m ? x : m;
+        }
+        __syncthreads();
+        if ((c & 31) == 0) red[c >> 5] = m;
+        __syncthreads();
+        return exp7_of_maxbits(red[0] > red[1] ? red[0] : red[1]);
+    };
+    int emax = PE7_ZERO;
+    for (int d = 1; d <= n_delta; ++d) emax = max(emax, tile_exp(d));
+    if (c == 0) eW[(int64_t)blockIdx.y * 64 + j] = (int16_t)emax;
+    for (int d = 1; d <= n_delta; ++d) {
+        const int pe = tile_exp(d);
+        if (c == 0) {
+            const int e = max(pe - emax, -126);
+            sW[((int64_t)blockIdx.y * n_delta + d - 1) * 64 + j] = __int_as_float((e + 127) << 23);
+        }
+        uint16_t s[7];
+        digits7((unsigned long long)__double_as_longlong(w[64 * d + j - c]), pe, s);
+        const int64_t o = ((int64_t)blockIdx.y * 64 + j) * ldw + (int64_t)(d - 1) * 64 + c;
+#pragma unroll
+        for (int q = 0; q < 7; ++q) out.p[q][o] = s[q];
+    }
+}
+
+// Near history of step j of a 64-step block in FP64: S[i] = init[i] + sum_{r0 <= r < j} w[j - r] D_r[i] from the
+// block's FP64 rows (init: the far sums, may be null). Two nodes per thread; the rows are read again by
+// every later step of the block, so they are left in L2. FP64-pipe bound: one multiply-add per row.
+__global__ void __launch_bounds__(256) k_near64(const double2 *__restrict__ rows, int64_t P2, int r0, int j,
+                                                const double *__restrict__ wlag, int64_t wstride,
+                                                const int *__restrict__ cta_col, const int *__restrict__ col_lag,
+                                                const double2 *__restrict__ init, double2 *__restrict__ S)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P2) return;
+    const double *w = wlag;
+    if (cta_col) {                                   // a 512-node group's column: its weights and window
+        const int c = cta_col[blockIdx.x];
+        w += (int64_t)c * wstride;
+        if (col_lag) r0 = max(r0, j - col_lag[c]);
+    }
+    double2 s = init ? __ldcs(init + i) : make_double2(0.0, 0.0);
+    int r = r0;
+    for (; r + 8 <= j; r += 8) {
+        double2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldcg(rows + (int64_t)(r + u) * P2 + i);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const double x = __ldg(w + (j - r - u));
+            s.x = fma(x, v[u].x, s.x);
+            s.y = fma(x, v[u].y, s.y);
+        }
+    }
+    if (r < j) {                                     // the last rows, loaded together
+        double2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = r + u < j ? __ldcg(rows + (int64_t)(r + u) * P2 + i) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (r + u < j) {
+                const double x = __ldg(w + (j - r - u));
+                s.x = fma(x, v[u].x, s.x);
+                s.y = fma(x, v[u].y, s.y);
+            }
+        }
+    }
+    S[i] = s;
+}
+
+int launch_near64(cudaStream_t st, const double *rows, int64_t P, int r0, int j, const double *wlag, const double *init,
+                  double *S, const int *cta_col, const int *col_lag, int64_t wstride)
+{
+    k_near64<<<(unsigned)((P / 2 + 255) / 256), 256, 0, st>>>((const double2 *)rows, P / 2, r0, j, wlag, wstride, cta_col,
+                                                              col_lag, (const double2 *)init, (double2 *)S);
+    FPDE_LAUNCHED(1);
+    return FPDE_OK;
+}
+
+int hist7_alloc(Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles)
+{
+    h->rows = (nodes + 127) / 128 * 128;
+    h->n_delta = (max_steps - 1) / 64;
+    h->ld = h->ldw = (int64_t)h->n_delta * 64;
+    h->ldp = h->n_delta;
+    h->w_tiles = w_tiles;
+    bool fail = false;
+    for (int q = 0; q < 7 && !fail; ++q)
+        fail = dev_alloc((void **)&h->a[q], (size_t)h->rows * h->ld * 2) ||
+               dev_alloc((void **)&h->w[q], (size_t)w_tiles * 64 * h->ldw * 2);
+    fail = fail || dev_alloc((void **)&h->pA, (size_t)h->rows * h->ldp * sizeof(int16_t)) ||
+           dev_alloc((void **)&h->eA, (size_t)h->rows * sizeof(int16_t)) ||
+           dev_alloc((void **)&h->eW, (size_t)w_tiles * 64 * sizeof(int16_t)) ||
+           dev_alloc((void **)&h->sW, (size_t)w_tiles * h->n_delta * 64 * sizeof(float));
+    int rc = fail ? FPDE_ERR_NOMEM : FPDE_OK;
+    if (!rc) {
+        const void *a[7], *w[7];
+        for (int q = 0; q < 7; ++q) { a[q] = h->a[q]; w[q] = h->w[q]; }
+        rc = far_plan7_init(p, a, h->rows, h->ld, w, h->ldw, w_tiles);
+    }
+    // rows past the nodes are never converted: their (unused) sums only need readable exponents
+    if (!rc && (cudaMemset(h->pA, 0, (size_t)h->rows * h->ldp * sizeof(int16_t)) != cudaSuccess ||
+                cudaMemset(h->eA, 0, (size_t)h->rows * sizeof(int16_t)) != cudaSuccess))
+        rc = FPDE_ERR_CUDA;
+    if (rc) hist7_free(h);
+    return rc;
+}
+
+void hist7_free(Hist7 *h)
+{
+    for (int q = 0; q < 7; ++q) {
+        dev_free(h->a[q]);
+        dev_free(h->w[q]);
+    }
+    dev_free(h->pA);
+    dev_free(h->eA);
+    dev_free(h->eW);
+    dev_free(h->sW);
+    *h = Hist7();
+}
+
+int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t wstride)
+{
+    Slices7 o;
+    for (int q = 0; q < 7; ++q) o.p[q] = h.w[q];
+    k_wgen7<<<dim3(64, (unsigned)h.w_tiles), 64, 0, st>>>(wlag, wstride, o, h.ldw, h.n_delta, h.sW, h.eW);
+    FPDE_LAUNCHED(1);
+    return FPDE_OK;
+}
+
+int hist7_convert(cudaStream_t st, const Hist7 &h, const double *rows64, int64_t P, int64_t nvalid, int64_t n0)
+{
+    Slices7 o;
+    for (int q = 0; q < 7; ++q) o.p[q] = h.a[q];
+    const int64_t threads = nvalid * CONV7_LANES;
+    k_convert7<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(rows64, P, nvalid, o, h.ld, n0 - 64, h.pA, h.ldp,
+                                                                  (int)(n0 / 64) - 1, h.eA);
+    FPDE_LAUNCHED(1);
+    return FPDE_OK;
 }
 
 int launch_block_prep3(cudaStream_t st, const SplitPrep3 &p, int64_t n0, bool weights)

@@ -579,6 +579,256 @@ __global__ void __launch_bounds__(THREADS3, 1)
     }
 }
 
+// ------------------------------------------------------------------------------------
+// FP64 form (seven bf16 slices per operand). A[i][t] = 2^pA[i][t/64] sum_s a_s 2^-9s with integer digits
+// |a_s| <= 256 (base 512, balanced: 63 bits from a row block's largest value down), W likewise per (step,
+// 64-lag tile). This is the scheme of splitting FP64 operands into slices whose products a lower-
+// precision matrix unit sums without rounding (Ozaki, Ogita, Oishi, Rump 2012). Per 64-column k-tile the
+// products of level L = s + t,
+//     X_L = sum a_s w_t 2^-9L,   |X_L| 2^9L <= (L + 1) 2^22,
+// are exact in FP32 accumulators for L = 0 .. 3 (and for 4 unless its digits conspire: the bound is 1.25
+// 2^24); levels 5 and 6 share one (rounded 2^-60 below X_0) and higher ones are dropped (2^-60 of a
+// k-tile's largest term each): 28 products. With six slices and 21 products (levels 0 to 5) the sums were
+// 1.5 times further from exact ones than the FP64 chain's, with six and 26 products 1.1 to 1.2 times (small
+// increments beside a block's largest lost bits). The epilogue adds the six accumulators into three
+// floats (h, m, l) per output by error-free sums, and the result leaves as FP64. Its error against exact sums is below that of an FP64 multiply-add chain
+// over the same terms, whose rounding grows with the number of terms.
+// What bounds it: shared memory. A k-tile of 128 rows x 64 steps takes 112 MMAs (M = 128, N = 64, K = 16)
+// that read 6 KB each next to 168 KB of TMA writes: 6,560 cycles at 128 B per cycle; the tensor
+// cores' own time is 3,600, the fold's about 4,000 on the FP32 pipes. The FP64 pipe would take 320,000.
+// Operands come as 32-column half tiles (64-byte swizzle, two 84 KB stages); the six accumulators
+// of 64 columns rotate through eight TMEM slots, the widest level first, so that a k-tile's MMAs start
+// while the one before is folded.
+constexpr int F7_BK = 32;
+constexpr int F7_A = BM * F7_BK * 2, F7_W = BN * F7_BK * 2;   // one slice of a stage: 8 KB, 4 KB
+constexpr int F7_STAGE = 7 * (F7_A + F7_W);                   // 84 KB
+constexpr int F7_STAGES = 2, F7_SLOTS = 8, F7_LEV = 6;
+constexpr int F7_SMEM = 1024 + F7_STAGES * F7_STAGE + 256;
+
+struct __align__(64) FarMaps7 {
+    CUtensorMap a[7], w[7];
+};
+
+__device__ __forceinline__ uint64_t sdesc_sw64(uint32_t saddr)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);        // start address
+    d |= (uint64_t)1 << 16;                          // leading byte offset (unused for swizzled K-major)
+    d |= (uint64_t)(512 >> 4) << 32;                 // stride byte offset: 8 rows x 64 B
+    d |= (uint64_t)1 << 46;                          // descriptor version (tcgen05)
+    d |= (uint64_t)4 << 61;                          // SWIZZLE_64B
+    return d;
+}
+
+// (a, e): a + b exactly
+__device__ __forceinline__ float two_sum(float &a, float b)
+{
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    a = s;
+    return e;
+}
+// x 2^e for a finite x (e in a range where 2^e is normal), exact unless the result leaves FP64's range
+__device__ __forceinline__ double scale_f64(double x, int e)
+{
+    const int hi = __double2hiint(x), f = (hi >> 20) & 0x7FF;
+    if (f + e > 0 && f + e < 0x7FF && f > 0 && f < 0x7FF) return __hiloint2double(hi + e * (1 << 20), __double2loint(x));
+    return scalbn(x, e);
+}
+
+struct Far7Args {
+    double *C;
+    int64_t ldc_split, ldc_col, rows;
+    int kt_begin, kt_end, kt_per, n_split;           // k-tiles [kt_begin, kt_end); the block's index is kt_end
+    const int16_t *pA;                               // [rows][ldp]
+    const int16_t *eA;                               // [rows]: largest pA of the row so far
+    int64_t ldp;
+    const float *sW;                                 // [weight tiles][n_delta][64]: 2^(pW - eW)
+    const int16_t *eW;                               // [weight tiles][64]: largest pW of the step
+    int n_delta;
+    const int *wcol;
+    uint32_t idesc;
+    unsigned *flags;
+};
+
+__global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__ FarMaps7 maps, const Far7Args p)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t *bars = (uint64_t *)(smem + F7_STAGES * F7_STAGE);
+    uint64_t *full = bars, *empty = bars + F7_STAGES, *sfull = bars + 2 * F7_STAGES, *sempty = sfull + F7_SLOTS;
+    uint64_t *mma_done = sempty + F7_SLOTS;
+    volatile uint32_t *tmem_slot = (volatile uint32_t *)(mma_done + 1);
+    volatile int *abort_s = (volatile int *)(mma_done + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_items = (int)(p.rows / BM) * p.n_split;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < F7_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < F7_SLOTS; ++s) { mbar_init(&sfull[s], 1); mbar_init(&sempty[s], 256); }
+        mbar_init(mma_done, 1);
+        *abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32((const void *)tmem_slot)),
+                     "r"(F7_SLOTS * BN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    auto k_range = [&](int item, int &mt, int &ks, int &k0, int &k1) {
+        mt = item / p.n_split;
+        ks = item % p.n_split;
+        k0 = p.kt_begin + ks * p.kt_per;
+        k1 = min(k0 + p.kt_per, p.kt_end);
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {                                   // TMA producer: half tiles
+            int g = 0, mt, ks, k0, k1;
+            bool ok = true;
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                k_range(item, mt, ks, k0, k1);
+                const int yw = (p.wcol ? p.wcol[mt] : 0) * BN;
+                for (int h = 2 * k0; h < 2 * k1; ++h, ++g) {
+                    const int s = g % F7_STAGES;
+                    if (!mbar_wait(&empty[s], ((uint32_t)(g / F7_STAGES) & 1u) ^ 1u, p.flags, abort_s)) { ok = false; break; }
+                    uint8_t *st = smem + s * F7_STAGE;
+                    mbar_expect_tx(&full[s], F7_STAGE);
+                    // the weights depend on the distance between the block and the k-tile only
+                    const int xa = h * F7_BK, xw = (p.kt_end - (h >> 1) - 1) * BK + (h & 1) * F7_BK;
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) tma_load_2d(st + q * F7_A, &maps.a[q], xa, mt * BM, &full[s]);
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) tma_load_2d(st + 7 * F7_A + q * F7_W, &maps.w[q], xw, yw, &full[s]);
+                }
+            }
+            for (int it = (g > F7_STAGES ? g - F7_STAGES : 0); it < g; ++it) {   // own copies in flight
+                const unsigned long long t0 = gtimer();
+                while (!mbar_try_wait(&full[it % F7_STAGES], (uint32_t)(it / F7_STAGES) & 1u) && gtimer() - t0 < WAIT_NS) {}
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {                                   // MMA issuer
+            int g = 0, c = 0, mt, ks, k0, k1;              // half tiles, TMEM slots used so far
+            bool ok = true;
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                k_range(item, mt, ks, k0, k1);
+                for (int h = 2 * k0; h < 2 * k1 && ok && !*abort_s; ++h, ++g) {
+                    const int s = g % F7_STAGES;
+                    if (!mbar_wait(&full[s], (uint32_t)(g / F7_STAGES) & 1u, p.flags, abort_s)) { ok = false; break; }
+                    tc_fence_after();
+                    const bool second = h & 1;
+                    const uint64_t dst = sdesc_sw64(smem_u32(smem + s * F7_STAGE));
+                    const uint32_t dlo = (uint32_t)dst, dhi = (uint32_t)(dst >> 32);
+                    // accumulator 0: levels 6 and 5; 1 .. 5: levels 4 .. 0
+#pragma unroll
+                    for (int l = 0; l < F7_LEV; ++l) {
+                        const int sl = (c + l) % F7_SLOTS;
+                        if (!second) {
+                            if (!mbar_wait(&sempty[sl], ((uint32_t)((c + l) / F7_SLOTS) & 1u) ^ 1u, p.flags, abort_s)) { ok = false; break; }
+                            tc_fence_after();
+                        }
+                        const uint32_t x = tmem + (uint32_t)(sl * BN);
+                        bool acc = second;
+#pragma unroll
+                        for (int lev = l == 0 ? 6 : 5 - l; lev >= 5 - l; --lev)
+#pragma unroll
+                            for (int sa = 0; sa <= lev; ++sa)
+#pragma unroll
+                                for (int k = 0; k < F7_BK / 16; ++k) {
+                                    const uint32_t o = dlo + (uint32_t)(k * 2);
+                                    umma_lo(x, o + (uint32_t)(sa * F7_A >> 4),
+                                            o + (uint32_t)((7 * F7_A + (lev - sa) * F7_W) >> 4), dhi, p.idesc, acc ? 1u : 0u);
+                                    acc = true;
+                                }
+                        if (second) umma_commit(&sfull[sl]);
+                    }
+                    umma_commit(&empty[s]);
+                    if (second) c += F7_LEV;
+                }
+            }
+            umma_commit(mma_done);
+            const unsigned long long t0 = gtimer();
+            while (!mbar_try_wait(mma_done, 0) && gtimer() - t0 < WAIT_NS) {}
+        }
+    } else {
+        // 8 epilogue warps: TMEM lane quadrant warp % 4, columns c0 .. c0 + 31
+        const int q = warp & 3, c0 = 32 * ((warp - 2) >> 2);
+        int c = 0, mt, ks, k0, k1;
+        bool ok = true;
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            k_range(item, mt, ks, k0, k1);
+            const int64_t row = (int64_t)mt * BM + q * 32 + lane;
+            const int wt = p.wcol ? p.wcol[mt] : 0;
+            const int16_t *pAr = p.pA + row * p.ldp;
+            const int eA = p.eA[row];
+            const float *sW = p.sW + (int64_t)wt * p.n_delta * BN + c0;
+            float hh[32], mm[32], ll[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) hh[j] = mm[j] = ll[j] = 0.f;
+            int e_nx = k0 < k1 ? (int)pAr[k0] : 0;
+            for (int kt = k0; kt < k1 && ok; ++kt, c += F7_LEV) {
+                const float sa = pow2f(max(e_nx - eA, -127));
+                if (kt + 1 < k1) e_nx = pAr[kt + 1];
+                const float4 *w4 = reinterpret_cast<const float4 *>(sW + (int64_t)(p.kt_end - kt - 1) * BN);
+#pragma unroll
+                for (int l = 0; l < F7_LEV; ++l) {
+                    const int sl = (c + l) % F7_SLOTS;
+                    if (!mbar_wait(&sfull[sl], (uint32_t)((c + l) / F7_SLOTS) & 1u, p.flags, abort_s)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(sl * BN + c0);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        float v[16];
+                        tmem_ld16(ta + 16 * b, v);
+                        float ws[16];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const float4 x = __ldg(w4 + 4 * b + k);
+                            ws[4 * k] = x.x; ws[4 * k + 1] = x.y; ws[4 * k + 2] = x.z; ws[4 * k + 3] = x.w;
+                        }
+                        tmem_ld_wait();
+                        if (b == 1) {
+                            tc_fence_before();
+                            mbar_arrive(&sempty[sl]);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) {
+                            const int j = 16 * b + k;
+                            const float x = v[k] * (sa * ws[k]);          // exact: powers of two
+                            if (l <= 3) {                                 // levels 6 + 5, 4, 3, 2
+                                ll[j] += two_sum(mm[j], x);
+                            } else {                                      // levels 1, 0
+                                const float e = two_sum(hh[j], x);
+                                ll[j] += two_sum(mm[j], e);
+                            }
+                        }
+                    }
+                }
+            }
+            if (ok) {
+                const int16_t *eW = p.eW + (int64_t)wt * BN + c0;
+                double *out = p.C + (int64_t)ks * p.ldc_split + row + (int64_t)c0 * p.ldc_col;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const double d = f2d_bits(hh[j]) + (f2d_bits(mm[j]) + f2d_bits(ll[j]));
+                    out[(int64_t)j * p.ldc_col] = scale_f64(d, eA + (int)__ldg(eW + j));
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(F7_SLOTS * BN));
+    }
+}
+
 // ---------------------------------------------------------------- host side
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -599,8 +849,8 @@ static EncodeTiledFn encode_fn()
     return fn;
 }
 
-// 2D tensor map over a row-major [rows][cols] array of 16-bit values, box 64 cols x box_rows.
-static int make_map(CUtensorMap *tm, const void *base, int64_t rows, int64_t cols, int box_rows)
+// 2D tensor map over a row-major [rows][cols] array of 16-bit values, box 64 (or 32) cols x box_rows.
+static int make_map(CUtensorMap *tm, const void *base, int64_t rows, int64_t cols, int box_rows, int box_cols = BK)
 {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return set_error(FPDE_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
@@ -608,10 +858,11 @@ static int make_map(CUtensorMap *tm, const void *base, int64_t rows, int64_t col
         return set_error(FPDE_ERR_ARG, "tensor map: row pitch and base must be 16-byte aligned");
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)(cols * 2)};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     cuuint32_t es[2] = {1, 1};
     CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(base), dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == BK ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(FPDE_ERR_ARG, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return FPDE_OK;
@@ -699,6 +950,48 @@ int far3_launch(cudaStream_t st, const FarPlan3 *p, int k_cols, double *C, int64
         tc::k_far_tc3<1><<<(unsigned)grid, tc::THREADS3, tc::Far3Cfg<1>::SMEM, st>>>(
             *m, C, ldc_split, ldc_col, p->rows, kt_begin, kt_total, kt_per, splits, p->idesc, pA, pW, ldp, wcol,
             n_sets, grp0, ldc_grp, flags);
+    FPDE_LAUNCHED(1);
+    return FPDE_OK;
+}
+
+int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int64_t lda, const void *const w[7], int64_t ldw,
+                   int w_tiles)
+{
+    if (rows % tc::BM != 0 || lda % tc::BK != 0 || ldw % tc::BK != 0)
+        return set_error(FPDE_ERR_ARG, "far contraction: rows must be a multiple of 128, pitches of 64");
+    static_assert(sizeof(tc::FarMaps7) <= sizeof(p->maps), "map storage");
+    tc::FarMaps7 *m = (tc::FarMaps7 *)p->maps;
+    int rc;
+    for (int q = 0; q < 7; ++q)
+        if ((rc = tc::make_map(&m->a[q], a[q], rows, lda, tc::BM, tc::F7_BK)) ||
+            (rc = tc::make_map(&m->w[q], w[q], (int64_t)tc::BN * w_tiles, ldw, tc::BN, tc::F7_BK)))
+            return rc;
+    p->rows = rows;
+    p->idesc = tc::idesc_f16(1, tc::BM, tc::BN);
+    cudaError_t e = smem_opt_in((const void *)tc::k_far_tc7, tc::F7_SMEM);
+    if (e != cudaSuccess) return set_error(FPDE_ERR_CUDA, "far kernel smem attribute: %s", cudaGetErrorString(e));
+    return FPDE_OK;
+}
+
+int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_begin, int k_cols, double *C, int64_t ldc_split,
+                int64_t ldc_col, int splits, unsigned *flags, const int *wcol)
+{
+    if (k_cols % tc::BK != 0 || k_begin % tc::BK != 0 || k_begin < 0 || k_begin > k_cols)
+        return set_error(FPDE_ERR_ARG, "far contraction: K range must be in multiples of 64");
+    if (k_cols == k_begin) return FPDE_OK;
+    tc::Far7Args a;
+    a.kt_begin = k_begin / tc::BK;
+    a.kt_end = k_cols / tc::BK;
+    if (a.kt_end - a.kt_begin > h.n_delta) return set_error(FPDE_ERR_ARG, "far contraction: weight tiles out of range");
+    splits = std::max(1, std::min(splits, FAR_MAX_SPLITS));
+    a.kt_per = (a.kt_end - a.kt_begin + splits - 1) / splits;      // every split is written, possibly with zeros
+    a.n_split = splits;
+    a.C = C; a.ldc_split = ldc_split; a.ldc_col = ldc_col; a.rows = p->rows;
+    a.pA = h.pA; a.eA = h.eA; a.ldp = h.ldp; a.sW = h.sW; a.eW = h.eW; a.n_delta = h.n_delta; a.wcol = wcol;
+    a.idesc = p->idesc; a.flags = flags;
+    const int64_t items = (p->rows / tc::BM) * splits;
+    const unsigned grid = (unsigned)std::min<int64_t>(items, device_sm_count());
+    tc::k_far_tc7<<<grid, tc::THREADS3, tc::F7_SMEM, st>>>(*(const tc::FarMaps7 *)p->maps, a);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }

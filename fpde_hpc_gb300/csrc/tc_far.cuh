@@ -48,6 +48,41 @@ int far3_launch(cudaStream_t st, const FarPlan3 *p, int k_cols, double *C, int64
                 int splits, const int8_t *pA, const float *pW, int64_t ldp, unsigned *flags,
                 const int *wcol = nullptr, int k_begin = 0, int n_grp = 1, int grp0 = 0);
 
+// FP64 form (seven slices of 9 bits; tc_far.cu): slices, exponents and weight tables of a history. The
+// weights w[n0 + j - t] of a block at n0 depend on its distance from a k-tile only, so their tiles
+// (distance 1 .. n_delta blocks) are formed once.
+struct Hist7 {
+    uint16_t *a[7] = {};   // [rows][ld] node-major slices
+    uint16_t *w[7] = {};   // [w_tiles 64][ldw]: column (d-1) 64 + c: lag 64 d + j - c
+    int16_t *pA = nullptr, *eA = nullptr;      // [rows][ldp] exponents per (node, block); [rows] largest so far
+    int16_t *eW = nullptr;                     // [w_tiles][64] largest exponent of the step's weights
+    float *sW = nullptr;                       // [w_tiles][n_delta][64] 2^(exponent - eW)
+    int64_t rows = 0, ld = 0, ldw = 0, ldp = 0;
+    int n_delta = 0, w_tiles = 1;
+};
+struct FarPlan7 {
+    alignas(64) unsigned char maps[14 * 128];
+    int64_t rows = 0;
+    uint32_t idesc = 0;
+};
+// Allocate for `nodes` rows and max_steps columns (FPDE_ERR_NOMEM leaves nothing behind), free.
+int hist7_alloc(Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles);
+void hist7_free(Hist7 *h);
+// Weight tiles from w[lag] (w_tiles rows of wstride values, lag < 64 n_delta + 64), once.
+int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t wstride);
+// The finished block [n0 - 64, n0) of increments (64 rows of P) into the slices.
+int hist7_convert(cudaStream_t st, const Hist7 &h, const double *rows64, int64_t P, int64_t nvalid, int64_t n0);
+// S[i] = init[i] + sum_{r0 <= r < j} w[j - r] rows_r[i] in FP64 (init may be null; per-column weights and
+// windows with cta_col and col_lag).
+int launch_near64(cudaStream_t st, const double *rows, int64_t P, int r0, int j, const double *wlag, const double *init,
+                  double *S, const int *cta_col = nullptr, const int *col_lag = nullptr, int64_t wstride = 0);
+int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int64_t lda, const void *const w[7], int64_t ldw,
+                   int w_tiles);
+// C[split ldc_split + j ldc_col + row] = sum over the split's share of columns [k_begin, k_cols) of
+// A[row][t] w[k_cols + j - t], j < 64, in FP64.
+int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_begin, int k_cols, double *C, int64_t ldc_split,
+                int64_t ldc_col, int splits, unsigned *flags, const int *wcol = nullptr);
+
 // float -> double from the bits (integer instructions only; exact for every float).
 __device__ __forceinline__ double f2d_bits(float x)
 {
