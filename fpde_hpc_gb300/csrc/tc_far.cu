@@ -620,11 +620,57 @@ __device__ __forceinline__ uint64_t sdesc_sw64(uint32_t saddr)
     return d;
 }
 
-// (a, e): a + b exactly
-__device__ __forceinline__ float two_sum(float &a, float b)
+// Two floats in one 64-bit register: one instruction per operation on both (the fold is bound by issue
+// slots: 8 warps x 32 columns x about 60 operations per k-tile).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float x, float y)
 {
-    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a += b, returns the rounding error (TwoSum); and with b = v sc exactly (sc a power of two).
+__device__ __forceinline__ f32x2 two_sum2(f32x2 &a, f32x2 b)
+{
+    const f32x2 s = add2(a, b), nb = sub2(a, s);        // -(what of b went into s)
+    const f32x2 e = add2(sub2(a, add2(s, nb)), add2(b, nb));
+    a = s;
+    return e;
+}
+__device__ __forceinline__ f32x2 two_sum2(f32x2 &a, f32x2 v, f32x2 sc)
+{
+    const f32x2 s = fma2(v, sc, a), nb = sub2(a, s);
+    const f32x2 e = add2(sub2(a, add2(s, nb)), fma2(v, sc, nb));
     a = s;
     return e;
 }
@@ -767,45 +813,41 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
             const int16_t *pAr = p.pA + row * p.ldp;
             const int eA = p.eA[row];
             const float *sW = p.sW + (int64_t)wt * p.n_delta * BN + c0;
-            float hh[32], mm[32], ll[32];
+            f32x2 hh[16], mm[16], ll[16];                     // columns 2j, 2j + 1
 #pragma unroll
-            for (int j = 0; j < 32; ++j) hh[j] = mm[j] = ll[j] = 0.f;
+            for (int j = 0; j < 16; ++j) hh[j] = mm[j] = ll[j] = 0ull;
             int e_nx = k0 < k1 ? (int)pAr[k0] : 0;
             for (int kt = k0; kt < k1 && ok; ++kt, c += F7_LEV) {
-                const float sa = pow2f(max(e_nx - eA, -127));
+                const float sa1 = pow2f(max(e_nx - eA, -127));
+                const f32x2 sa = pack2(sa1, sa1);
                 if (kt + 1 < k1) e_nx = pAr[kt + 1];
                 const float4 *w4 = reinterpret_cast<const float4 *>(sW + (int64_t)(p.kt_end - kt - 1) * BN);
-#pragma unroll
+                // not unrolled: the levels share two bodies (into m, into h), which have to stay in the
+                // instruction cache (unrolled, the warps waited for instructions most of the time)
+#pragma unroll 1
                 for (int l = 0; l < F7_LEV; ++l) {
                     const int sl = (c + l) % F7_SLOTS;
                     if (!mbar_wait(&sfull[sl], (uint32_t)((c + l) / F7_SLOTS) & 1u, p.flags, abort_s)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(sl * BN + c0);
+                    float v[32];
+                    tmem_ld16(ta, v);
+                    tmem_ld16(ta + 16, v + 16);
+                    tmem_ld_wait();
+                    tc_fence_before();
+                    mbar_arrive(&sempty[sl]);
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        float v[16];
-                        tmem_ld16(ta + 16 * b, v);
-                        float ws[16];
+                    for (int k = 0; k < 8; ++k) {
+                        const float4 x = __ldg(w4 + k);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const float4 x = __ldg(w4 + 4 * b + k);
-                            ws[4 * k] = x.x; ws[4 * k + 1] = x.y; ws[4 * k + 2] = x.z; ws[4 * k + 3] = x.w;
-                        }
-                        tmem_ld_wait();
-                        if (b == 1) {
-                            tc_fence_before();
-                            mbar_arrive(&sempty[sl]);
-                        }
-#pragma unroll
-                        for (int k = 0; k < 16; ++k) {
-                            const int j = 16 * b + k;
-                            const float x = v[k] * (sa * ws[k]);          // exact: powers of two
-                            if (l <= 3) {                                 // levels 6 + 5, 4, 3, 2
-                                ll[j] += two_sum(mm[j], x);
-                            } else {                                      // levels 1, 0
-                                const float e = two_sum(hh[j], x);
-                                ll[j] += two_sum(mm[j], e);
-                            }
+                        for (int u = 0; u < 2; ++u) {
+                            const int j = 2 * k + u;
+                            const f32x2 sc = mul2(sa, u ? pack2(x.z, x.w) : pack2(x.x, x.y));   // powers of two
+                            const f32x2 y = pack2(v[2 * j], v[2 * j + 1]);
+                            if (l <= 3)                                       // levels 6 + 5, 4, 3, 2
+                                ll[j] = add2(ll[j], two_sum2(mm[j], y, sc));
+                            else                                              // levels 1, 0
+                                ll[j] = add2(ll[j], two_sum2(mm[j], two_sum2(hh[j], y, sc)));
                         }
                     }
                 }
@@ -814,9 +856,12 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
                 const int16_t *eW = p.eW + (int64_t)wt * BN + c0;
                 double *out = p.C + (int64_t)ks * p.ldc_split + row + (int64_t)c0 * p.ldc_col;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const double d = f2d_bits(hh[j]) + (f2d_bits(mm[j]) + f2d_bits(ll[j]));
-                    out[(int64_t)j * p.ldc_col] = scale_f64(d, eA + (int)__ldg(eW + j));
+                for (int j = 0; j < 16; ++j) {
+                    const float2 h = unpack2(hh[j]), m = unpack2(mm[j]), l = unpack2(ll[j]);
+                    const double d0 = f2d_bits(h.x) + (f2d_bits(m.x) + f2d_bits(l.x));
+                    const double d1 = f2d_bits(h.y) + (f2d_bits(m.y) + f2d_bits(l.y));
+                    out[(int64_t)(2 * j) * p.ldc_col] = scale_f64(d0, eA + (int)__ldg(eW + 2 * j));
+                    out[(int64_t)(2 * j + 1) * p.ldc_col] = scale_f64(d1, eA + (int)__ldg(eW + 2 * j + 1));
                 }
             }
         }
