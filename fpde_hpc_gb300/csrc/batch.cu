@@ -396,7 +396,7 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
                 splits = far_splits((int)(nb0 / 64), b->Ptot);
                 if (j == 0) {                                        // far history t < nb0, per column
                     SplitPrep3 sp;
-                    sp.ring = b->ring; sp.P = b->Ptot; sp.nvalid = b->Ptot; sp.ld = b->ld16; sp.wlag = b->wlag;
+                    sp.ring = b->ring; sp.P = b->Ptot; sp.nvalid = b->Ptot; sp.ld = b->ld16; sp.rows = b->Ptot; sp.wlag = b->wlag;
                     for (int q = 0; q < 3; ++q) { sp.hist[q] = b->h3[q]; sp.w[q] = b->w3[q]; }
                     sp.pA = b->pA; sp.pW = b->pW; sp.ldp = b->ldp; sp.ncols = b->n_cols; sp.wstride = b->LW;
                     if ((rc = launch_block_prep3(st, sp, nb0))) return rc;

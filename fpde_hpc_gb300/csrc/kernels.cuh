@@ -41,14 +41,14 @@ struct SplitPrep {
 // next contraction (K = n0).
 int launch_block_prep(cudaStream_t st, const SplitPrep &p, int64_t n0);
 
-// Exact three-slice form: history slices and per-(node, block) exponents, weight slices and
-// per-(step, k-tile) exponents.
+// Exact three-slice form, tile-major: history slices [ld/64][rows][64] with exponents pA [k-tile][rows],
+// weight slices [ld/64][64 n_grp ncols][64] with scales pW [k-tile][64 n_grp ncols].
 struct SplitPrep3 {
     const double *ring = nullptr;
     int64_t P = 0, nvalid = 0;
     uint16_t *hist[3] = {nullptr, nullptr, nullptr};
     uint16_t *w[3] = {nullptr, nullptr, nullptr};
-    int64_t ld = 0;
+    int64_t ld = 0, rows = 0;            // columns, rows (nodes rounded up to 128) of the slices
     int8_t *pA = nullptr;                // per (node, k-tile) exponents
     float *pW = nullptr;                 // per (step, k-tile) scales 2^e of the weight tiles
     int64_t ldp = 0;

@@ -1487,7 +1487,7 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
                     // convert the finished block; at a super-block start also the weight slices of
                     // all its steps (the first super-block's later blocks need them too)
                     SplitPrep3 sp;
-                    sp.ring = L->ring; sp.P = L->P; sp.nvalid = nodes_hist; sp.ld = L->ld16; sp.wlag = L->wlag;
+                    sp.ring = L->ring; sp.P = L->P; sp.nvalid = nodes_hist; sp.ld = L->ld16; sp.rows = L->rows16; sp.wlag = L->wlag;
                     for (int q = 0; q < 3; ++q) { sp.hist[q] = L->h3[q]; sp.w[q] = L->w3[q]; }
                     sp.pA = L->pA; sp.pW = L->pW; sp.ldp = L->ldp; sp.n_grp = sbk;
                     if ((rc = launch_block_prep3(st, sp, nb0, m == 0))) return rc;

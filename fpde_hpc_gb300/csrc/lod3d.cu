@@ -1303,7 +1303,7 @@ static int lod_enqueue(fpde_lod3d *L, cudaStream_t st, int64_t n0, int steps, in
                 splits = far_kt > 0 ? far_splits(far_kt, L->rows16) : 0;
                 if (j == 0) {                                        // far history t < nb0
                     SplitPrep3 sp;
-                    sp.ring = L->ring; sp.P = L->P; sp.nvalid = L->G; sp.ld = L->ld16; sp.wlag = L->wlag;
+                    sp.ring = L->ring; sp.P = L->P; sp.nvalid = L->G; sp.ld = L->ld16; sp.rows = L->rows16; sp.wlag = L->wlag;
                     for (int q = 0; q < 3; ++q) { sp.hist[q] = L->h3[q]; sp.w[q] = L->w3[q]; }
                     sp.pA = L->pA; sp.pW = L->pW; sp.ldp = L->ldp;
                     if ((rc = launch_block_prep3(st, sp, nb0))) return rc;

@@ -181,8 +181,8 @@ __device__ __forceinline__ int exp_of_maxbits(unsigned long long mbits)
 constexpr int CONV_LANES = 4, CONV_ROWS = 64 / CONV_LANES;
 __global__ void __launch_bounds__(256) k_convert3(const double *__restrict__ ring, int64_t P, int64_t nvalid,
                                                   uint16_t *__restrict__ h0, uint16_t *__restrict__ h1,
-                                                  uint16_t *__restrict__ h2, int64_t ld, int64_t col0,
-                                                  int8_t *__restrict__ pA, int64_t ldp, int blk)
+                                                  uint16_t *__restrict__ h2, int64_t rows,
+                                                  int8_t *__restrict__ pA, int blk)
 {
     const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t node = gt / CONV_LANES;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) k_convert3(const double *__restrict__ rin
     }
     if (!live) return;
     const int pe = exp_of_maxbits(mb);
-    if (part == 0) pA[node * ldp + blk] = (int8_t)pe;
+    if (part == 0) pA[blk * rows + node] = (int8_t)pe;
 #pragma unroll
     for (int g = 0; g < CONV_ROWS / 8; ++g) {
         uint16_t a[8], b[8], c[8];
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) k_convert3(const double *__restrict__ rin
         vb.z = b[4] | ((uint32_t)b[5] << 16); vb.w = b[6] | ((uint32_t)b[7] << 16);
         vc.x = c[0] | ((uint32_t)c[1] << 16); vc.y = c[2] | ((uint32_t)c[3] << 16);
         vc.z = c[4] | ((uint32_t)c[5] << 16); vc.w = c[6] | ((uint32_t)c[7] << 16);
-        const int64_t o = node * ld + col0 + r0 + 8 * g;
+        const int64_t o = (blk * rows + node) * 64 + r0 + 8 * g;
         *(uint4 *)(h0 + o) = va;
         *(uint4 *)(h1 + o) = vb;
         *(uint4 *)(h2 + o) = vc;
@@ -234,14 +234,15 @@ __global__ void __launch_bounds__(256) k_convert3(const double *__restrict__ rin
 // past n0 their contraction over the super-block's own history.
 __global__ void __launch_bounds__(64) k_wgen3(const double *__restrict__ wlag_all, int64_t wstride, int n0,
                                               uint16_t *__restrict__ w0, uint16_t *__restrict__ w1,
-                                              uint16_t *__restrict__ w2, int64_t ld, float *__restrict__ pW,
-                                              int64_t ldp, int n_grp, int kt_lim)
+                                              uint16_t *__restrict__ w2, float *__restrict__ pW, int n_grp,
+                                              int kt_lim)
 {
     __shared__ double red[2];
     const int kt = blockIdx.x, r = blockIdx.y;
     if (kt >= n0 / 64 + r / 64 || kt >= kt_lim) return;  // the whole CTA (uniform)
     const int j = r + 64 * n_grp * blockIdx.z;
     const double *wlag = wlag_all + (int64_t)blockIdx.z * wstride;
+    const int64_t row = (int64_t)kt * (64 * n_grp * gridDim.z) + j;   // of the tile-major slices
     const int t = kt * 64 + threadIdx.x;
     const double v = wlag[n0 + r - t];
     double m = fabs(v);
@@ -252,12 +253,12 @@ __global__ void __launch_bounds__(64) k_wgen3(const double *__restrict__ wlag_al
     m = fmax(red[0], red[1]);
     const int pe = exp_of_maxbits((unsigned long long)__double_as_longlong(m));
     if (threadIdx.x == 0)                                // the scale 2^pe, exact (pe in [-127, 127])
-        pW[(int64_t)j * ldp + kt] = pe >= -126 ? __int_as_float((pe + 127) << 23) : __int_as_float(0x00400000);
+        pW[row] = pe >= -126 ? __int_as_float((pe + 127) << 23) : __int_as_float(0x00400000);
     uint16_t a, b, c;
     digits3(fixed16(v, pe), a, b, c);
-    w0[(int64_t)j * ld + t] = a;
-    w1[(int64_t)j * ld + t] = b;
-    w2[(int64_t)j * ld + t] = c;
+    w0[row * 64 + threadIdx.x] = a;
+    w1[row * 64 + threadIdx.x] = b;
+    w2[row * 64 + threadIdx.x] = c;
 }
 
 // ---- seven-slice form: x 2^-pe = sum_s a_s 2^-9s, |x| < 2^(pe+8), balanced base-512 digits |a_s| <= 256
@@ -495,7 +496,7 @@ int launch_block_prep3(cudaStream_t st, const SplitPrep3 &p, int64_t n0, bool we
         const int blk = (int)(n0 / 64) - 1;
         const int64_t threads = p.nvalid * CONV_LANES;
         k_convert3<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(p.ring, p.P, p.nvalid, p.hist[0], p.hist[1],
-                                                                      p.hist[2], p.ld, n0 - 64, p.pA, p.ldp, blk);
+                                                                      p.hist[2], p.rows, p.pA, blk);
         FPDE_LAUNCHED(1);
     }
     if (weights && n0 / 64 + (p.n_grp > 0 ? p.n_grp : 1) - 1 > 0) {
@@ -504,7 +505,7 @@ int launch_block_prep3(cudaStream_t st, const SplitPrep3 &p, int64_t n0, bool we
         // columns stop at the slices' pitch: a later block of the super-block exists only below the
         // step capacity, so its contraction never reaches past it
         const int kt_lim = (int)std::min<int64_t>(p.ld / 64, p.ldp);
-        k_wgen3<<<g, 64, 0, st>>>(p.wlag, p.wstride, (int)n0, p.w[0], p.w[1], p.w[2], p.ld, p.pW, p.ldp, ng, kt_lim);
+        k_wgen3<<<g, 64, 0, st>>>(p.wlag, p.wstride, (int)n0, p.w[0], p.w[1], p.w[2], p.pW, ng, kt_lim);
         FPDE_LAUNCHED(1);
     }
     return FPDE_OK;

@@ -168,16 +168,23 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v)
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[k]);
 }
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float *v)
-{
-    uint32_t r[4];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(taddr));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __uint_as_float(r[k]);
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Four floats from shared memory, not moved ahead of other volatile operations.
+__device__ __forceinline__ float4 lds4(const float *p)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(smem_u32(p)));
+    return v;
+}
+// After the wait: no use of the loaded values is scheduled before it.
+template <int N>
+__device__ __forceinline__ void tmem_loaded(float *v)
+{
+#pragma unroll
+    for (int k = 0; k < N; ++k) asm volatile("" : "+f"(v[k]));
+}
 
 struct __align__(64) FarMaps {
     CUtensorMap a_hi, a_lo, w_hi, w_lo;
@@ -345,6 +352,11 @@ __global__ void __launch_bounds__(THREADS, 1)
 // into lo together with that sum's rounding error. The leading product is therefore free of
 // accumulation error, whatever the rounding of the tensor core's FP32 adder, and the FP32
 // rounding of lo stays near 2^-31 of the partial per k-tile.
+// What bounds it: the fold. A 128 x 128 k-tile (NG = 2) takes 24 MMAs of 64 cycles and 2,300 cycles of
+// shared memory, the fold of its two accumulators 3,000 (nine packed operations per column pair and 128 KB
+// out of TMEM); loads and MMAs hide behind it. One column at a time, its scale by a shuffle, in 168
+// registers it took 4,300. 16 epilogue warps of 32 columns were slower (3,250). At 65,536 rows, 256 steps
+// and 2,560 columns a launch takes 459 us (625 before).
 constexpr int THREADS3 = 64 + 8 * 32;                         // TMA warp, MMA warp, 8 epilogue warps
 
 // Shape of the three-slice kernel for NG weight groups (64 steps each) per item: one MMA of
@@ -357,9 +369,24 @@ struct Far3Cfg {
     static constexpr int STAGE = 3 * A_BYTES + 3 * WB;        // 72 KB (NG 1), 96 KB (NG 2)
     static constexpr int STAGES = NG == 1 ? 3 : 2;
     static constexpr int TMEM = 4 * N;                        // 2 buffers x (X0, X12)
-    static constexpr int SMEM = 1024 + STAGES * STAGE + 256;
     static constexpr int COLS = N / 2;                        // columns per epilogue warp
-    static constexpr int CH = NG == 1 ? 32 : 4;               // columns per TMEM read batch
+    static constexpr int CH = 16;                             // columns per TMEM read batch
+    static constexpr int EW = 8;                              // epilogue warps
+    // A warpgroup for TMA and MMA, the others for the epilogue. At NG = 2 the epilogue takes the registers
+    // that the first warpgroup gives back (the shares add up to what the block is launched with).
+    static constexpr int THREADS = 128 + 32 * EW;
+    static constexpr int REGS = 168, REGS_ISSUE = 40, REGS_FOLD = 232;   // NG = 2
+    static_assert(NG != 2 || (128 * REGS_ISSUE + 32 * EW * REGS_FOLD <= THREADS * REGS && THREADS * REGS <= 65536),
+                  "register shares");
+    static constexpr int SCALES = EW * 2 * COLS * 4;          // per epilogue warp: two k-tiles' column scales
+    static constexpr int SMEM = 1024 + STAGES * STAGE + SCALES + 256;
+};
+
+// Where a k-tile's boxes and scales are: row-major slices ([rows][ld], scales [rows][ldp]) or tile-major
+// ones ([k-tile][rows][64], scales [k-tile][rows]), in which a box is one contiguous 16 KB.
+struct Far3Layout {
+    int x_kt, ya_kt, yw_kt;                                   // box coordinates per k-tile
+    int64_t pa_row, pa_kt, pw_row, pw_kt;                     // strides of the scales
 };
 
 struct __align__(64) FarMaps3 {
@@ -372,24 +399,76 @@ __device__ __forceinline__ float pow2f(int e)
     return e >= -126 ? __int_as_float((e + 127) << 23) : __int_as_float(0x00400000);
 }
 
+// Two floats in one 64-bit register, one instruction per operation on both: the folds of the accumulators
+// are bound by issue slots and by the latency of their dependent operations, not by the FP32 lanes.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float x, float y)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a - b: exactly one multiply-add (a packed subtract costs two more instructions for the signs).
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, 0xBF800000BF800000ull, a); }
+// a += b, returns the rounding error (TwoSum); and with b = v sc exactly (sc a power of two).
+__device__ __forceinline__ f32x2 two_sum2(f32x2 &a, f32x2 b)
+{
+    const f32x2 s = add2(a, b), nb = sub2(a, s);        // -(what of b went into s)
+    const f32x2 e = add2(sub2(a, add2(s, nb)), add2(b, nb));
+    a = s;
+    return e;
+}
+__device__ __forceinline__ f32x2 two_sum2(f32x2 &a, f32x2 v, f32x2 sc)
+{
+    const f32x2 s = fma2(v, sc, a), nb = sub2(a, s);
+    const f32x2 e = add2(sub2(a, add2(s, nb)), fma2(v, sc, nb));
+    a = s;
+    return e;
+}
+
 // Persistent: gridDim.x CTAs (at most one per SM) walk the items (128-row tile mt, k-split ks,
 // weight-group set gi of NG groups) = blockIdx.x, blockIdx.x + gridDim.x, ...; the TMA producer,
 // the MMA issuer and the epilogue follow the same static sequence of k-tiles, so the pipeline runs
 // on across item boundaries and TMEM is allocated once. Every item writes its partial (zeros if
 // its k range is empty).
 template <int NG>
-__global__ void __launch_bounds__(THREADS3, 1)
+__global__ void __launch_bounds__(Far3Cfg<NG>::THREADS, 1)
     k_far_tc3(const __grid_constant__ FarMaps3 maps, double *__restrict__ C, int64_t ldc_split, int64_t ldc_col,
               int64_t rows, int kt_begin, int kt_total, int kt_per, int n_split, uint32_t idesc,
-              const int8_t *__restrict__ pA, const float *__restrict__ pW, int64_t ldp, const int *__restrict__ wcol,
-              int n_sets, int grp0, int64_t ldc_grp, unsigned *flags)
+              const int8_t *__restrict__ pA, const float *__restrict__ pW, const Far3Layout ly,
+              const int *__restrict__ wcol, int n_sets, int grp0, int64_t ldc_grp, unsigned *flags)
 {
     using Cfg = Far3Cfg<NG>;
     constexpr int STAGES = Cfg::STAGES, STAGE_BYTES3 = Cfg::STAGE, N = Cfg::N, COLS = Cfg::COLS, CH = Cfg::CH;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *stage_base = smem;
-    uint64_t *bars = (uint64_t *)(smem + STAGES * STAGE_BYTES3);
+    float *scales = (float *)(smem + STAGES * STAGE_BYTES3);
+    uint64_t *bars = (uint64_t *)(smem + STAGES * STAGE_BYTES3 + Cfg::SCALES);
     uint64_t *full = bars, *empty = bars + STAGES, *tfull = bars + 2 * STAGES, *tempty = bars + 2 * STAGES + 2;
     uint64_t *mma_done = bars + 2 * STAGES + 4;
     volatile uint32_t *tmem_slot = (volatile uint32_t *)(bars + 2 * STAGES + 5);
@@ -401,7 +480,7 @@ __global__ void __launch_bounds__(THREADS3, 1)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 256); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 32 * Cfg::EW); }
         mbar_init(mma_done, 1);
         *abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -417,80 +496,85 @@ __global__ void __launch_bounds__(THREADS3, 1)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == 0) {
-        if (lane == 0) {                                   // TMA producer
-            const CUtensorMap *wm = NG == 1 ? maps.w : maps.w2;
-            int g = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const int gi = item % n_sets, mk = item / n_sets;
-                const int mt = mk / n_split, ks = mk % n_split;
-                const int kt0 = kt_begin + ks * kt_per, kt1 = min(kt0 + kt_per, kt_total);
-                for (int kt = kt0; kt < kt1; ++kt, ++g) {
-                    const int s = g % STAGES;
-                    const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
-                    if (!mbar_wait(&empty[s], ph ^ 1u, flags, abort_s)) { ok = false; break; }
-                    uint8_t *st = stage_base + s * STAGE_BYTES3;
-                    mbar_expect_tx(&full[s], STAGE_BYTES3);
-                    const int x = kt * BK, y = mt * BM, yw = ((wcol ? wcol[mt] : 0) + grp0 + NG * gi) * BN;
+    if (warp < 4) {
+        if constexpr (NG == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_ISSUE));
+        if (warp == 0) {
+            if (lane == 0) {                                   // TMA producer
+                const CUtensorMap *wm = NG == 1 ? maps.w : maps.w2;
+                int g = 0;
+                bool ok = true;
+                for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                    const int gi = item % n_sets, mk = item / n_sets;
+                    const int mt = mk / n_split, ks = mk % n_split;
+                    const int kt0 = kt_begin + ks * kt_per, kt1 = min(kt0 + kt_per, kt_total);
+                    for (int kt = kt0; kt < kt1; ++kt, ++g) {
+                        const int s = g % STAGES;
+                        const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+                        if (!mbar_wait(&empty[s], ph ^ 1u, flags, abort_s)) { ok = false; break; }
+                        uint8_t *st = stage_base + s * STAGE_BYTES3;
+                        mbar_expect_tx(&full[s], STAGE_BYTES3);
+                        const int x = kt * ly.x_kt, y = kt * ly.ya_kt + mt * BM;
+                        const int yw = kt * ly.yw_kt + ((wcol ? wcol[mt] : 0) + grp0 + NG * gi) * BN;
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) tma_load_2d(st + q * A_BYTES, &maps.a[q], x, y, &full[s]);
+                        for (int q = 0; q < 3; ++q) tma_load_2d(st + q * A_BYTES, &maps.a[q], x, y, &full[s]);
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) tma_load_2d(st + 3 * A_BYTES + q * Cfg::WB, &wm[q], x, yw, &full[s]);
-                }
-            }
-            for (int it = (g > STAGES ? g - STAGES : 0); it < g; ++it) {   // own copies in flight
-                const int s = it % STAGES;
-                const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-                unsigned long long t0 = gtimer();
-                while (!mbar_try_wait(&full[s], ph) && gtimer() - t0 < WAIT_NS) {}
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {                                   // MMA issuer: one k-tile per chunk
-            int g = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const int ks = (item / n_sets) % n_split;
-                const int kt0 = kt_begin + ks * kt_per, kt1 = min(kt0 + kt_per, kt_total);
-                for (int kt = kt0; kt < kt1 && !*abort_s; ++kt, ++g) {
-                    const int buf = g & 1;
-                    const uint32_t use = (uint32_t)(g >> 1);
-                    if (!mbar_wait(&tempty[buf], (use & 1u) ^ 1u, flags, abort_s)) { ok = false; break; }
-                    tc_fence_after();
-                    const int s = g % STAGES;
-                    const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
-                    if (!mbar_wait(&full[s], ph, flags, abort_s)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t x0 = tmem + (uint32_t)(buf * 2 * N), x12 = x0 + N;
-                    const uint64_t dst = sdesc_sw128(smem_u32(stage_base + s * STAGE_BYTES3));
-                    const uint32_t dlo = (uint32_t)dst, dhi = (uint32_t)(dst >> 32);
-                    constexpr uint32_t A1 = A_BYTES >> 4, A2 = 2 * A_BYTES >> 4;
-                    constexpr uint32_t W0 = 3 * A_BYTES >> 4, W1 = W0 + (Cfg::WB >> 4), W2 = W0 + (2 * Cfg::WB >> 4);
-#pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        const uint32_t o = dlo + (uint32_t)(k * 2);      // +32 bytes per K=16 step
-                        const uint32_t acc = k ? 1u : 0u;
-                        umma_lo(x0, o, o + W0, dhi, idesc, acc);
-                        umma_lo(x12, o, o + W1, dhi, idesc, acc);
-                        umma_lo(x12, o + A1, o + W0, dhi, idesc, 1u);
-                        umma_lo(x12, o, o + W2, dhi, idesc, 1u);
-                        umma_lo(x12, o + A1, o + W1, dhi, idesc, 1u);
-                        umma_lo(x12, o + A2, o + W0, dhi, idesc, 1u);
+                        for (int q = 0; q < 3; ++q) tma_load_2d(st + 3 * A_BYTES + q * Cfg::WB, &wm[q], x, yw, &full[s]);
                     }
-                    umma_commit(&empty[s]);
-                    umma_commit(&tfull[buf]);
+                }
+                for (int it = (g > STAGES ? g - STAGES : 0); it < g; ++it) {   // own copies in flight
+                    const int s = it % STAGES;
+                    const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
+                    unsigned long long t0 = gtimer();
+                    while (!mbar_try_wait(&full[s], ph) && gtimer() - t0 < WAIT_NS) {}
                 }
             }
-            umma_commit(mma_done);
-            const unsigned long long t0 = gtimer();
-            while (!mbar_try_wait(mma_done, 0) && gtimer() - t0 < WAIT_NS) {}
+        } else if (warp == 1) {
+            if (lane == 0) {                                   // MMA issuer: one k-tile per chunk
+                int g = 0;
+                bool ok = true;
+                for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                    const int ks = (item / n_sets) % n_split;
+                    const int kt0 = kt_begin + ks * kt_per, kt1 = min(kt0 + kt_per, kt_total);
+                    for (int kt = kt0; kt < kt1 && !*abort_s; ++kt, ++g) {
+                        const int buf = g & 1;
+                        const uint32_t use = (uint32_t)(g >> 1);
+                        if (!mbar_wait(&tempty[buf], (use & 1u) ^ 1u, flags, abort_s)) { ok = false; break; }
+                        tc_fence_after();
+                        const int s = g % STAGES;
+                        const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+                        if (!mbar_wait(&full[s], ph, flags, abort_s)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t x0 = tmem + (uint32_t)(buf * 2 * N), x12 = x0 + N;
+                        const uint64_t dst = sdesc_sw128(smem_u32(stage_base + s * STAGE_BYTES3));
+                        const uint32_t dlo = (uint32_t)dst, dhi = (uint32_t)(dst >> 32);
+                        constexpr uint32_t A1 = A_BYTES >> 4, A2 = 2 * A_BYTES >> 4;
+                        constexpr uint32_t W0 = 3 * A_BYTES >> 4, W1 = W0 + (Cfg::WB >> 4), W2 = W0 + (2 * Cfg::WB >> 4);
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k) {
+                            const uint32_t o = dlo + (uint32_t)(k * 2);      // +32 bytes per K=16 step
+                            const uint32_t acc = k ? 1u : 0u;
+                            umma_lo(x0, o, o + W0, dhi, idesc, acc);
+                            umma_lo(x12, o, o + W1, dhi, idesc, acc);
+                            umma_lo(x12, o + A1, o + W0, dhi, idesc, 1u);
+                            umma_lo(x12, o, o + W2, dhi, idesc, 1u);
+                            umma_lo(x12, o + A1, o + W1, dhi, idesc, 1u);
+                            umma_lo(x12, o + A2, o + W0, dhi, idesc, 1u);
+                        }
+                        umma_commit(&empty[s]);
+                        umma_commit(&tfull[buf]);
+                    }
+                }
+                umma_commit(mma_done);
+                const unsigned long long t0 = gtimer();
+                while (!mbar_try_wait(mma_done, 0) && gtimer() - t0 < WAIT_NS) {}
+            }
         }
     } else {
-        // 8 epilogue warps: warp w reads TMEM lane quadrant w % 4 (the hardware's rule) and
-        // folds columns [c0, c0 + COLS) with c0 = COLS * ((w - 2) / 4)
+        if constexpr (NG == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_FOLD));
+        // epilogue warps: warp w reads TMEM lane quadrant w % 4 (the hardware's rule) and
+        // folds columns [c0, c0 + COLS) with c0 = COLS * (w / 4 - 1)
         const int q = warp & 3;
-        const int c0 = COLS * ((warp - 2) >> 2);
+        const int c0 = COLS * ((warp >> 2) - 1);
         int g = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -501,65 +585,71 @@ __global__ void __launch_bounds__(THREADS3, 1)
             const int64_t row_c = row < rows ? row : rows - 1;
             // this lane's row exponents and its columns' (c0 + 32u + lane) weight-tile scales; the
             // next k-tile's set is loaded while the current one is folded (both miss L1 often:
-            // shared memory takes most of it), and each column's scale reaches the warp by a shuffle
+            // shared memory takes most of it); the column scales go through the warp's two rows of
+            // shared memory, from where each four reach all lanes with one load
             constexpr int NU = COLS / 32;
-            const int8_t *pAr = pA + row_c * ldp;
-            const float *pWl = pW + ((int64_t)((wcol ? wcol[mt] : 0) + grp0 + NG * gi) * BN + c0 + lane) * ldp;
-            int e_nx = kt0 < kt1 ? (int)pAr[kt0] : 0;
+            float *wrow = scales + (warp - 4) * (2 * COLS);
+            const int8_t *pAr = pA + row_c * ly.pa_row;
+            const float *pWl = pW + ((int64_t)((wcol ? wcol[mt] : 0) + grp0 + NG * gi) * BN + c0 + lane) * ly.pw_row;
+            int e_nx = kt0 < kt1 ? (int)pAr[kt0 * ly.pa_kt] : 0;
             float w_nx[NU];
 #pragma unroll
-            for (int u = 0; u < NU; ++u) w_nx[u] = kt0 < kt1 ? __ldg(pWl + (int64_t)32 * u * ldp + kt0) : 0.f;
-            float hi[COLS], lo[COLS];
+            for (int u = 0; u < NU; ++u) w_nx[u] = kt0 < kt1 ? __ldg(pWl + 32 * u * ly.pw_row + kt0 * ly.pw_kt) : 0.f;
+            f32x2 hi[COLS / 2], lo[COLS / 2];             // columns 2j, 2j + 1
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) { hi[j] = 0.f; lo[j] = 0.f; }
+            for (int j = 0; j < COLS / 2; ++j) hi[j] = lo[j] = 0ull;
             for (int kt = kt0; kt < kt1; ++kt, ++g) {
                 const int buf = g & 1;
                 const uint32_t use = (uint32_t)(g >> 1);
                 const int e_cur = e_nx;
-                float w_cur[NU];
+                float *wcur = wrow + buf * COLS;          // last read two k-tiles ago
 #pragma unroll
-                for (int u = 0; u < NU; ++u) w_cur[u] = w_nx[u];
+                for (int u = 0; u < NU; ++u) wcur[32 * u + lane] = w_nx[u];
+                __syncwarp();
                 if (kt + 1 < kt1) {
-                    e_nx = (int)pAr[kt + 1];
+                    e_nx = (int)pAr[(kt + 1) * ly.pa_kt];
 #pragma unroll
-                    for (int u = 0; u < NU; ++u) w_nx[u] = __ldg(pWl + (int64_t)32 * u * ldp + kt + 1);
+                    for (int u = 0; u < NU; ++u) w_nx[u] = __ldg(pWl + 32 * u * ly.pw_row + (kt + 1) * ly.pw_kt);
                 }
                 if (!mbar_wait(&tfull[buf], use & 1u, flags, abort_s)) { ok = false; break; }
                 tc_fence_after();
                 // 2^pA * 2^pW: a product of powers of two, exact while it stays normal
-                const float sa = pow2f(e_cur);
+                const float sa1 = pow2f(e_cur);
+                const f32x2 sa = pack2(sa1, sa1);
                 const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 2 * N + c0);
+                // batches of CH columns of both accumulators, the next one in flight while one is folded
+                constexpr int NB = COLS / CH;
+                float v0[2][CH], v1[2][CH];
+                tmem_ld16(tb, v0[0]);
+                tmem_ld16(tb + N, v1[0]);
 #pragma unroll
-                for (int h = 0; h < COLS / CH; ++h) {
-                    // a batch of CH columns of both accumulators in flight before one wait
-                    float v0[CH], v1[CH];
-                    if constexpr (CH == 4) {
-                        tmem_ld4(tb + CH * h, v0);
-                        tmem_ld4(tb + N + CH * h, v1);
+                for (int h = 0; h < NB; ++h) {
+                    float *x0 = v0[h & 1], *x12 = v1[h & 1];
+                    tmem_ld_wait();
+                    tmem_loaded<CH>(x0);
+                    tmem_loaded<CH>(x12);
+                    if (h + 1 < NB) {
+                        tmem_ld16(tb + CH * (h + 1), v0[(h + 1) & 1]);
+                        tmem_ld16(tb + N + CH * (h + 1), v1[(h + 1) & 1]);
                     } else {
+                        tc_fence_before();
+                        mbar_arrive(&tempty[buf]);
+                    }
 #pragma unroll
-                        for (int b = 0; b < CH / 16; ++b) {
-                            tmem_ld16(tb + CH * h + 16 * b, v0 + 16 * b);
-                            tmem_ld16(tb + N + CH * h + 16 * b, v1 + 16 * b);
+                    for (int jj = 0; jj < CH; jj += 4) {
+                        const float4 w = lds4(wcur + CH * h + jj);
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int j = (CH * h + jj) / 2 + u, i = jj + 2 * u;
+                            const f32x2 sc = mul2(sa, u ? pack2(w.z, w.w) : pack2(w.x, w.y));
+                            // X0 (exact integer sum) enters hi by TwoSum; X12, 2^-8 of it, goes straight
+                            // into lo with the rounding error (FP32 rounding of lo is ~2^-31 of hi per
+                            // k-tile)
+                            const f32x2 e = two_sum2(hi[j], pack2(x0[i], x0[i + 1]), sc);
+                            lo[j] = fma2(pack2(x12[i], x12[i + 1]), sc, add2(lo[j], e));
                         }
                     }
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int jj = 0; jj < CH; ++jj) {
-                        const int j = CH * h + jj;
-                        const float sc = sa * __shfl_sync(0xffffffffu, w_cur[j >> 5], j & 31);
-                        // X0 (exact integer sum) enters hi by TwoSum; X12, 2^-8 of it, goes straight
-                        // into lo with the rounding error (FP32 rounding of lo is ~2^-31 of hi per
-                        // k-tile)
-                        const float x = v0[jj] * sc;           // exact (power-of-two scaling)
-                        const float s = hi[j] + x, bb = s - hi[j];
-                        const float e = (hi[j] - (s - bb)) + (x - bb);
-                        hi[j] = s;
-                        lo[j] = fmaf(v1[jj], sc, lo[j] + e);
-                    }
                 }
-                tc_fence_before();
-                mbar_arrive(&tempty[buf]);
             }
             if (ok && row < rows) {                   // float pairs: no FP64 work here
                 // column c of the item is step c % 64 of group NG gi + c / 64, i.e. at
@@ -567,7 +657,11 @@ __global__ void __launch_bounds__(THREADS3, 1)
                 float2 *out = reinterpret_cast<float2 *>(C + (int64_t)ks * ldc_split + (int64_t)NG * gi * ldc_grp + row) +
                               (int64_t)c0 * ldc_col;
 #pragma unroll
-                for (int j = 0; j < COLS; ++j) out[(int64_t)j * ldc_col] = make_float2(hi[j], lo[j]);
+                for (int j = 0; j < COLS / 2; ++j) {
+                    const float2 h = unpack2(hi[j]), l = unpack2(lo[j]);
+                    out[(int64_t)(2 * j) * ldc_col] = make_float2(h.x, l.x);
+                    out[(int64_t)(2 * j + 1) * ldc_col] = make_float2(h.y, l.y);
+                }
             }
         }
     }
@@ -620,60 +714,6 @@ __device__ __forceinline__ uint64_t sdesc_sw64(uint32_t saddr)
     return d;
 }
 
-// Two floats in one 64-bit register: one instruction per operation on both (the fold is bound by issue
-// slots: 8 warps x 32 columns x about 60 operations per k-tile).
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float x, float y)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-// a += b, returns the rounding error (TwoSum); and with b = v sc exactly (sc a power of two).
-__device__ __forceinline__ f32x2 two_sum2(f32x2 &a, f32x2 b)
-{
-    const f32x2 s = add2(a, b), nb = sub2(a, s);        // -(what of b went into s)
-    const f32x2 e = add2(sub2(a, add2(s, nb)), add2(b, nb));
-    a = s;
-    return e;
-}
-__device__ __forceinline__ f32x2 two_sum2(f32x2 &a, f32x2 v, f32x2 sc)
-{
-    const f32x2 s = fma2(v, sc, a), nb = sub2(a, s);
-    const f32x2 e = add2(sub2(a, add2(s, nb)), fma2(v, sc, nb));
-    a = s;
-    return e;
-}
 // x 2^e for a finite x (e in a range where 2^e is normal), exact unless the result leaves FP64's range
 __device__ __forceinline__ double scale_f64(double x, int e)
 {
@@ -834,6 +874,7 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
                     tmem_ld16(ta, v);
                     tmem_ld16(ta + 16, v + 16);
                     tmem_ld_wait();
+                    tmem_loaded<32>(v);
                     tc_fence_before();
                     mbar_arrive(&sempty[sl]);
 #pragma unroll
@@ -934,7 +975,7 @@ int far_plan_init(FarPlan *p, const void *a_hi, const void *a_lo, int64_t rows, 
 }
 
 int far_plan3_init(FarPlan3 *p, const void *const a[3], int64_t rows, int64_t lda, const void *const w[3],
-                   int64_t ldw, int w_tiles)
+                   int64_t ldw, int w_tiles, bool tiled)
 {
     if (rows % tc::BM != 0 || lda % tc::BK != 0 || ldw % tc::BK != 0)
         return set_error(FPDE_ERR_ARG, "far contraction: rows must be a multiple of 128, pitches of 64");
@@ -942,18 +983,21 @@ int far_plan3_init(FarPlan3 *p, const void *const a[3], int64_t rows, int64_t ld
     tc::FarMaps3 *m = (tc::FarMaps3 *)p->maps;
     int rc;
     const int64_t w_rows = (int64_t)tc::BN * (w_tiles > 0 ? w_tiles : 1);
+    const int64_t ra = tiled ? rows * (lda / tc::BK) : rows, rw = tiled ? w_rows * (ldw / tc::BK) : w_rows;
+    const int64_t ca = tiled ? tc::BK : lda, cw = tiled ? tc::BK : ldw;
     for (int q = 0; q < 3; ++q) {
-        if ((rc = tc::make_map(&m->a[q], a[q], rows, lda, tc::BM))) return rc;
-        if ((rc = tc::make_map(&m->w[q], w[q], w_rows, ldw, tc::BN))) return rc;
+        if ((rc = tc::make_map(&m->a[q], a[q], ra, ca, tc::BM))) return rc;
+        if ((rc = tc::make_map(&m->w[q], w[q], rw, cw, tc::BN))) return rc;
         // 128-row weight boxes (two groups per item) exist only when the slices hold two tiles
         if (w_rows >= 2 * tc::BN) {
-            if ((rc = tc::make_map(&m->w2[q], w[q], w_rows, ldw, 2 * tc::BN))) return rc;
+            if ((rc = tc::make_map(&m->w2[q], w[q], rw, cw, 2 * tc::BN))) return rc;
         } else {
             m->w2[q] = m->w[q];
         }
     }
     p->rows = rows;
     p->w_rows = w_rows;
+    p->tiled = tiled;
     p->idesc = tc::idesc_f16(1, tc::BM, tc::BN);
     p->idesc2 = tc::idesc_f16(1, tc::BM, 2 * tc::BN);
     cudaError_t e = smem_opt_in((const void *)tc::k_far_tc3<1>, tc::Far3Cfg<1>::SMEM);
@@ -987,13 +1031,15 @@ int far3_launch(cudaStream_t st, const FarPlan3 *p, int k_cols, double *C, int64
     if (grid > n_sets) grid -= grid % n_sets;
     const tc::FarMaps3 *m = (const tc::FarMaps3 *)p->maps;
     const int64_t ldc_grp = (int64_t)tc::BN * ldc_col;
+    const tc::Far3Layout ly = p->tiled ? tc::Far3Layout{0, (int)p->rows, (int)p->w_rows, 1, p->rows, 1, p->w_rows}
+                                       : tc::Far3Layout{tc::BK, 0, 0, ldp, 1, ldp, 1};
     if (ng == 2)
-        tc::k_far_tc3<2><<<(unsigned)grid, tc::THREADS3, tc::Far3Cfg<2>::SMEM, st>>>(
-            *m, C, ldc_split, ldc_col, p->rows, kt_begin, kt_total, kt_per, splits, p->idesc2, pA, pW, ldp, wcol,
+        tc::k_far_tc3<2><<<(unsigned)grid, tc::Far3Cfg<2>::THREADS, tc::Far3Cfg<2>::SMEM, st>>>(
+            *m, C, ldc_split, ldc_col, p->rows, kt_begin, kt_total, kt_per, splits, p->idesc2, pA, pW, ly, wcol,
             n_sets, grp0, ldc_grp, flags);
     else
-        tc::k_far_tc3<1><<<(unsigned)grid, tc::THREADS3, tc::Far3Cfg<1>::SMEM, st>>>(
-            *m, C, ldc_split, ldc_col, p->rows, kt_begin, kt_total, kt_per, splits, p->idesc, pA, pW, ldp, wcol,
+        tc::k_far_tc3<1><<<(unsigned)grid, tc::Far3Cfg<1>::THREADS, tc::Far3Cfg<1>::SMEM, st>>>(
+            *m, C, ldc_split, ldc_col, p->rows, kt_begin, kt_total, kt_per, splits, p->idesc, pA, pW, ly, wcol,
             n_sets, grp0, ldc_grp, flags);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
@@ -1125,7 +1171,7 @@ extern "C" int fpde_far_contract3(fpde_ctx *ctx, const void *const a[3], int64_t
     FPDE_CHECK_ARG(a && w && a[0] && a[1] && a[2] && w[0] && w[1] && w[2] && pA && pW && C, "null argument");
     FPDE_CHECK_ARG(rows > 0 && k_cols >= 0 && k_cols <= lda && k_cols <= ldw && ldp * 64 >= k_cols, "bad shape");
     FarPlan3 plan;
-    if ((rc = far_plan3_init(&plan, a, rows, lda, w, ldw))) return rc;
+    if ((rc = far_plan3_init(&plan, a, rows, lda, w, ldw, 1, false))) return rc;
     if (splits <= 0) splits = far_splits(k_cols / 64, rows);
     if (splits > FAR_MAX_SPLITS) splits = FAR_MAX_SPLITS;
     float *pWs = nullptr;

@@ -23,18 +23,20 @@ int far_launch(cudaStream_t st, const FarPlan *p, int k_cols, double *C, int64_t
                int splits, double out_scale, const double *out_scale_ptr, unsigned *flags);
 int far_splits(int kt_total, int64_t rows);
 
-// Exact-slice variant: three bf16 slices per operand, per-(row, k-tile) exponents pA
-// ([rows][ldp] int8) and per-(j, k-tile) scales pW = 2^e ([64][ldp] float: the epilogue
-// multiplies by them without rebuilding each power of two).
+// Exact-slice variant: three bf16 slices per operand, per-(row, k-tile) exponents pA (int8) and
+// per-(j, k-tile) scales pW = 2^e (float: the epilogue multiplies by them without rebuilding each
+// power of two). Tile-major (what the engines keep): slices [ld/64][rows][64], pA [k-tile][rows], pW
+// [k-tile][w_rows]. Row-major (the public contraction): slices [rows][ld], pA and pW [rows][ldp].
 struct FarPlan3 {
     alignas(64) unsigned char maps[9 * 128];
     int64_t rows = 0;
     int64_t w_rows = 0;                        // rows of the W slices (64 per weight tile)
+    bool tiled = true;
     uint32_t idesc = 0, idesc2 = 0;            // MMA instruction descriptors for N = 64 and 128
 };
 // w_tiles: number of 64-row weight tiles in the W slices (columns of an ensemble; 1 otherwise).
 int far_plan3_init(FarPlan3 *p, const void *const a[3], int64_t rows, int64_t lda, const void *const w[3],
-                   int64_t ldw, int w_tiles = 1);
+                   int64_t ldw, int w_tiles = 1, bool tiled = true);
 // Writes each partial as a float pair (hi, lo) into the 8-byte slot of C (the fold's float-
 // float value; hi + lo is exact in FP64): read it with ff_to_double.
 // wcol (device, may be null): per 128-row tile the weight tile (column of an ensemble) it uses,
