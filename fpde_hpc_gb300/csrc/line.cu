@@ -326,16 +326,17 @@ __global__ void __launch_bounds__(LT) k_line_solve(LineSolveArgs p)
 
 // ---------------------------------------------------------------------------------------
 // Persistent form for the split path: one cooperative launch advances steps j0 .. j0+nsteps-1
-// of a 64-step block, with two warp roles per CTA:
+// of a 64-step block, with three warp roles per CTA:
 //   solver warps (LTS threads, SP nodes each): the chunk's right-hand side, the two sweeps and
-//     scans, the exchange of the two chunk aggregates with all other chunks (one row of value
-//     slots per step, each written once per launch and polled until it leaves the all-bits-set
-//     pattern) and the new state; state and time-invariant data stay in registers for the
-//     whole launch;
-//   history warps (LTS threads): during step j, the far partials and the near history of
+//     scans, the two chunk aggregates for all other chunks (one row of value slots per step, each
+//     written once per launch) and the new state; state and time-invariant data stay in registers
+//     for the whole launch;
+//   history warps (LTS threads): during step j, the near history and the far partials of
 //     step j+1 for every node of the chunk except the newest increment (which the solver
-//     adds), handed over in shared memory.
-// The two roles meet at one CTA barrier per step; the solver warps synchronise among
+//     adds), handed over in shared memory;
+//   carry warps (LTS threads): poll every chunk's aggregates until they leave the all-bits-set
+//     pattern and form this chunk's carries.
+// The roles meet at one CTA barrier per step; the solver warps synchronise among
 // themselves with a named barrier. The near-history work thus overlaps the latency-bound
 // scans and the exchange.
 //
@@ -450,28 +451,50 @@ struct Near64 {
     static __device__ __forceinline__ const W *scale(const LineBlockArgs &p) { return p.ng; }
 };
 
-// acc += far partials of steps j .. j+NJ-1 (NJ accumulators; every load issued first).
-template <class H, int SP, int NJ>
-__device__ __forceinline__ void far_fold(const LineBlockArgs &p, int ht, int a, int b, int j, H (&acc)[NJ][SP])
+// The far partials of step j for this thread's nodes, added after the near sums: loaded before those
+// (far_load), so that their latency passes behind them, where registers can hold them (SP <= 4), else by
+// far_add itself, one split at a time.
+template <int SP>
+constexpr int FAR_SLOTS = SP <= 4 ? FAR_MAX_SPLITS : 1;
+template <int SP>
+__device__ __forceinline__ void far_load1(const LineBlockArgs &p, int ht, int a, int b, int j, int k, double (&v)[SP])
 {
-    double v[NJ][FAR_MAX_SPLITS][SP];
 #pragma unroll
-    for (int m = 0; m < NJ; ++m)
+    for (int q = 0; q < SP; ++q) {
+        const int64_t node = a + ht + LTS * q;
+        v[q] = (k < p.KS && node < b && j < BLK)
+                   ? __ldcg(p.cfar + ((int64_t)k * p.far_ld + p.far_row0 + j) * p.P + node)
+                   : 0.0;
+    }
+}
+template <int SP>
+__device__ __forceinline__ void far_load(const LineBlockArgs &p, int ht, int a, int b, int j,
+                                         double (&v)[FAR_SLOTS<SP>][SP])
+{
+    if constexpr (FAR_SLOTS<SP> == FAR_MAX_SPLITS) {
+#pragma unroll
+        for (int k = 0; k < FAR_MAX_SPLITS; ++k) far_load1<SP>(p, ht, a, b, j, k, v[k]);
+    }
+}
+template <class H, int SP>
+__device__ __forceinline__ void far_add(const LineBlockArgs &p, int ht, int a, int b, int j,
+                                        double (&v)[FAR_SLOTS<SP>][SP], H *acc)
+{
+    if constexpr (FAR_SLOTS<SP> == FAR_MAX_SPLITS) {
 #pragma unroll
         for (int k = 0; k < FAR_MAX_SPLITS; ++k)
+            if (k < p.KS) {
 #pragma unroll
-            for (int q = 0; q < SP; ++q) {
-                const int64_t node = a + ht + LTS * q;
-                v[m][k][q] = (k < p.KS && node < b && j + m < BLK)
-                                 ? __ldcg(p.cfar + ((int64_t)k * p.far_ld + p.far_row0 + j + m) * p.P + node)
-                                 : 0.0;
+                for (int q = 0; q < SP; ++q) acc[q].add(v[k][q], p.far_pairs);
             }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < p.KS; ++k) {
+            far_load1<SP>(p, ht, a, b, j, k, v[0]);
 #pragma unroll
-    for (int m = 0; m < NJ; ++m)
-#pragma unroll
-        for (int k = 0; k < FAR_MAX_SPLITS; ++k)
-#pragma unroll
-            for (int q = 0; q < SP; ++q) acc[m][q].add(v[m][k][q], p.far_pairs);
+            for (int q = 0; q < SP; ++q) acc[q].add(v[0][q], p.far_pairs);
+        }
+    }
 }
 
 // acc += sum_{r < rmax} w[j - r] D_r for this thread's nodes (rows of the row ring in global memory,
@@ -480,7 +503,7 @@ template <class H, int SP>
 __device__ __forceinline__ void near_rows(const LineBlockArgs &p, int ht, int a, int b, int j, int rmax, H *acc)
 {
     using Row = typename H::Row;
-    constexpr int RB = SP <= 4 ? 8 : 4;                  // rows per batch
+    constexpr int RB = SP <= 2 ? 8 : (SP == 4 ? 4 : 2);  // rows per batch
     int64_t node[SP];
 #pragma unroll
     for (int q = 0; q < SP; ++q) node[q] = a + ht + LTS * q;
@@ -625,10 +648,21 @@ __device__ __forceinline__ void history_store_scaled(int ht, int a, int b, const
 // GB300 runs FP64 at 2 DFMA/clk/SM (a warp's FP64 instruction holds its scheduler's FP64 pipe
 // for ~64 cycles), so the history warps sum in float-float on the FP32 pipe (ringf, wff: the
 // increments and weights as float pairs; the solver hands each new FP64 row over in shared
-// memory and the history warps convert it), and the four history warps form the four carry
-// dot products side by side.
+// memory and the history warps convert it).
+// What bounds a step: the FP64 pipe of each quarter SM (about 70 cycles per warp instruction) and the
+// scans' latencies; the history sums run beside. The exchange has a warpgroup of its own, its four warps
+// forming the four carry dot products side by side: polled by the history warps, it took 2,400 of their
+// 9,900 cycles a step at 65,536 nodes (SP = 4), and the solver waited for them. With it, and the far
+// partials loaded ahead of the near sums instead of waited for (1,300 cycles), far product included: a
+// split step of 16,384 nodes with an explicit part 3.2 us (3.7 before), of 65,536 nodes 8.1 (8.5); an
+// FP64 step of 1,000 nodes 3.8 (4.2), of 65,536 nodes 15.6 (16.6).
+constexpr int BST = 3 * LTS;             // threads: solver, history and carry warpgroups
+// registers a thread: the solver keeps its nodes' state and coefficients; the shares add up to what the
+// block is launched with
+constexpr int BS_REGS = 168, BS_SOLVER = 248, BS_HISTORY = 176, BS_CARRY = 80;
+static_assert(BS_SOLVER + BS_HISTORY + BS_CARRY <= 3 * BS_REGS && BST * BS_REGS <= 65536, "register shares");
 template <class H, int SP, bool EXPL>
-__global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
+__global__ void __launch_bounds__(BST, 1) k_line_block_spec(LineBlockArgs p)
 {
     using Row = typename H::Row;
     constexpr bool FF = std::is_same<H, NearFF>::value;
@@ -653,13 +687,11 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
         sCb[tid / NWS][tid % NWS] = wc[NWS * NWS + tid];
     }
 
-    if (!solver) {
-        // ============== history warps: H_t = far^t + sum_{0 <= r <= t-3} w[t-r] D_r.
-        // H_{t+3} is summed before X(s+1) from every row but D_t; after X(s+1) D_t arrives in
-        // sD, is converted into the float-pair ring and its one term completes H_{t+3}.
-        const int ht = tid - LTS;
-        const int lane = tid & 31, hw = ht >> 5;
-        // history warp hw's carry dot product over the chunks' aggregates: 0 Lf[c].Y (c_in),
+    if (tid >= 2 * LTS) {
+        // ============== carry warps
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(BS_CARRY));
+        const int lane = tid & 31, hw = (tid - 2 * LTS) >> 5;
+        // carry warp hw's dot product over the chunks' aggregates: 0 Lf[c].Y (c_in),
         // 1 Mb[c].U0, 2 Kb[c].Y, 3 Lf[G].Y (the flux end's y; unused at a Dirichlet end)
         const bool flux = p.rkind != FPDE_BC_DIRICHLET;
         const double *cvec = hw == 0 ? p.Lf + (int64_t)c * G
@@ -726,6 +758,22 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
                 }
             }
         };
+        __syncthreads_or(0);                                                // start
+        for (int s = 0; s < p.nsteps; ++s) {
+            __syncthreads();                                                // X(s): s_red has been read
+            if (s_abort) return;
+            carries(s);
+            asm volatile("bar.arrive 2, %0;" ::"n"(2 * LTS) : "memory");      // (C): carries of step t
+        }
+        return;
+    }
+    if (!solver) {
+        // ============== history warps: H_t = sum_{0 <= r <= t-3} w[t-r] D_r + far^t.
+        // H_{t+3} is summed before X(s+1) from every row but D_t; after X(s+1) D_t arrives in
+        // sD, is converted into the float-pair ring and its one term and the far partials complete
+        // H_{t+3}.
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(BS_HISTORY));
+        const int ht = tid - LTS;
         constexpr int NR = SpecRing<SP>::NR;
         Row *sR = reinterpret_cast<Row *>(spec_rows);
         const int rlo0 = max(0, p.j0 - NR);              // rows of earlier launches into the ring
@@ -742,19 +790,25 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
             const int i = a + ht + LTS * q;
             sg[q] = i < b ? __ldg(H::scale(p) + i) : H::zero();
         }
-        H h3[3][SP];                                     // H_j0, H_j0+1, H_j0+2
-        far_fold<H, SP, 3>(p, ht, a, b, p.j0, h3);
-        near_rows_split<H, SP>(p, sR, ht, a, b, p.j0, max(p.j0 - 2, 0), rlo0, h3[0]);
-        history_store_scaled<H, SP>(ht, a, b, h3[0], sg, sS[p.j0 & 1]);
+        double fv[FAR_SLOTS<SP>][SP];
+        // H_j, complete, of one of the launch's first three steps
+        auto first = [&](int j, H (&h)[SP]) {
+            far_load<SP>(p, ht, a, b, j, fv);
+#pragma unroll
+            for (int q = 0; q < SP; ++q) h[q] = H();
+            near_rows_split<H, SP>(p, sR, ht, a, b, j, max(j - 2, 0), rlo0, h);
+        };
+        H acc[SP];
+        first(p.j0, acc);
+        far_add<H, SP>(p, ht, a, b, p.j0, fv, acc);
+        history_store_scaled<H, SP>(ht, a, b, acc, sg, sS[p.j0 & 1]);
         __syncthreads_or(0);                                                // start: the solver's prologue
         if (p.j0 + 1 < jend) {                                              // runs beside the rest
-            near_rows_split<H, SP>(p, sR, ht, a, b, p.j0 + 1, max(p.j0 - 1, 0), rlo0, h3[1]);
-            history_store_scaled<H, SP>(ht, a, b, h3[1], sg, sS[(p.j0 + 1) & 1]);
+            first(p.j0 + 1, acc);
+            far_add<H, SP>(p, ht, a, b, p.j0 + 1, fv, acc);
+            history_store_scaled<H, SP>(ht, a, b, acc, sg, sS[(p.j0 + 1) & 1]);
         }
-        H acc[SP];
-#pragma unroll
-        for (int q = 0; q < SP; ++q) acc[q] = h3[2][q];
-        if (p.j0 + 2 < jend) near_rows_split<H, SP>(p, sR, ht, a, b, p.j0 + 2, p.j0, rlo0, acc);   // complete
+        if (p.j0 + 2 < jend) first(p.j0 + 2, acc);       // its far partials are added below
         const typename H::W w3 = __ldg(H::weights(p) + 3);
         for (int s = 0; s < p.nsteps; ++s) {
             __syncthreads();                                                // X(s): D_{t-1} is in sD
@@ -774,14 +828,14 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
                     }
                 }
             }
-            if (t + 2 < jend) history_store_scaled<H, SP>(ht, a, b, acc, sg, sS[t & 1]);
-            carries(s);
-            asm volatile("bar.arrive 2, %0;" ::"n"(2 * LTS) : "memory");      // (C): carries of step t
+            if (t + 2 < jend) {
+                far_add<H, SP>(p, ht, a, b, t + 2, fv, acc);
+                history_store_scaled<H, SP>(ht, a, b, acc, sg, sS[t & 1]);
+            }
             if (t + 3 < jend) {
-                H f[1][SP];
-                far_fold<H, SP, 1>(p, ht, a, b, t + 3, f);
+                far_load<SP>(p, ht, a, b, t + 3, fv);
 #pragma unroll
-                for (int q = 0; q < SP; ++q) acc[q] = f[0][q];
+                for (int q = 0; q < SP; ++q) acc[q] = H();
                 near_rows_split<H, SP>(p, sR, ht, a, b, t + 3, t, max(0, t - NR), acc);
             }
         }
@@ -789,6 +843,7 @@ __global__ void __launch_bounds__(2 * LTS, 1) k_line_block_spec(LineBlockArgs p)
     }
 
     // ===================================================================== solver warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(BS_SOLVER));
     const int lane = tid & 31, warp = tid >> 5;
     const int i0 = a + tid * SP;
     const int i1 = min(i0 + SP, b);
@@ -1332,7 +1387,7 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     a.chunk = L->chunk;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(L->G);
-    cfg.blockDim = dim3(2 * LTS);
+    cfg.blockDim = dim3(BST);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1724,7 +1779,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
         for (auto fn : {k_line_block_spec<NearFF, LSEG, false>, k_line_block_spec<NearFF, LSEG, true>,
                         k_line_block_spec<Near64, LSEG, false>}) {
             int n_sm = 0;
-            FPDE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n_sm, fn, 2 * LTS, SpecRing<LSEG>::bytes));
+            FPDE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n_sm, fn, BST, SpecRing<LSEG>::bytes));
             per_sm = std::min(per_sm, n_sm);
         }
     }
