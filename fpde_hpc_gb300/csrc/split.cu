@@ -263,7 +263,6 @@ __global__ void __launch_bounds__(64) k_wgen3(const double *__restrict__ wlag_al
 
 // ---- seven-slice form: x 2^-pe = sum_s a_s 2^-9s, |x| < 2^(pe+8), balanced base-512 digits |a_s| <= 256
 // of the 63-bit integer v = rint(x 2^(54-pe)); each digit is stored as the bf16 value a_s 2^-9s (exact).
-constexpr int PE7_ZERO = -4096;                      // exponent of an all-zero block
 __device__ __forceinline__ int exp7_of_maxbits(unsigned long long mbits)
 {
     const int ex = (int)((mbits >> 52) & 0x7FF);
@@ -297,7 +296,7 @@ struct Slices7 { uint16_t *p[7]; };
 // row's largest block exponent so far.
 constexpr int CONV7_LANES = 8, CONV7_ROWS = 64 / CONV7_LANES;
 __global__ void __launch_bounds__(256) k_convert7(const double *__restrict__ rows64, int64_t P, int64_t nvalid, Slices7 out,
-                                                  int64_t ld, int64_t col0, int16_t *__restrict__ pA, int64_t ldp, int blk,
+                                                  int64_t rows, int16_t *__restrict__ pA, int blk,
                                                   int16_t *__restrict__ eA)
 {
     const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -321,13 +320,13 @@ __global__ void __launch_bounds__(256) k_convert7(const double *__restrict__ row
     if (!live) return;
     const int pe = exp7_of_maxbits(mb);
     if (part == 0) {
-        pA[node * ldp + blk] = (int16_t)pe;
+        pA[blk * rows + node] = (int16_t)pe;
         eA[node] = (int16_t)(blk == 0 ? pe : max((int)eA[node], pe));
     }
     uint16_t d[CONV7_ROWS][7];
 #pragma unroll
     for (int k = 0; k < CONV7_ROWS; ++k) digits7(v[k], pe, d[k]);
-    const int64_t o = node * ld + col0 + r0;
+    const int64_t o = ((2 * blk + r0 / 32) * rows + node) * 32 + r0 % 32;
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
         uint4 x;
@@ -339,7 +338,7 @@ __global__ void __launch_bounds__(256) k_convert7(const double *__restrict__ row
 
 // grid (64 steps j, weight tiles), 64 threads: every distance's tile of step j, two passes (the largest
 // exponent first).
-__global__ void __launch_bounds__(64) k_wgen7(const double *__restrict__ wlag_all, int64_t wstride, Slices7 out, int64_t ldw,
+__global__ void __launch_bounds__(64) k_wgen7(const double *__restrict__ wlag_all, int64_t wstride, Slices7 out,
                                               int n_delta, float *__restrict__ sW, int16_t *__restrict__ eW)
 {
     __shared__ unsigned long long red[2];
@@ -368,7 +367,7 @@ __global__ void __launch_bounds__(64) k_wgen7(const double *__restrict__ wlag_al
         }
         uint16_t s[7];
         digits7((unsigned long long)__double_as_longlong(w[64 * d + j - c]), pe, s);
-        const int64_t o = ((int64_t)blockIdx.y * 64 + j) * ldw + (int64_t)(d - 1) * 64 + c;
+        const int64_t o = (((int64_t)2 * (d - 1) + c / 32) * (64 * gridDim.y) + 64 * blockIdx.y + j) * 32 + c % 32;
 #pragma unroll
         for (int q = 0; q < 7; ++q) out.p[q][o] = s[q];
     }
@@ -432,14 +431,12 @@ int hist7_alloc(Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles
 {
     h->rows = (nodes + 127) / 128 * 128;
     h->n_delta = (max_steps - 1) / 64;
-    h->ld = h->ldw = (int64_t)h->n_delta * 64;
-    h->ldp = h->n_delta;
     h->w_tiles = w_tiles;
     bool fail = false;
     for (int q = 0; q < 7 && !fail; ++q)
-        fail = dev_alloc((void **)&h->a[q], (size_t)h->rows * h->ld * 2) ||
-               dev_alloc((void **)&h->w[q], (size_t)w_tiles * 64 * h->ldw * 2);
-    fail = fail || dev_alloc((void **)&h->pA, (size_t)h->rows * h->ldp * sizeof(int16_t)) ||
+        fail = dev_alloc((void **)&h->a[q], (size_t)h->rows * h->n_delta * 128) ||
+               dev_alloc((void **)&h->w[q], (size_t)w_tiles * 64 * h->n_delta * 128);
+    fail = fail || dev_alloc((void **)&h->pA, (size_t)h->rows * h->n_delta * sizeof(int16_t)) ||
            dev_alloc((void **)&h->eA, (size_t)h->rows * sizeof(int16_t)) ||
            dev_alloc((void **)&h->eW, (size_t)w_tiles * 64 * sizeof(int16_t)) ||
            dev_alloc((void **)&h->sW, (size_t)w_tiles * h->n_delta * 64 * sizeof(float));
@@ -447,10 +444,10 @@ int hist7_alloc(Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles
     if (!rc) {
         const void *a[7], *w[7];
         for (int q = 0; q < 7; ++q) { a[q] = h->a[q]; w[q] = h->w[q]; }
-        rc = far_plan7_init(p, a, h->rows, h->ld, w, h->ldw, w_tiles);
+        rc = far_plan7_init(p, a, h->rows, h->n_delta, w, w_tiles);
     }
     // rows past the nodes are never converted: their (unused) sums only need readable exponents
-    if (!rc && (cudaMemset(h->pA, 0, (size_t)h->rows * h->ldp * sizeof(int16_t)) != cudaSuccess ||
+    if (!rc && (cudaMemset(h->pA, 0, (size_t)h->rows * h->n_delta * sizeof(int16_t)) != cudaSuccess ||
                 cudaMemset(h->eA, 0, (size_t)h->rows * sizeof(int16_t)) != cudaSuccess))
         rc = FPDE_ERR_CUDA;
     if (rc) hist7_free(h);
@@ -474,7 +471,7 @@ int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t w
 {
     Slices7 o;
     for (int q = 0; q < 7; ++q) o.p[q] = h.w[q];
-    k_wgen7<<<dim3(64, (unsigned)h.w_tiles), 64, 0, st>>>(wlag, wstride, o, h.ldw, h.n_delta, h.sW, h.eW);
+    k_wgen7<<<dim3(64, (unsigned)h.w_tiles), 64, 0, st>>>(wlag, wstride, o, h.n_delta, h.sW, h.eW);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }
@@ -484,8 +481,8 @@ int hist7_convert(cudaStream_t st, const Hist7 &h, const double *rows64, int64_t
     Slices7 o;
     for (int q = 0; q < 7; ++q) o.p[q] = h.a[q];
     const int64_t threads = nvalid * CONV7_LANES;
-    k_convert7<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(rows64, P, nvalid, o, h.ld, n0 - 64, h.pA, h.ldp,
-                                                                  (int)(n0 / 64) - 1, h.eA);
+    k_convert7<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(rows64, P, nvalid, o, h.rows, h.pA, (int)(n0 / 64) - 1,
+                                                                  h.eA);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }

@@ -687,17 +687,24 @@ __global__ void __launch_bounds__(Far3Cfg<NG>::THREADS, 1)
 // increments beside a block's largest lost bits). The epilogue adds the six accumulators into three
 // floats (h, m, l) per output by error-free sums, and the result leaves as FP64. Its error against exact sums is below that of an FP64 multiply-add chain
 // over the same terms, whose rounding grows with the number of terms.
-// What bounds it: shared memory. A k-tile of 128 rows x 64 steps takes 112 MMAs (M = 128, N = 64, K = 16)
-// that read 6 KB each next to 168 KB of TMA writes: 6,560 cycles at 128 B per cycle; the tensor
-// cores' own time is 3,600, the fold's about 4,000 on the FP32 pipes. The FP64 pipe would take 320,000.
-// Operands come as 32-column half tiles (64-byte swizzle, two 84 KB stages); the six accumulators
-// of 64 columns rotate through eight TMEM slots, the widest level first, so that a k-tile's MMAs start
-// while the one before is folded.
+// What bounds it: no one unit. A k-tile of 128 rows x 64 steps takes 112 MMAs (M = 128, N = 64, K = 16)
+// that read 6 KB each next to 168 KB of TMA writes: 6,600 cycles of shared memory at 128 B per cycle; the
+// tensor cores' own time is 3,600, the fold's 4,000 on the FP32 pipes and 3,000 of TMEM reads, HBM's 5,000.
+// Measured 10,600: the FP64 pipe would take 320,000. At 65,536 rows the product over one k-tile takes 50 us,
+// over ten 227 us. On the way: 8 epilogue warps of 32 columns, their conversions to FP64 with branches, and
+// two stages of node-major slices took 102 and 302 us; the conversions alone 58 of each.
+// Operands come as 32-column half tiles (64-byte swizzle), contiguous in memory: three stages of the history
+// (it comes from HBM), two of the weights (they come from L2). 16-column stages of 32-byte swizzle let more
+// be in flight, but were slower (26 %). The six accumulators of 64 columns rotate through eight TMEM slots,
+// the widest level first, so that a k-tile's MMAs start while the one before is folded.
 constexpr int F7_BK = 32;
 constexpr int F7_A = BM * F7_BK * 2, F7_W = BN * F7_BK * 2;   // one slice of a stage: 8 KB, 4 KB
-constexpr int F7_STAGE = 7 * (F7_A + F7_W);                   // 84 KB
-constexpr int F7_STAGES = 2, F7_SLOTS = 8, F7_LEV = 6;
-constexpr int F7_SMEM = 1024 + F7_STAGES * F7_STAGE + 256;
+constexpr int F7_STA = 7 * F7_A, F7_STW = 7 * F7_W;           // a stage: 56 KB of history, 28 KB of weights
+constexpr int F7_NA = 3, F7_NW = 2, F7_SLOTS = 8, F7_LEV = 6;
+constexpr int F7_SMEM = 1024 + F7_NA * F7_STA + F7_NW * F7_STW + 256;
+static_assert(F7_SMEM <= 227 * 1024, "shared memory");
+constexpr int F7_COLS = 16, F7_EW = 4 * (BN / F7_COLS);       // columns per epilogue warp, epilogue warps
+constexpr int F7_THREADS = 128 + 32 * F7_EW;                  // a TMA, an MMA and two idle warps, the epilogue
 
 struct __align__(64) FarMaps7 {
     CUtensorMap a[7], w[7];
@@ -726,9 +733,9 @@ struct Far7Args {
     double *C;
     int64_t ldc_split, ldc_col, rows;
     int kt_begin, kt_end, kt_per, n_split;           // k-tiles [kt_begin, kt_end); the block's index is kt_end
-    const int16_t *pA;                               // [rows][ldp]
+    const int16_t *pA;                               // [k-tile][rows]
     const int16_t *eA;                               // [rows]: largest pA of the row so far
-    int64_t ldp;
+    int w_rows;                                      // 64 per weight tile
     const float *sW;                                 // [weight tiles][n_delta][64]: 2^(pW - eW)
     const int16_t *eW;                               // [weight tiles][64]: largest pW of the step
     int n_delta;
@@ -737,20 +744,22 @@ struct Far7Args {
     unsigned *flags;
 };
 
-__global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__ FarMaps7 maps, const Far7Args p)
+__global__ void __launch_bounds__(F7_THREADS, 1) k_far_tc7(const __grid_constant__ FarMaps7 maps, const Far7Args p)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t *bars = (uint64_t *)(smem + F7_STAGES * F7_STAGE);
-    uint64_t *full = bars, *empty = bars + F7_STAGES, *sfull = bars + 2 * F7_STAGES, *sempty = sfull + F7_SLOTS;
-    uint64_t *mma_done = sempty + F7_SLOTS;
+    uint8_t *smw = smem + F7_NA * F7_STA;                  // the weights' stages
+    uint64_t *bars = (uint64_t *)(smw + F7_NW * F7_STW);
+    uint64_t *full = bars, *empty = full + F7_NA, *fullw = empty + F7_NA, *emptyw = fullw + F7_NW;
+    uint64_t *sfull = emptyw + F7_NW, *sempty = sfull + F7_SLOTS, *mma_done = sempty + F7_SLOTS;
     volatile uint32_t *tmem_slot = (volatile uint32_t *)(mma_done + 1);
     volatile int *abort_s = (volatile int *)(mma_done + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_items = (int)(p.rows / BM) * p.n_split;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < F7_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int s = 0; s < F7_SLOTS; ++s) { mbar_init(&sfull[s], 1); mbar_init(&sempty[s], 256); }
+        for (int s = 0; s < F7_NA; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < F7_NW; ++s) { mbar_init(&fullw[s], 1); mbar_init(&emptyw[s], 1); }
+        for (int s = 0; s < F7_SLOTS; ++s) { mbar_init(&sfull[s], 1); mbar_init(&sempty[s], 32 * F7_EW); }
         mbar_init(mma_done, 1);
         *abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -765,37 +774,48 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    // the splits of a row tile differ in length when they do not divide the k-tiles: the rotation gives every
+    // CTA each of them in turn where the grid is a multiple of their count
     auto k_range = [&](int item, int &mt, int &ks, int &k0, int &k1) {
         mt = item / p.n_split;
-        ks = item % p.n_split;
+        ks = (item + (gridDim.x % p.n_split ? 0 : item / gridDim.x)) % p.n_split;
         k0 = p.kt_begin + ks * p.kt_per;
         k1 = min(k0 + p.kt_per, p.kt_end);
     };
 
     if (warp == 0) {
         if (lane == 0) {                                   // TMA producer: half tiles
-            int g = 0, mt, ks, k0, k1;
+            int g = 0, ga = 0, mt, ks, k0, k1;
             bool ok = true;
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 k_range(item, mt, ks, k0, k1);
                 const int yw = (p.wcol ? p.wcol[mt] : 0) * BN;
                 for (int h = 2 * k0; h < 2 * k1; ++h, ++g) {
-                    const int s = g % F7_STAGES;
-                    if (!mbar_wait(&empty[s], ((uint32_t)(g / F7_STAGES) & 1u) ^ 1u, p.flags, abort_s)) { ok = false; break; }
-                    uint8_t *st = smem + s * F7_STAGE;
-                    mbar_expect_tx(&full[s], F7_STAGE);
+                    const int s = g % F7_NA, sw = g % F7_NW;
+                    if (!mbar_wait(&empty[s], ((uint32_t)(g / F7_NA) & 1u) ^ 1u, p.flags, abort_s)) { ok = false; break; }
+                    uint8_t *st = smem + s * F7_STA;
+                    mbar_expect_tx(&full[s], F7_STA);
+                    const int ya = h * (int)p.rows + mt * BM;
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) tma_load_2d(st + q * F7_A, &maps.a[q], 0, ya, &full[s]);
+                    ++ga;
+                    if (!mbar_wait(&emptyw[sw], ((uint32_t)(g / F7_NW) & 1u) ^ 1u, p.flags, abort_s)) { ok = false; break; }
+                    st = smw + sw * F7_STW;
+                    mbar_expect_tx(&fullw[sw], F7_STW);
                     // the weights depend on the distance between the block and the k-tile only
-                    const int xa = h * F7_BK, xw = (p.kt_end - (h >> 1) - 1) * BK + (h & 1) * F7_BK;
+                    const int y = (2 * (p.kt_end - (h >> 1) - 1) + (h & 1)) * p.w_rows + yw;
 #pragma unroll
-                    for (int q = 0; q < 7; ++q) tma_load_2d(st + q * F7_A, &maps.a[q], xa, mt * BM, &full[s]);
-#pragma unroll
-                    for (int q = 0; q < 7; ++q) tma_load_2d(st + 7 * F7_A + q * F7_W, &maps.w[q], xw, yw, &full[s]);
+                    for (int q = 0; q < 7; ++q) tma_load_2d(st + q * F7_W, &maps.w[q], 0, y, &fullw[sw]);
                 }
             }
-            for (int it = (g > F7_STAGES ? g - F7_STAGES : 0); it < g; ++it) {   // own copies in flight
-                const unsigned long long t0 = gtimer();
-                while (!mbar_try_wait(&full[it % F7_STAGES], (uint32_t)(it / F7_STAGES) & 1u) && gtimer() - t0 < WAIT_NS) {}
-            }
+            auto landed = [&](uint64_t *bar, int n, int stages) {   // own copies in flight
+                for (int it = (n > stages ? n - stages : 0); it < n; ++it) {
+                    const unsigned long long t0 = gtimer();
+                    while (!mbar_try_wait(&bar[it % stages], (uint32_t)(it / stages) & 1u) && gtimer() - t0 < WAIT_NS) {}
+                }
+            };
+            landed(full, ga, F7_NA);
+            landed(fullw, g, F7_NW);
         }
     } else if (warp == 1) {
         if (lane == 0) {                                   // MMA issuer
@@ -804,12 +824,14 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
             for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
                 k_range(item, mt, ks, k0, k1);
                 for (int h = 2 * k0; h < 2 * k1 && ok && !*abort_s; ++h, ++g) {
-                    const int s = g % F7_STAGES;
-                    if (!mbar_wait(&full[s], (uint32_t)(g / F7_STAGES) & 1u, p.flags, abort_s)) { ok = false; break; }
+                    const int s = g % F7_NA, sw = g % F7_NW;
+                    if (!mbar_wait(&full[s], (uint32_t)(g / F7_NA) & 1u, p.flags, abort_s) ||
+                        !mbar_wait(&fullw[sw], (uint32_t)(g / F7_NW) & 1u, p.flags, abort_s)) { ok = false; break; }
                     tc_fence_after();
                     const bool second = h & 1;
-                    const uint64_t dst = sdesc_sw64(smem_u32(smem + s * F7_STAGE));
+                    const uint64_t dst = sdesc_sw64(smem_u32(smem + s * F7_STA));
                     const uint32_t dlo = (uint32_t)dst, dhi = (uint32_t)(dst >> 32);
+                    const uint32_t wlo = (uint32_t)sdesc_sw64(smem_u32(smw + sw * F7_STW));
                     // accumulator 0: levels 6 and 5; 1 .. 5: levels 4 .. 0
 #pragma unroll
                     for (int l = 0; l < F7_LEV; ++l) {
@@ -826,14 +848,14 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
                             for (int sa = 0; sa <= lev; ++sa)
 #pragma unroll
                                 for (int k = 0; k < F7_BK / 16; ++k) {
-                                    const uint32_t o = dlo + (uint32_t)(k * 2);
-                                    umma_lo(x, o + (uint32_t)(sa * F7_A >> 4),
-                                            o + (uint32_t)((7 * F7_A + (lev - sa) * F7_W) >> 4), dhi, p.idesc, acc ? 1u : 0u);
+                                    umma_lo(x, dlo + (uint32_t)(k * 2 + (sa * F7_A >> 4)),
+                                            wlo + (uint32_t)(k * 2 + ((lev - sa) * F7_W >> 4)), dhi, p.idesc, acc ? 1u : 0u);
                                     acc = true;
                                 }
                         if (second) umma_commit(&sfull[sl]);
                     }
                     umma_commit(&empty[s]);
+                    umma_commit(&emptyw[sw]);
                     if (second) c += F7_LEV;
                 }
             }
@@ -841,26 +863,27 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
             const unsigned long long t0 = gtimer();
             while (!mbar_try_wait(mma_done, 0) && gtimer() - t0 < WAIT_NS) {}
         }
-    } else {
-        // 8 epilogue warps: TMEM lane quadrant warp % 4, columns c0 .. c0 + 31
-        const int q = warp & 3, c0 = 32 * ((warp - 2) >> 2);
+    } else if (warp >= 4) {
+        // epilogue warps: TMEM lane quadrant warp % 4, columns c0 .. c0 + F7_COLS - 1
+        const int q = warp & 3, c0 = F7_COLS * ((warp >> 2) - 1);
         int c = 0, mt, ks, k0, k1;
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
             k_range(item, mt, ks, k0, k1);
             const int64_t row = (int64_t)mt * BM + q * 32 + lane;
             const int wt = p.wcol ? p.wcol[mt] : 0;
-            const int16_t *pAr = p.pA + row * p.ldp;
+            const int16_t *pAr = p.pA + row;
             const int eA = p.eA[row];
             const float *sW = p.sW + (int64_t)wt * p.n_delta * BN + c0;
-            f32x2 hh[16], mm[16], ll[16];                     // columns 2j, 2j + 1
+            constexpr int NP = F7_COLS / 2;
+            f32x2 hh[NP], mm[NP], ll[NP];                     // columns 2j, 2j + 1
 #pragma unroll
-            for (int j = 0; j < 16; ++j) hh[j] = mm[j] = ll[j] = 0ull;
-            int e_nx = k0 < k1 ? (int)pAr[k0] : 0;
+            for (int j = 0; j < NP; ++j) hh[j] = mm[j] = ll[j] = 0ull;
+            int e_nx = k0 < k1 ? (int)pAr[k0 * p.rows] : 0;
             for (int kt = k0; kt < k1 && ok; ++kt, c += F7_LEV) {
                 const float sa1 = pow2f(max(e_nx - eA, -127));
                 const f32x2 sa = pack2(sa1, sa1);
-                if (kt + 1 < k1) e_nx = pAr[kt + 1];
+                if (kt + 1 < k1) e_nx = pAr[(kt + 1) * p.rows];
                 const float4 *w4 = reinterpret_cast<const float4 *>(sW + (int64_t)(p.kt_end - kt - 1) * BN);
                 // not unrolled: the levels share two bodies (into m, into h), which have to stay in the
                 // instruction cache (unrolled, the warps waited for instructions most of the time)
@@ -870,15 +893,14 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
                     if (!mbar_wait(&sfull[sl], (uint32_t)((c + l) / F7_SLOTS) & 1u, p.flags, abort_s)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(sl * BN + c0);
-                    float v[32];
+                    float v[F7_COLS];
                     tmem_ld16(ta, v);
-                    tmem_ld16(ta + 16, v + 16);
                     tmem_ld_wait();
-                    tmem_loaded<32>(v);
+                    tmem_loaded<F7_COLS>(v);
                     tc_fence_before();
                     mbar_arrive(&sempty[sl]);
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
+                    for (int k = 0; k < F7_COLS / 4; ++k) {
                         const float4 x = __ldg(w4 + k);
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
@@ -896,13 +918,37 @@ __global__ void __launch_bounds__(THREADS3, 1) k_far_tc7(const __grid_constant__
             if (ok) {
                 const int16_t *eW = p.eW + (int64_t)wt * BN + c0;
                 double *out = p.C + (int64_t)ks * p.ldc_split + row + (int64_t)c0 * p.ldc_col;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
+                // the usual exponents: the result's own exponent moves, without its edge cases
+                const int ew = eW[lane % F7_COLS] == PE7_ZERO ? 0 : eW[lane % F7_COLS], ea = eA == PE7_ZERO ? 0 : eA;
+                const int lo = ea + __reduce_min_sync(0xffffffffu, ew), hi = ea + __reduce_max_sync(0xffffffffu, ew);
+                const bool usual = __all_sync(0xffffffffu, lo > -800 && hi < 800);
+                auto value = [&](int j, double (&d)[2]) {
                     const float2 h = unpack2(hh[j]), m = unpack2(mm[j]), l = unpack2(ll[j]);
-                    const double d0 = f2d_bits(h.x) + (f2d_bits(m.x) + f2d_bits(l.x));
-                    const double d1 = f2d_bits(h.y) + (f2d_bits(m.y) + f2d_bits(l.y));
-                    out[(int64_t)(2 * j) * p.ldc_col] = scale_f64(d0, eA + (int)__ldg(eW + 2 * j));
-                    out[(int64_t)(2 * j + 1) * p.ldc_col] = scale_f64(d1, eA + (int)__ldg(eW + 2 * j + 1));
+                    d[0] = f2d_bits(h.x) + (f2d_bits(m.x) + f2d_bits(l.x));
+                    d[1] = f2d_bits(h.y) + (f2d_bits(m.y) + f2d_bits(l.y));
+                };
+                if (usual) {
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) {
+                        double d[2];
+                        value(j, d);
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int e = ea + __shfl_sync(0xffffffffu, ew, 2 * j + u), dh = __double2hiint(d[u]);
+                            out[(int64_t)(2 * j + u) * p.ldc_col] =
+                                __hiloint2double(dh & 0x7FF00000 ? dh + e * (1 << 20) : 0, __double2loint(d[u]));
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) {
+                        double d[2];
+                        value(j, d);
+#pragma unroll
+                        for (int u = 0; u < 2; ++u)
+                            out[(int64_t)(2 * j + u) * p.ldc_col] =
+                                scale_f64(d[u], ea + __shfl_sync(0xffffffffu, ew, 2 * j + u));
+                    }
                 }
             }
         }
@@ -1045,17 +1091,15 @@ int far3_launch(cudaStream_t st, const FarPlan3 *p, int k_cols, double *C, int64
     return FPDE_OK;
 }
 
-int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int64_t lda, const void *const w[7], int64_t ldw,
-                   int w_tiles)
+int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int n_tiles, const void *const w[7], int w_tiles)
 {
-    if (rows % tc::BM != 0 || lda % tc::BK != 0 || ldw % tc::BK != 0)
-        return set_error(FPDE_ERR_ARG, "far contraction: rows must be a multiple of 128, pitches of 64");
+    if (rows % tc::BM != 0) return set_error(FPDE_ERR_ARG, "far contraction: rows must be a multiple of 128");
     static_assert(sizeof(tc::FarMaps7) <= sizeof(p->maps), "map storage");
     tc::FarMaps7 *m = (tc::FarMaps7 *)p->maps;
     int rc;
     for (int q = 0; q < 7; ++q)
-        if ((rc = tc::make_map(&m->a[q], a[q], rows, lda, tc::BM, tc::F7_BK)) ||
-            (rc = tc::make_map(&m->w[q], w[q], (int64_t)tc::BN * w_tiles, ldw, tc::BN, tc::F7_BK)))
+        if ((rc = tc::make_map(&m->a[q], a[q], 2 * n_tiles * rows, tc::F7_BK, tc::BM, tc::F7_BK)) ||
+            (rc = tc::make_map(&m->w[q], w[q], (int64_t)2 * n_tiles * tc::BN * w_tiles, tc::F7_BK, tc::BN, tc::F7_BK)))
             return rc;
     p->rows = rows;
     p->idesc = tc::idesc_f16(1, tc::BM, tc::BN);
@@ -1078,11 +1122,11 @@ int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_begin,
     a.kt_per = (a.kt_end - a.kt_begin + splits - 1) / splits;      // every split is written, possibly with zeros
     a.n_split = splits;
     a.C = C; a.ldc_split = ldc_split; a.ldc_col = ldc_col; a.rows = p->rows;
-    a.pA = h.pA; a.eA = h.eA; a.ldp = h.ldp; a.sW = h.sW; a.eW = h.eW; a.n_delta = h.n_delta; a.wcol = wcol;
+    a.pA = h.pA; a.eA = h.eA; a.w_rows = tc::BN * h.w_tiles; a.sW = h.sW; a.eW = h.eW; a.n_delta = h.n_delta; a.wcol = wcol;
     a.idesc = p->idesc; a.flags = flags;
     const int64_t items = (p->rows / tc::BM) * splits;
     const unsigned grid = (unsigned)std::min<int64_t>(items, device_sm_count());
-    tc::k_far_tc7<<<grid, tc::THREADS3, tc::F7_SMEM, st>>>(*(const tc::FarMaps7 *)p->maps, a);
+    tc::k_far_tc7<<<grid, tc::F7_THREADS, tc::F7_SMEM, st>>>(*(const tc::FarMaps7 *)p->maps, a);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }

@@ -54,14 +54,16 @@ int far3_launch(cudaStream_t st, const FarPlan3 *p, int k_cols, double *C, int64
 // weights w[n0 + j - t] of a block at n0 depend on its distance from a k-tile only, so their tiles
 // (distance 1 .. n_delta blocks) are formed once.
 struct Hist7 {
-    uint16_t *a[7] = {};   // [rows][ld] node-major slices
-    uint16_t *w[7] = {};   // [w_tiles 64][ldw]: column (d-1) 64 + c: lag 64 d + j - c
-    int16_t *pA = nullptr, *eA = nullptr;      // [rows][ldp] exponents per (node, block); [rows] largest so far
+    // half-tile-major slices: a box of the product (128 nodes or 64 steps x 32 columns) is contiguous
+    uint16_t *a[7] = {};   // [2 n_delta half blocks][rows][32]
+    uint16_t *w[7] = {};   // [2 n_delta][w_tiles 64][32]: column c of distance d, half c / 32: lag 64 d + j - c
+    int16_t *pA = nullptr, *eA = nullptr;      // [n_delta][rows] exponents per (block, node); [rows] largest so far
     int16_t *eW = nullptr;                     // [w_tiles][64] largest exponent of the step's weights
     float *sW = nullptr;                       // [w_tiles][n_delta][64] 2^(exponent - eW)
-    int64_t rows = 0, ld = 0, ldw = 0, ldp = 0;
+    int64_t rows = 0;
     int n_delta = 0, w_tiles = 1;
 };
+constexpr int PE7_ZERO = -4096;                // exponent of an all-zero block
 struct FarPlan7 {
     alignas(64) unsigned char maps[14 * 128];
     int64_t rows = 0;
@@ -78,8 +80,7 @@ int hist7_convert(cudaStream_t st, const Hist7 &h, const double *rows64, int64_t
 // windows with cta_col and col_lag).
 int launch_near64(cudaStream_t st, const double *rows, int64_t P, int r0, int j, const double *wlag, const double *init,
                   double *S, const int *cta_col = nullptr, const int *col_lag = nullptr, int64_t wstride = 0);
-int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int64_t lda, const void *const w[7], int64_t ldw,
-                   int w_tiles);
+int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int n_tiles, const void *const w[7], int w_tiles);
 // C[split ldc_split + j ldc_col + row] = sum over the split's share of columns [k_begin, k_cols) of
 // A[row][t] w[k_cols + j - t], j < 64, in FP64.
 int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_begin, int k_cols, double *C, int64_t ldc_split,
@@ -89,22 +90,11 @@ int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_begin,
 __device__ __forceinline__ double f2d_bits(float x)
 {
     const uint32_t b = (uint32_t)__float_as_int(x);
-    const uint64_t sign = (uint64_t)(b >> 31) << 63;
-    const uint32_t e = (b >> 23) & 0xFFu, m = b & 0x7FFFFFu;
-    uint64_t r;
-    if (e == 0) {
-        if (m == 0) {
-            r = sign;
-        } else {                                        // subnormal: m * 2^-149
-            const int k = 31 - __clz((int)m);           // highest set bit, 0..22
-            r = sign | ((uint64_t)(k - 149 + 1023) << 52) | (((uint64_t)m << (52 - k)) & 0xFFFFFFFFFFFFFull);
-        }
-    } else if (e == 0xFFu) {
-        r = sign | (0x7FFull << 52) | ((uint64_t)m << 29);
-    } else {
-        r = sign | ((uint64_t)(e - 127 + 1023) << 52) | ((uint64_t)m << 29);
-    }
-    return __longlong_as_double((long long)r);
+    const bool tiny = (b & 0x7F800000u) == 0;               // zero or subnormal: scaled by 2^64 first
+    const uint32_t y = tiny ? (uint32_t)__float_as_int(__fmul_rn(x, 18446744073709551616.f)) : b, m = y & 0x7FFFFFFFu;
+    uint32_t hi = (m >> 3) + (tiny ? (896u - 64u) << 20 : m >= 0x7F800000u ? 1792u << 20 : 896u << 20);
+    hi = (m == 0 ? 0u : hi) | (b & 0x80000000u);
+    return __hiloint2double((int)hi, (int)(y << 29));
 }
 // A far-contraction slot (float pair) as one double: hi + lo, exact.
 __device__ __forceinline__ double ff_to_double(double slot)
