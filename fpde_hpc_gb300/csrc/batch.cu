@@ -17,7 +17,7 @@
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
 // three-slice tensor-core contraction of all history before the block with one weight tile
 // per column (tc_far.cu; each 128-row tile picks its column's tile), and per step the near
-// history in float-float from a 64-row float-pair ring (k_near_history_ff); the solve writes
+// history in float-float from a 64-row float-pair ring (k_near_pre_ff, k_near_history_sub); the solve writes
 // each increment to that ring and to the FP64 one the conversion reads.
 // The alpha recurrence is time-invariant and precomputed on the host per column.
 #include <algorithm>
@@ -417,8 +417,8 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
                         return rc;
                     ++k;
                 }
-                if ((rc = launch_near_history_ff(st, b->ringf, b->Ptot, j, b->wff, b->cfar, splits, 1, b->Sn, b->cta_col,
-                                                 b->LW, use_pre ? b->pre : nullptr, j0)))
+                if ((rc = launch_near_history_sub(st, b->ringf, b->Ptot, j, b->wff, b->Sn, use_pre ? b->pre : nullptr,
+                                                  b->cta_col, b->LW)))
                     return rc;
                 ++k;
                 KS = 1;

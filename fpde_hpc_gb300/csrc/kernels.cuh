@@ -65,14 +65,16 @@ int launch_block_prep3(cudaStream_t st, const SplitPrep3 &p, int64_t n0, bool we
 //   S[i] = sum_{q<KS} far_q[j][i] + sum_{r<j} w[j-r] D_r[i],
 // far partials [KS][64][P] (float pairs when pairs != 0), in float-float arithmetic on the FP32
 // pipe (GB300 issues 2 DFMA/clk/SM) from the float-pair ring (ringf [64][P]) and float-pair lag
-// weights (wff, per column at wff + col * wstride when cta_col is given: each 512-node group's
-// column); one FP64 add per node.
+// weights (wff); one FP64 add per node.
 int launch_near_history_ff(cudaStream_t st, const float2 *ringf, int64_t P, int j, const float2 *wff,
-                           const double *cfar, int KS, int pairs, double *S, const int *cta_col = nullptr,
-                           int64_t wstride = 0, const float2 *pre = nullptr, int r0 = 0);
-// Sub-blocks of the near history: the partial sums of NEAR_SUB steps from the rows before j0
-// (pre: NEAR_SUB rows of P float pairs).
+                           const double *cfar, int KS, int pairs, double *S);
+// The same in sub-blocks of NEAR_SUB steps (weights per column at wff + col * wstride when cta_col is
+// given: each 512-node group's column): the partial sums of a sub-block's steps from the far partials
+// and the rows before it (pre: NEAR_SUB rows of P float pairs), once, and per step S from pre (null: 0)
+// and the sub-block's rows before j.
 constexpr int NEAR_SUB = 8;
+int launch_near_history_sub(cudaStream_t st, const float2 *ringf, int64_t P, int j, const float2 *wff, double *S,
+                            const float2 *pre, const int *cta_col = nullptr, int64_t wstride = 0);
 int launch_near_pre_ff(cudaStream_t st, const float2 *ringf, int64_t P, int j0, const float2 *wff, const double *cfar,
                        int KS, int pairs, float2 *pre, const int *cta_col = nullptr, int64_t wstride = 0);
 

@@ -10,7 +10,7 @@
 //   5. append        : D_n = U - U_old over the grid (the snapshot of the step, :5733-5745)
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
 // three-slice tensor-core contraction of all history before the block (tc_far.cu, as for
-// lines) and, per step, k_near_history_ff: the far partials plus the near history in
+// lines) and, per step, k_near_history_sub: the far partials plus the near history in
 // float-float from the 64-row float-pair ring of the block's increments (step 5 writes it
 // beside the FP64 ring that the conversion reads).
 // Each pass is a Thomas solve per line with R = Rlap + lam (A_/B/R :3095-3142). For a
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(128, SEGLEN <= 16 ? 5 : 4) k_lod_pass_seg(LodP
 // rows older than j0, with those steps' far partials: pre[u][i] = far(j0+u) + sum_{r<j0}
 // w[j0+u-r] ring[r], in float-float (two nodes per thread, (hi, lo) of each). Each row is read
 // once per NEAR_SUB steps instead of once per step; a step then adds only the rows of its own
-// sub-block (k_near_history_ff with pre).
+// sub-block (k_near_history_sub).
 __global__ void __launch_bounds__(256) k_near_pre_ff(const float4 *__restrict__ ringf, int64_t P2, int j0,
                                                      const float2 *__restrict__ wff_all,
                                                      const double2 *__restrict__ cfar, int KS, int pairs,
@@ -899,24 +899,42 @@ __global__ void __launch_bounds__(256) k_near_pre_ff(const float4 *__restrict__ 
     for (int u = 0; u < NEAR_SUB; ++u) pre[(int64_t)u * P2 + i] = make_float4(h[u][0], l[u][0], h[u][1], l[u][1]);
 }
 
-// Two nodes per thread: S = far partials of step j + sum_{r<j} w[j-r] ring[r] in float-float; with
-// pre (the sub-block's partial sums of k_near_pre_ff, sub-block start r0), S = pre[j-r0] + the rows
-// r0 .. j-1.
-__global__ void __launch_bounds__(256) k_near_history_ff(const float4 *__restrict__ ringf, int64_t P2, int j,
-                                                         const float2 *__restrict__ wff_all,
-                                                         const double2 *__restrict__ cfar, int KS, int pairs,
-                                                         double2 *__restrict__ S, const int *__restrict__ cta_col,
-                                                         int64_t wstride, const float4 *__restrict__ pre, int r0)
+// A step inside its sub-block: S = pre (the sub-block's partial sums of the step from k_near_pre_ff, or
+// 0) + the sub-block's R rows before it, two nodes per thread. HBM-bound, 16 + 8 R bytes a node; R is a
+// template argument because a run-time count under the unrolled row loop kept the integer pipe at 77 %
+// and HBM at 25 to 45 % (3D grid of 128^3, 1,024 steps: 175.6 -> 173.1 ms; 512 columns, 2,048 steps: 361 -> 355).
+template <int R>
+__global__ void __launch_bounds__(256) k_near_history_sub(const float4 *__restrict__ rows, int64_t P2,
+                                                          const float2 *__restrict__ wff_all,
+                                                          double2 *__restrict__ S, const int *__restrict__ cta_col,
+                                                          int64_t wstride, const float4 *__restrict__ pre)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P2) return;
     const float2 *wff = cta_col ? wff_all + (int64_t)cta_col[blockIdx.x] * wstride : wff_all;
-    float h0 = 0.f, l0 = 0.f, h1 = 0.f, l1 = 0.f;
-    if (pre) {
-        const float4 v = __ldcs(pre + (int64_t)(j - r0) * P2 + i);
-        h0 = v.x; l0 = v.y; h1 = v.z; l1 = v.w;
-        KS = 0;
+    const float4 p = pre ? __ldcs(pre + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[R > 0 ? R : 1];
+#pragma unroll
+    for (int u = 0; u < R; ++u) v[u] = __ldcg(rows + (int64_t)u * P2 + i);
+    float h0 = p.x, l0 = p.y, h1 = p.z, l1 = p.w;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const float2 w = __ldg(wff + (R - u));
+        ff_fma(h0, l0, w, make_float2(v[u].x, v[u].y));
+        ff_fma(h1, l1, w, make_float2(v[u].z, v[u].w));
     }
+    S[i] = make_double2(f2d_bits(h0) + f2d_bits(l0), f2d_bits(h1) + f2d_bits(l1));
+}
+
+// Two nodes per thread: S = far partials of step j + sum_{r<j} w[j-r] ring[r] in float-float.
+__global__ void __launch_bounds__(256) k_near_history_ff(const float4 *__restrict__ ringf, int64_t P2, int j,
+                                                         const float2 *__restrict__ wff,
+                                                         const double2 *__restrict__ cfar, int KS, int pairs,
+                                                         double2 *__restrict__ S)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P2) return;
+    float h0 = 0.f, l0 = 0.f, h1 = 0.f, l1 = 0.f;
     for (int q = 0; q < KS; ++q) {
         const double2 v = __ldcs(cfar + ((int64_t)q * 64 + j) * P2 + i);
         const float2 f0 = pairs ? *reinterpret_cast<const float2 *>(&v.x) : d2ff(v.x);
@@ -924,7 +942,7 @@ __global__ void __launch_bounds__(256) k_near_history_ff(const float4 *__restric
         ff_add(h0, l0, f0.x, f0.y);
         ff_add(h1, l1, f1.x, f1.y);
     }
-    int r = pre ? r0 : 0;
+    int r = 0;
     for (; r + 8 <= j; r += 8) {
         float4 v[8];
 #pragma unroll
@@ -956,13 +974,35 @@ __global__ void __launch_bounds__(256) k_near_history_ff(const float4 *__restric
 }
 
 int launch_near_history_ff(cudaStream_t st, const float2 *ringf, int64_t P, int j, const float2 *wff,
-                           const double *cfar, int KS, int pairs, double *S, const int *cta_col, int64_t wstride,
-                           const float2 *pre, int r0)
+                           const double *cfar, int KS, int pairs, double *S)
 {
     k_near_history_ff<<<(unsigned)((P / 2 + 255) / 256), 256, 0, st>>>((const float4 *)ringf, P / 2, j, wff,
-                                                                       (const double2 *)cfar, KS, pairs,
-                                                                       (double2 *)S, cta_col, wstride,
-                                                                       (const float4 *)pre, r0);
+                                                                       (const double2 *)cfar, KS, pairs, (double2 *)S);
+    FPDE_LAUNCHED(1);
+    return FPDE_OK;
+}
+
+int launch_near_history_sub(cudaStream_t st, const float2 *ringf, int64_t P, int j, const float2 *wff, double *S,
+                            const float2 *pre, const int *cta_col, int64_t wstride)
+{
+    const int R = j % NEAR_SUB;
+    const unsigned grid = (unsigned)((P / 2 + 255) / 256);
+    const float4 *rows = (const float4 *)(ringf + (int64_t)(j - R) * P);
+    const float4 *pr = pre ? (const float4 *)(pre + (int64_t)R * P) : nullptr;
+    static_assert(NEAR_SUB == 8, "one case per row count");
+#define NEAR_HISTORY_SUB(n) \
+    case n: k_near_history_sub<n><<<grid, 256, 0, st>>>(rows, P / 2, wff, (double2 *)S, cta_col, wstride, pr); break
+    switch (R) {
+        NEAR_HISTORY_SUB(0);
+        NEAR_HISTORY_SUB(1);
+        NEAR_HISTORY_SUB(2);
+        NEAR_HISTORY_SUB(3);
+        NEAR_HISTORY_SUB(4);
+        NEAR_HISTORY_SUB(5);
+        NEAR_HISTORY_SUB(6);
+        NEAR_HISTORY_SUB(7);
+    }
+#undef NEAR_HISTORY_SUB
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }
@@ -1325,8 +1365,7 @@ static int lod_enqueue(fpde_lod3d *L, cudaStream_t st, int64_t n0, int steps, in
                     if ((rc = launch_near_pre_ff(st, L->ringf, L->P, j0, L->wff, L->cfar, splits, 1, L->pre))) return rc;
                     ++k;
                 }
-                if ((rc = launch_near_history_ff(st, L->ringf, L->P, j, L->wff, L->cfar, splits, 1, L->Sn, nullptr, 0,
-                                                 use_pre ? L->pre : nullptr, j0)))
+                if ((rc = launch_near_history_sub(st, L->ringf, L->P, j, L->wff, L->Sn, use_pre ? L->pre : nullptr)))
                     return rc;
                 ++k;
                 KS = 1;
