@@ -54,6 +54,7 @@ int far3_launch(cudaStream_t st, const FarPlan3 *p, int k_cols, double *C, int64
 // weights w[n0 + j - t] of a block at n0 depend on its distance from a k-tile only, so their tiles
 // (distance 1 .. n_delta blocks) are formed once.
 struct Hist7 {
+    void *base = nullptr;  // the one allocation that holds all of them
     // half-tile-major slices: a box of the product (128 nodes or 64 steps x 32 columns) is contiguous
     uint16_t *a[7] = {};   // [2 n_delta half blocks][rows][32]
     uint16_t *w[7] = {};   // [2 n_delta][w_tiles 64][32]: column c of distance d, half c / 32: lag 64 d + j - c
