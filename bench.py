@@ -870,10 +870,10 @@ def _probe(line, u0_dev, steps, every):
 #   k_far_tc3 (two weight groups per item, a 256-step super-block): reads per row x history
 #     column, writes (the float-pair partials) per launch and row;
 #   k_line_block_spec: bytes per node-step (64 steps x 65,537 nodes per launch).
-NCU_FAR = {"read_per_row_col": 623.12e6 / (65664 * 1536), "write_per_row": 122.56e6 / 65664,
-           "source": "profiles/k_far_tc3_super_N65536_K1536.md"}
-NCU_SOLVE = {"per_node_step": (82.01e6 + 27.51e6) / (64 * 65537), "fp64_pipe_active": 0.4844,
-             "source": "profiles/k_line_block_spec_N65536_2048steps.md"}
+NCU_FAR = {"read_per_row_col": 514.54e6 / (65664 * 1280), "write_per_row": 108.04e6 / 65664,
+           "source": "profiles/k_far_tc3_super_N65536_K1280.md"}
+NCU_SOLVE = {"per_node_step": (43.63e6 + 12.77e6) / (64 * 65537), "fp64_pipe_active": 0.5169,
+             "source": "profiles/k_line_block_spec_N65536_400steps.md"}
 
 
 def _kernel_entry(t, name, peak, peak_src, scale=1.0):
