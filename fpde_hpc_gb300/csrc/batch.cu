@@ -370,8 +370,17 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
                 k += 2;
             }
             if (n >= 1) {                                            // far sums + the block's earlier rows
-                if ((rc = launch_near64(st, b->ring, b->Ptot, 0, j, b->wlag, nb0 > 0 ? b->cfar + (int64_t)j * b->Ptot : nullptr,
-                                        b->part, b->cta_col, b->col_lag, b->LW)))
+                // the rows before the step's 8-step sub-block go into its far sums once per sub-block
+                const int j0 = j - j % NEAR_SUB;
+                double *far = b->cfar + (int64_t)j * b->Ptot;
+                if (j == j0 && j0 > 0) {
+                    if ((rc = launch_near64_pre(st, b->ring, b->Ptot, j0, b->wlag, 64, nb0 > 0 ? far : nullptr, far,
+                                                b->cta_col, b->col_lag, b->LW)))
+                        return rc;
+                    ++k;
+                }
+                if ((rc = launch_near64(st, b->ring, b->Ptot, j0, j, b->wlag, nb0 > 0 || j0 > 0 ? far : nullptr, b->part,
+                                        b->cta_col, b->col_lag, b->LW)))
                     return rc;
                 ++k;
                 KS = 1;

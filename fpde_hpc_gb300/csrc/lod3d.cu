@@ -1308,9 +1308,18 @@ static int lod_enqueue(fpde_lod3d *L, cudaStream_t st, int64_t n0, int steps, in
                 }
             }
             if (n >= 1) {                                            // far sums + the block's earlier rows
-                const double *far = nb0 > kb0 ? L->cfar + (int64_t)j * L->P : nullptr;
-                const int r0 = std::max<int>(0, (int)std::min<int64_t>(j, j - (int64_t)L->max_lag));
-                if ((rc = launch_near64(st, L->ring, L->P, r0, j, L->wlag, far, L->part))) return rc;
+                // the rows before the step's 8-step sub-block go into its far sums once per sub-block
+                const int j0 = j - j % NEAR_SUB;
+                const int lag = (int)std::min<int64_t>(L->max_lag, 64);
+                double *far = L->cfar + (int64_t)j * L->P;
+                if (j == j0 && j0 > 0) {
+                    if ((rc = launch_near64_pre(st, L->ring, L->P, j0, L->wlag, lag, nb0 > kb0 ? far : nullptr, far)))
+                        return rc;
+                    ++k;
+                }
+                if ((rc = launch_near64(st, L->ring, L->P, std::max(j0, j - lag), j, L->wlag,
+                                        nb0 > kb0 || j0 > 0 ? far : nullptr, L->part)))
+                    return rc;
                 ++k;
                 KS = 1;
             }

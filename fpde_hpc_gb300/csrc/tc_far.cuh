@@ -77,6 +77,11 @@ void hist7_free(Hist7 *h);
 int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t wstride);
 // The finished block [n0 - 64, n0) of increments (64 rows of P) into the slices.
 int hist7_convert(cudaStream_t st, const Hist7 &h, const double *rows64, int64_t P, int64_t nvalid, int64_t n0);
+// out[u P + i] = init[u P + i] + sum_{0 <= r < j0} w[j0 + u - r] rows_r[i], u < 8, over the lags up to `lag`
+// (per column with col_lag), in FP64; init may be null (0) or out itself. j0 is a multiple of 8.
+int launch_near64_pre(cudaStream_t st, const double *rows, int64_t P, int j0, const double *wlag, int lag,
+                      const double *init, double *out, const int *cta_col = nullptr, const int *col_lag = nullptr,
+                      int64_t wstride = 0);
 // S[i] = init[i] + sum_{r0 <= r < j} w[j - r] rows_r[i] in FP64 (init may be null; per-column weights and
 // windows with cta_col and col_lag).
 int launch_near64(cudaStream_t st, const double *rows, int64_t P, int r0, int j, const double *wlag, const double *init,
