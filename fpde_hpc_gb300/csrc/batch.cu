@@ -14,11 +14,13 @@
 //                        solution, its last y and first u; the column's last chunk to finish solves
 //                        the column's chunk-level recurrences for every chunk's carries
 //   3. k_batch_join    : u = u^chunk + c_in KF + c_out CB, writing U and D_n
+// FP64 where the digit slices and weight tiles fit: step 1 becomes k_far_tc7 per 64-step block, k_near64_pre
+// per 8 steps and k_near64 per step, as for the 3D grids.
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
 // three-slice tensor-core contraction of all history before the block with one weight tile
 // per column (tc_far.cu; each 128-row tile picks its column's tile), and per step the near
-// history in float-float from a 64-row float-pair ring (k_near_pre_ff, k_near_history_sub); the solve writes
-// each increment to that ring and to the FP64 one the conversion reads.
+// history in float-float from a 64-row float-pair ring (k_near_pre_ff, k_near_history_sub); the solve
+// writes each increment to that ring and to the FP64 one the conversion reads.
 // The alpha recurrence is time-invariant and precomputed on the host per column.
 #include <algorithm>
 #include <cmath>

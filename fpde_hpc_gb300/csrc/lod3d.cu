@@ -8,6 +8,9 @@
 //   3. _M pass       : lines along j for every (i, k); Om = -lam U
 //   4. sN pass       : lines along i for every (j, k); Om = -lam U
 //   5. append        : D_n = U - U_old over the grid (the snapshot of the step, :5733-5745)
+// FP64 with lag weights, where the digit slices fit: step 1 becomes, per 64-step block, the seven-slice
+// tensor-core contraction of all history before the block (k_far_tc7), and the block's own rows in FP64
+// (k_near64_pre once per 8 steps, k_near64 per step).
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
 // three-slice tensor-core contraction of all history before the block (tc_far.cu, as for
 // lines) and, per step, k_near_history_sub: the far partials plus the near history in

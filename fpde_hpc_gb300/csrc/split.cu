@@ -7,6 +7,8 @@
 // The power-of-two scales keep fp16 operands inside its normal range; they are exact, and
 // A*W keeps its value up to the single global factor 2^kexp undone in the epilogue.
 // bf16 has float's exponent range and runs unscaled (sexp = kexp = 0).
+// Three slices (k_convert3, k_wgen3) and seven slices (k_convert7, k_wgen7) are exact digits with a block
+// exponent each, stored k-tile by k-tile; k_near64_pre and k_near64 sum a block's own rows in FP64.
 #include <algorithm>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
