@@ -1,11 +1,12 @@
 // 1D line problem (fpde_line_*): the plain FP64 path and the split-precision path.
 //
 // Per time step n (fpde_hpc_1d.cpp calc_step / U1 with the history applied every step):
-//   FP64 path, blocks of 64 steps (the rule; lines without requested launch parameters)
-//     at n0:  k_far64: the history t < n0 of the block's 64 steps in one FP64 product
+//   FP64 path, blocks of 64 steps (the rule)
+//     at n0:  k_far_tc7: the history t < n0 for the block's 64 steps on the tensor cores, exact digit
+//             products with FP64 accuracy (k_far64, in FP64, where the digit slices do not fit)
 //     steps of the block: k_line_block_spec as on the split path, its near history in FP64 too
-//   FP64 path, one launch each per step (requested launch parameters, lines of over 1,024 nodes
-//   per SM)
+//   FP64 path, one launch each per step (explicit part, Richards, requested GEMV splits, lines of over
+//   1,024 nodes per SM)
 //     1. k_l1_partial : part[ks][i] = sum_t w[n-t] D_t[i]        (FP64 history GEMV)
 //     2. k_line_solve : S = sum_ks part, Om = -lam U + src + S, Thomas solve, U <- U^{n+1},
 //                       D_n = U^{n+1} - U^n
