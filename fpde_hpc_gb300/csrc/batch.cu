@@ -689,7 +689,7 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
                 dev_alloc((void **)&b->cta_col, cta_col.size() * sizeof(int)) ||
                 (any_restrict && dev_alloc((void **)&b->col_lag, (size_t)n_cols * sizeof(int)));
     if (!fail && want7) {
-        b->x7 = hist7_alloc(&b->h7, &b->plan7, tot, max_steps, n_cols) == FPDE_OK;
+        b->x7 = hist7_alloc(ctx->stream, &b->h7, &b->plan7, tot, max_steps, n_cols) == FPDE_OK;
         if (!b->x7) clear_error();                                     // FP64 rows instead (8 bytes against 14)
     }
     if (!fail && b->x7) {

@@ -2034,7 +2034,7 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     if (!fail && b64 && L->max_steps > BLK) {
         // the far history in bf16 slices on the tensor cores; where they do not fit (14 bytes per node and
         // step against 8), FP64 rows and k_far64
-        L->x7 = hist7_alloc(&L->h7, &L->plan7, N + 1, L->max_steps, 1) == FPDE_OK;
+        L->x7 = hist7_alloc(ctx->stream, &L->h7, &L->plan7, N + 1, L->max_steps, 1) == FPDE_OK;
         if (!L->x7) clear_error();
     }
     if (!fail && !L->split) {

@@ -1580,7 +1580,7 @@ int fpde_lod3d_create(fpde_ctx *ctx, const fpde_lod3d_desc *desc, const double *
         // with the sums' rounding); rows of FP64 where the slices do not fit (14 bytes per node and step
         // against 8)
         if (!rich && !sfd && !vart && d.max_steps > 64) {
-            L->x7 = hist7_alloc(&L->h7, &L->plan7, L->G, d.max_steps, 1) == FPDE_OK;
+            L->x7 = hist7_alloc(ctx->stream, &L->h7, &L->plan7, L->G, d.max_steps, 1) == FPDE_OK;
             if (!L->x7) clear_error();
         }
         if (L->x7) {

@@ -466,7 +466,7 @@ int launch_near64(cudaStream_t st, const double *rows, int64_t P, int r0, int j,
     return FPDE_OK;
 }
 
-int hist7_alloc(Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles)
+int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles)
 {
     h->rows = (nodes + 127) / 128 * 128;
     h->n_delta = (max_steps - 1) / 64;
@@ -503,9 +503,11 @@ int hist7_alloc(Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles
         for (int q = 0; q < 7; ++q) { a[q] = h->a[q]; w[q] = h->w[q]; }
         rc = far_plan7_init(p, a, h->rows, h->n_delta, w, w_tiles);
     }
-    // rows past the nodes are never converted: their (unused) sums only need readable exponents
-    if (!rc && (cudaMemset(h->pA, 0, (size_t)h->rows * h->n_delta * sizeof(int16_t)) != cudaSuccess ||
-                cudaMemset(h->eA, 0, (size_t)h->rows * sizeof(int16_t)) != cudaSuccess))
+    // rows past the nodes are never converted: their (unused) sums only need readable exponents. On the
+    // context's stream: it does not wait for the default one, where a clear could still be queued when the
+    // first blocks are converted
+    if (!rc && (cudaMemsetAsync(h->pA, 0, (size_t)h->rows * h->n_delta * sizeof(int16_t), st) != cudaSuccess ||
+                cudaMemsetAsync(h->eA, 0, (size_t)h->rows * sizeof(int16_t), st) != cudaSuccess))
         rc = FPDE_ERR_CUDA;
     if (rc) hist7_free(h);
     return rc;

@@ -70,8 +70,8 @@ struct FarPlan7 {
     int64_t rows = 0;
     uint32_t idesc = 0;
 };
-// Allocate for `nodes` rows and max_steps columns (FPDE_ERR_NOMEM leaves nothing behind), free.
-int hist7_alloc(Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles);
+// Allocate for `nodes` rows and max_steps columns (FPDE_ERR_NOMEM leaves nothing behind; clears on st), free.
+int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles);
 void hist7_free(Hist7 *h);
 // Weight tiles from w[lag] (w_tiles rows of wstride values, lag < 64 n_delta + 64), once.
 int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t wstride);
