@@ -14,7 +14,7 @@
 //                        solution, its last y and first u; the column's last chunk to finish solves
 //                        the column's chunk-level recurrences for every chunk's carries
 //   3. k_batch_join    : u = u^chunk + c_in KF + c_out CB, writing U and D_n
-// FP64 where the digit slices and weight tiles fit: step 1 becomes k_far_tc7 per 64-step block, k_near64_pre
+// FP64 where the digit slices and weight tiles fit and every column's weights allow them: step 1 becomes k_far_tc7 per 64-step block, k_near64_pre
 // per 8 steps and k_near64 per step, as for the 3D grids.
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
 // three-slice tensor-core contraction of all history before the block with one weight tile
@@ -366,7 +366,7 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
             const int j = (int)(n - nb0);
             if (j == 0 && nb0 > 0) {
                 if ((rc = hist7_convert(st, b->h7, b->ring, b->Ptot, b->Ptot, nb0))) return rc;
-                if ((rc = far7_launch(st, &b->plan7, b->h7, 0, (int)nb0, b->cfar, (int64_t)64 * b->Ptot, b->Ptot, 1,
+                if ((rc = far7_launch(st, &b->plan7, b->h7, (int)nb0, b->cfar, (int64_t)64 * b->Ptot, b->Ptot, 1,
                                       b->ctx->d_flags, b->wcol)))
                     return rc;
                 k += 2;
@@ -376,13 +376,13 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
                 const int j0 = j - j % NEAR_SUB;
                 double *far = b->cfar + (int64_t)j * b->Ptot;
                 if (j == j0 && j0 > 0) {
-                    if ((rc = launch_near64_pre(st, b->ring, b->Ptot, j0, b->wlag, 64, nb0 > 0 ? far : nullptr, far,
-                                                b->cta_col, b->col_lag, b->LW)))
+                    if ((rc = launch_near64_pre(st, b->ring, b->Ptot, j0, b->wlag, nb0 > 0 ? far : nullptr, far,
+                                                b->cta_col, b->LW)))
                         return rc;
                     ++k;
                 }
-                if ((rc = launch_near64(st, b->ring, b->Ptot, j0, j, b->wlag, nb0 > 0 || j0 > 0 ? far : nullptr, b->part,
-                                        b->cta_col, b->col_lag, b->LW)))
+                if ((rc = launch_near64(st, b->ring, b->Ptot, j, b->wlag, nb0 > 0 || j0 > 0 ? far : nullptr, b->part,
+                                        b->cta_col, b->LW)))
                     return rc;
                 ++k;
                 KS = 1;
@@ -659,7 +659,7 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
     std::vector<int> hwcol;                                            // column of each 128-row tile
     // FP64 runs of more than a block also take the tables (up to 4 GB of weight tiles, 56 KB per column
     // and distance)
-    const bool want7 = !split && max_steps > 64 && (int64_t)n_cols * ((max_steps - 1) / 64) * 57344 <= (4ll << 30);
+    bool want7 = !split && max_steps > 64 && (int64_t)n_cols * ((max_steps - 1) / 64) * 57344 <= (4ll << 30);
     if (split || want7) {
         hwl.assign((size_t)n_cols * b->LW, 0.0);
         hwcol.assign(tot / 128, 0);
@@ -674,6 +674,7 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
             for (int64_t q = o / 128; q < (o + Pc) / 128; ++q) hwcol[q] = c;
         }
     }
+    for (int c = 0; c < n_cols && want7; ++c) want7 = slices7_hold(hwl.data() + (size_t)c * b->LW, max_steps - 1);
     const size_t tb = (size_t)tot * sizeof(double);
     bool fail = dev_alloc((void **)&b->ga, tb) || dev_alloc((void **)&b->g, tb) || dev_alloc((void **)&b->al, tb) ||
                 dev_alloc((void **)&b->lane, hlane.size() * sizeof(double)) ||

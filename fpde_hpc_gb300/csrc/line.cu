@@ -3,7 +3,8 @@
 // Per time step n (fpde_hpc_1d.cpp calc_step / U1 with the history applied every step):
 //   FP64 path, blocks of 64 steps (the rule)
 //     at n0:  k_far_tc7: the history t < n0 for the block's 64 steps on the tensor cores, exact digit
-//             products with FP64 accuracy (k_far64, in FP64, where the digit slices do not fit)
+//             products with FP64 accuracy (k_far64, in FP64, where the digit slices do not fit or the
+//             weights rule them out: windows, steeply falling weights)
 //     steps of the block: k_line_block_spec as on the split path, its near history in FP64 too
 //   FP64 path, one launch each per step (explicit part, Richards, requested GEMV splits, lines of over
 //   1,024 nodes per SM)
@@ -1461,15 +1462,14 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
         if (L->b64) {
             const int64_t nb0 = n - n % BLK, t0 = nb0 > L->max_lag ? nb0 - L->max_lag : 0;
             const int j = (int)(n - nb0);
-            const int64_t kb0 = t0 / BLK * BLK;                      // the oldest 64-step tile in the window
-            const int splits = nb0 == t0 ? 0 : L->x7 ? far_splits((int)((nb0 - kb0) / BLK), L->h7.rows) : 1;
+            const int splits = nb0 == t0 ? 0 : L->x7 ? far_splits((int)(nb0 / BLK), L->h7.rows) : 1;
             if (j == 0 && L->x7 && nb0 > 0) {
                 if ((rc = hist7_convert(st, L->h7, L->ring, L->P, L->N + 1, nb0))) return rc;
                 ++k;
             }
             if (j == 0 && splits > 0) {
                 if (L->x7) {
-                    if ((rc = far7_launch(st, &L->plan7, L->h7, (int)kb0, (int)nb0, L->cfar, (int64_t)BLK * L->P, L->P, splits,
+                    if ((rc = far7_launch(st, &L->plan7, L->h7, (int)nb0, L->cfar, (int64_t)BLK * L->P, L->P, splits,
                                           L->ctx->d_flags)))
                         return rc;
                 } else if ((rc = launch_far64(st, L->D, L->P, L->N, t0, nb0, L->wlag, L->cfar))) {
@@ -2031,9 +2031,9 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
                 (spec && (dev_alloc((void **)&L->sclane, hsl.size() * sizeof(double)) ||
                            dev_alloc((void **)&L->scwarp, hsw.size() * sizeof(double)))) ||
                 dev_alloc((void **)&L->barrier, 2 * sizeof(unsigned));
-    if (!fail && b64 && L->max_steps > BLK) {
+    if (!fail && b64 && L->max_steps > BLK && slices7_hold(wlag.data(), L->max_steps - 1)) {
         // the far history in bf16 slices on the tensor cores; where they do not fit (14 bytes per node and
-        // step against 8), FP64 rows and k_far64
+        // step against 8) or the weights rule them out, FP64 rows and k_far64
         L->x7 = hist7_alloc(ctx->stream, &L->h7, &L->plan7, N + 1, L->max_steps, 1) == FPDE_OK;
         if (!L->x7) clear_error();
     }

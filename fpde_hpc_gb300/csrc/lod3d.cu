@@ -8,7 +8,7 @@
 //   3. _M pass       : lines along j for every (i, k); Om = -lam U
 //   4. sN pass       : lines along i for every (j, k); Om = -lam U
 //   5. append        : D_n = U - U_old over the grid (the snapshot of the step, :5733-5745)
-// FP64 with lag weights, where the digit slices fit: step 1 becomes, per 64-step block, the seven-slice
+// FP64 with lag weights, where the digit slices fit and the weights allow them (slices7_hold): step 1 becomes, per 64-step block, the seven-slice
 // tensor-core contraction of all history before the block (k_far_tc7), and the block's own rows in FP64
 // (k_near64_pre once per 8 steps, k_near64 per step).
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
@@ -1299,29 +1299,21 @@ static int lod_enqueue(fpde_lod3d *L, cudaStream_t st, int64_t n0, int steps, in
         } else if (L->x7) {
             const int64_t nb0 = n - n % 64;
             const int j = (int)(n - nb0);
-            const int64_t kb0 = nb0 > L->max_lag ? (nb0 - L->max_lag) / 64 * 64 : 0;
             if (j == 0 && nb0 > 0) {
                 if ((rc = hist7_convert(st, L->h7, L->ring, L->P, L->G, nb0))) return rc;
-                ++k;
-                if (nb0 > kb0) {
-                    if ((rc = far7_launch(st, &L->plan7, L->h7, (int)kb0, (int)nb0, L->cfar, (int64_t)64 * L->P, L->P, 1,
-                                          L->ctx->d_flags)))
-                        return rc;
-                    ++k;
-                }
+                if ((rc = far7_launch(st, &L->plan7, L->h7, (int)nb0, L->cfar, (int64_t)64 * L->P, L->P, 1, L->ctx->d_flags)))
+                    return rc;
+                k += 2;
             }
             if (n >= 1) {                                            // far sums + the block's earlier rows
                 // the rows before the step's 8-step sub-block go into its far sums once per sub-block
                 const int j0 = j - j % NEAR_SUB;
-                const int lag = (int)std::min<int64_t>(L->max_lag, 64);
                 double *far = L->cfar + (int64_t)j * L->P;
                 if (j == j0 && j0 > 0) {
-                    if ((rc = launch_near64_pre(st, L->ring, L->P, j0, L->wlag, lag, nb0 > kb0 ? far : nullptr, far)))
-                        return rc;
+                    if ((rc = launch_near64_pre(st, L->ring, L->P, j0, L->wlag, nb0 > 0 ? far : nullptr, far))) return rc;
                     ++k;
                 }
-                if ((rc = launch_near64(st, L->ring, L->P, std::max(j0, j - lag), j, L->wlag,
-                                        nb0 > kb0 || j0 > 0 ? far : nullptr, L->part)))
+                if ((rc = launch_near64(st, L->ring, L->P, j, L->wlag, nb0 > 0 || j0 > 0 ? far : nullptr, L->part)))
                     return rc;
                 ++k;
                 KS = 1;
@@ -1578,15 +1570,17 @@ int fpde_lod3d_create(fpde_ctx *ctx, const fpde_lod3d_desc *desc, const double *
         // blocks of 64 steps, the older history in bf16 slices on the tensor cores, for the passes with
         // constant coefficients (space-fractional solves stop at a threshold, so their iterates would move
         // with the sums' rounding); rows of FP64 where the slices do not fit (14 bytes per node and step
-        // against 8)
+        // against 8) or the weights rule them out
+        const int64_t LW = L->max_steps + 64 + 1;
         if (!rich && !sfd && !vart && d.max_steps > 64) {
+            wlag.assign(LW, 0.0);
+            for (int64_t j = 1; j < LW; ++j) wlag[j] = wlag_at(j);
+        }
+        if (!wlag.empty() && slices7_hold(wlag.data(), L->max_steps - 1)) {
             L->x7 = hist7_alloc(ctx->stream, &L->h7, &L->plan7, L->G, d.max_steps, 1) == FPDE_OK;
             if (!L->x7) clear_error();
         }
         if (L->x7) {
-            const int64_t LW = L->max_steps + 64 + 1;
-            wlag.assign(LW, 0.0);
-            for (int64_t j = 1; j < LW; ++j) wlag[j] = wlag_at(j);
             fail = dev_alloc((void **)&L->ring, 64 * pbytes) || dev_alloc((void **)&L->cfar, 64 * pbytes) ||
                    dev_alloc((void **)&L->part, pbytes) || dev_alloc((void **)&L->wlag, LW * sizeof(double));
         } else {

@@ -10,6 +10,8 @@
 // Three slices (k_convert3, k_wgen3) and seven slices (k_convert7, k_wgen7) are exact digits with a block
 // exponent each, stored k-tile by k-tile; k_near64_pre and k_near64 sum a block's own rows in FP64.
 #include <algorithm>
+#include <cmath>
+#include <vector>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -377,93 +379,97 @@ __global__ void __launch_bounds__(64) k_wgen7(const double *__restrict__ wlag_al
 
 // Near history of a 64-step block in FP64, one node per thread, in sub-blocks of 8 steps: k_near64_pre adds
 // the block's rows before j0 to the far sums of the steps j0 .. j0 + 7 (out[u] = init[u] + sum_{r < j0}
-// w[j0 + u - r] D_r), k_near64 a step's own sub-block rows (S = init + sum_{r0 <= r < j} w[j - r] D_r); the
+// w[j0 + u - r] D_r), k_near64 a step's own sub-block rows (S = init + sum_{j0 <= r < j} w[j - r] D_r); the
 // order of the sums is that of one pass over the rows. FP64-pipe bound: one multiply-add per row and step.
 // k_near64_pre keeps the pipe 96 % busy. Read again for every step the rows bound it instead: 19.9 us per
 // step for 284,000 nodes (20.6 in one pass per step), 14.0 for 96 columns of 200 to 5,000 nodes (16.7).
 // CTAs of 64 nodes give the SMs equal shares (512 nodes: 22.2 and 17.5 in one pass).
 constexpr int N64_T = 64;
-__global__ void __launch_bounds__(N64_T) k_near64(const double *__restrict__ rows, int64_t P, int r0, int j,
+__global__ void __launch_bounds__(N64_T) k_near64(const double *__restrict__ rows, int64_t P, int j,
                                                   const double *__restrict__ wlag, int64_t wstride,
-                                                  const int *__restrict__ cta_col, const int *__restrict__ col_lag,
-                                                  const double *__restrict__ init, double *__restrict__ S)
+                                                  const int *__restrict__ cta_col, const double *__restrict__ init,
+                                                  double *__restrict__ S)
 {
     const int64_t i = (int64_t)blockIdx.x * N64_T + threadIdx.x;
     if (i >= P) return;
     const double *w = wlag;
-    if (cta_col) {                                   // a 512-node group's column: its weights and window
-        const int c = cta_col[blockIdx.x / (512 / N64_T)];
-        w += (int64_t)c * wstride;
-        if (col_lag) r0 = max(r0, j - col_lag[c]);
-    }
+    if (cta_col) w += (int64_t)cta_col[blockIdx.x / (512 / N64_T)] * wstride;      // a 512-node group's column
     double s = init ? __ldcs(init + i) : 0.0;
-    int r = r0;
-    for (; r + 8 <= j; r += 8) {
-        double v[8];
+    const int r = j - j % NEAR_SUB;
+    double v[NEAR_SUB];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = __ldcg(rows + (int64_t)(r + u) * P + i);
+    for (int u = 0; u < NEAR_SUB; ++u) v[u] = r + u < j ? __ldcg(rows + (int64_t)(r + u) * P + i) : 0.0;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) s = fma(__ldg(w + (j - r - u)), v[u], s);
-    }
-    if (r < j) {                                     // the last rows, loaded together
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = r + u < j ? __ldcg(rows + (int64_t)(r + u) * P + i) : 0.0;
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (r + u < j) s = fma(__ldg(w + (j - r - u)), v[u], s);
-    }
+    for (int u = 0; u < NEAR_SUB; ++u)
+        if (r + u < j) s = fma(__ldg(w + (j - r - u)), v[u], s);
     S[i] = s;
 }
 
 __global__ void __launch_bounds__(N64_T) k_near64_pre(const double *__restrict__ rows, int64_t P, int j0,
-                                                      const double *__restrict__ wlag, int64_t wstride, int lag,
-                                                      const int *__restrict__ cta_col, const int *__restrict__ col_lag,
-                                                      const double *init, double *out)
+                                                      const double *__restrict__ wlag, int64_t wstride,
+                                                      const int *__restrict__ cta_col, const double *init, double *out)
 {
     const int64_t i = (int64_t)blockIdx.x * N64_T + threadIdx.x;
     if (i >= P) return;
     const double *w = wlag;
-    if (cta_col) {
-        const int c = cta_col[blockIdx.x / (512 / N64_T)];
-        w += (int64_t)c * wstride;
-        if (col_lag) lag = col_lag[c];
-    }
+    if (cta_col) w += (int64_t)cta_col[blockIdx.x / (512 / N64_T)] * wstride;
     double s[NEAR_SUB];
 #pragma unroll
     for (int u = 0; u < NEAR_SUB; ++u) s[u] = init ? init[(int64_t)u * P + i] : 0.0;
     for (int r = 0; r < j0; r += NEAR_SUB) {             // j0 is a multiple of NEAR_SUB
-        if (r + NEAR_SUB - 1 < j0 - lag) continue;       // before every step's window
         double v[NEAR_SUB];
 #pragma unroll
         for (int q = 0; q < NEAR_SUB; ++q) v[q] = __ldcg(rows + (int64_t)(r + q) * P + i);
-        const bool all = r >= j0 + NEAR_SUB - 1 - lag;   // inside every step's window
 #pragma unroll
         for (int q = 0; q < NEAR_SUB; ++q)
 #pragma unroll
-            for (int u = 0; u < NEAR_SUB; ++u)
-                if (all || r + q >= j0 + u - lag) s[u] = fma(__ldg(w + (j0 + u - r - q)), v[q], s[u]);
+            for (int u = 0; u < NEAR_SUB; ++u) s[u] = fma(__ldg(w + (j0 + u - r - q)), v[q], s[u]);
     }
 #pragma unroll
     for (int u = 0; u < NEAR_SUB; ++u) out[(int64_t)u * P + i] = s[u];
 }
 
-int launch_near64_pre(cudaStream_t st, const double *rows, int64_t P, int j0, const double *wlag, int lag,
-                      const double *init, double *out, const int *cta_col, const int *col_lag, int64_t wstride)
+int launch_near64_pre(cudaStream_t st, const double *rows, int64_t P, int j0, const double *wlag, const double *init,
+                      double *out, const int *cta_col, int64_t wstride)
 {
-    k_near64_pre<<<(unsigned)((P + N64_T - 1) / N64_T), N64_T, 0, st>>>(rows, P, j0, wlag, wstride, lag, cta_col, col_lag,
-                                                                        init, out);
+    k_near64_pre<<<(unsigned)((P + N64_T - 1) / N64_T), N64_T, 0, st>>>(rows, P, j0, wlag, wstride, cta_col, init, out);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }
 
-int launch_near64(cudaStream_t st, const double *rows, int64_t P, int r0, int j, const double *wlag, const double *init,
-                  double *S, const int *cta_col, const int *col_lag, int64_t wstride)
+int launch_near64(cudaStream_t st, const double *rows, int64_t P, int j, const double *wlag, const double *init,
+                  double *S, const int *cta_col, int64_t wstride)
 {
-    k_near64<<<(unsigned)((P + N64_T - 1) / N64_T), N64_T, 0, st>>>(rows, P, r0, j, wlag, wstride, cta_col, col_lag, init,
-                                                                    S);
+    k_near64<<<(unsigned)((P + N64_T - 1) / N64_T), N64_T, 0, st>>>(rows, P, j, wlag, wstride, cta_col, init, S);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
+}
+
+bool slices7_hold(const double *w, int64_t lags)
+{
+    constexpr double NEAR = 256.0, ALL = 1099511627776.0;          // 2^8, 2^40
+    if (lags < 1) return true;
+    std::vector<double> a(lags), hi(lags), lo(lags);
+    for (int64_t l = 0; l < lags; ++l) {
+        a[l] = std::fabs(w[l + 1]);
+        if (!(a[l] >= 2.2250738585072014e-308) || !std::isfinite(a[l])) return false;
+    }
+    const auto all = std::minmax_element(a.begin(), a.end());
+    if (*all.second > ALL * *all.first) return false;
+    // extremes of [l, l + 63]: from l to its group's end and from the next group's start to l + 63
+    for (int64_t l = lags - 1; l >= 0; --l) {
+        const bool end = l == lags - 1 || l % 64 == 63;
+        hi[l] = end ? a[l] : std::max(a[l], hi[l + 1]);
+        lo[l] = end ? a[l] : std::min(a[l], lo[l + 1]);
+    }
+    double h = 0.0, m = 0.0;
+    for (int64_t l = 0; l < lags; ++l) {
+        h = l % 64 == 0 ? a[l] : std::max(h, a[l]);
+        m = l % 64 == 0 ? a[l] : std::min(m, a[l]);
+        const int64_t first = std::max<int64_t>(l - 63, 0);
+        if (std::max(h, hi[first]) > NEAR * std::min(m, lo[first])) return false;
+    }
+    return true;
 }
 
 int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles)

@@ -733,7 +733,7 @@ __device__ __forceinline__ double scale_f64(double x, int e)
 struct Far7Args {
     double *C;
     int64_t ldc_split, ldc_col, rows;
-    int kt_begin, kt_end, kt_per, n_split;           // k-tiles [kt_begin, kt_end); the block's index is kt_end
+    int kt_end, kt_per, n_split;                     // k-tiles [0, kt_end); the block's index is kt_end
     const int16_t *pA;                               // [k-tile][rows]
     const int16_t *eA;                               // [rows]: largest pA of the row so far
     int w_rows;                                      // 64 per weight tile
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(F7_THREADS, 1) k_far_tc7(const __grid_constant
     auto k_range = [&](int item, int &mt, int &ks, int &k0, int &k1) {
         mt = item / p.n_split;
         ks = (item + (gridDim.x % p.n_split ? 0 : item / gridDim.x)) % p.n_split;
-        k0 = p.kt_begin + ks * p.kt_per;
+        k0 = ks * p.kt_per;
         k1 = min(k0 + p.kt_per, p.kt_end);
     };
 
@@ -1109,18 +1109,17 @@ int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int n_tile
     return FPDE_OK;
 }
 
-int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_begin, int k_cols, double *C, int64_t ldc_split,
+int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_cols, double *C, int64_t ldc_split,
                 int64_t ldc_col, int splits, unsigned *flags, const int *wcol)
 {
-    if (k_cols % tc::BK != 0 || k_begin % tc::BK != 0 || k_begin < 0 || k_begin > k_cols)
+    if (k_cols % tc::BK != 0 || k_cols < 0)
         return set_error(FPDE_ERR_ARG, "far contraction: K range must be in multiples of 64");
-    if (k_cols == k_begin) return FPDE_OK;
+    if (k_cols == 0) return FPDE_OK;
     tc::Far7Args a;
-    a.kt_begin = k_begin / tc::BK;
     a.kt_end = k_cols / tc::BK;
-    if (a.kt_end - a.kt_begin > h.n_delta) return set_error(FPDE_ERR_ARG, "far contraction: weight tiles out of range");
+    if (a.kt_end > h.n_delta) return set_error(FPDE_ERR_ARG, "far contraction: weight tiles out of range");
     splits = std::max(1, std::min(splits, FAR_MAX_SPLITS));
-    a.kt_per = (a.kt_end - a.kt_begin + splits - 1) / splits;      // every split is written, possibly with zeros
+    a.kt_per = (a.kt_end + splits - 1) / splits;                   // every split is written, possibly with zeros
     a.n_split = splits;
     a.C = C; a.ldc_split = ldc_split; a.ldc_col = ldc_col; a.rows = p->rows;
     a.pA = h.pA; a.eA = h.eA; a.w_rows = tc::BN * h.w_tiles; a.sW = h.sW; a.eW = h.eW; a.n_delta = h.n_delta; a.wcol = wcol;

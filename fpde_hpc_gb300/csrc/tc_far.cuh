@@ -77,19 +77,25 @@ void hist7_free(Hist7 *h);
 int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t wstride);
 // The finished block [n0 - 64, n0) of increments (64 rows of P) into the slices.
 int hist7_convert(cudaStream_t st, const Hist7 &h, const double *rows64, int64_t P, int64_t nvalid, int64_t n0);
-// out[u P + i] = init[u P + i] + sum_{0 <= r < j0} w[j0 + u - r] rows_r[i], u < 8, over the lags up to `lag`
-// (per column with col_lag), in FP64; init may be null (0) or out itself. j0 is a multiple of 8.
-int launch_near64_pre(cudaStream_t st, const double *rows, int64_t P, int j0, const double *wlag, int lag,
-                      const double *init, double *out, const int *cta_col = nullptr, const int *col_lag = nullptr,
-                      int64_t wstride = 0);
-// S[i] = init[i] + sum_{r0 <= r < j} w[j - r] rows_r[i] in FP64 (init may be null; per-column weights and
-// windows with cta_col and col_lag).
-int launch_near64(cudaStream_t st, const double *rows, int64_t P, int r0, int j, const double *wlag, const double *init,
-                  double *S, const int *cta_col = nullptr, const int *col_lag = nullptr, int64_t wstride = 0);
+// Whether the slices hold the sums of the lag weights w[1 .. lags] with FP64's accuracy. A block's increments
+// and a tile's weights are fixed-point numbers of 62 bits below the largest, so a small product keeps
+// few bits beside a large increment; that is no loss while the large one enters the same sum with a weight that
+// is not much smaller, and it is one where it carries none (a window) or hardly any. So: no weight is 0, any
+// 64 neighbouring ones lie within a factor of 2^8 (1 at most 45 for Caputo weights of any order in (0, 1)) and all
+// within 2^40 (the accumulators' floats reach 2^-100 below the largest block and tile). A window of 3 lags in
+// which increments fell by 1.4 binary orders per step was off by 0.93 of the state, weights of 2^-l by 5e-9.
+bool slices7_hold(const double *w, int64_t lags);
+// out[u P + i] = init[u P + i] + sum_{0 <= r < j0} w[j0 + u - r] rows_r[i], u < 8, in FP64; init may be null (0)
+// or out itself. j0 is a multiple of 8. Per-column weights with cta_col.
+int launch_near64_pre(cudaStream_t st, const double *rows, int64_t P, int j0, const double *wlag, const double *init,
+                      double *out, const int *cta_col = nullptr, int64_t wstride = 0);
+// S[i] = init[i] + sum_{j - j % 8 <= r < j} w[j - r] rows_r[i] in FP64 (init may be null).
+int launch_near64(cudaStream_t st, const double *rows, int64_t P, int j, const double *wlag, const double *init,
+                  double *S, const int *cta_col = nullptr, int64_t wstride = 0);
 int far_plan7_init(FarPlan7 *p, const void *const a[7], int64_t rows, int n_tiles, const void *const w[7], int w_tiles);
-// C[split ldc_split + j ldc_col + row] = sum over the split's share of columns [k_begin, k_cols) of
+// C[split ldc_split + j ldc_col + row] = sum over the split's share of columns [0, k_cols) of
 // A[row][t] w[k_cols + j - t], j < 64, in FP64.
-int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_begin, int k_cols, double *C, int64_t ldc_split,
+int far7_launch(cudaStream_t st, const FarPlan7 *p, const Hist7 &h, int k_cols, double *C, int64_t ldc_split,
                 int64_t ldc_col, int splits, unsigned *flags, const int *wcol = nullptr);
 
 // float -> double from the bits (integer instructions only; exact for every float).
