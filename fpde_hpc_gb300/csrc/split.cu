@@ -266,19 +266,20 @@ __global__ void __launch_bounds__(64) k_wgen3(const double *__restrict__ wlag_al
 }
 
 // ---- seven-slice form: x 2^-pe = sum_s a_s 2^-9s, |x| < 2^(pe+8), balanced base-512 digits |a_s| <= 256
-// of the 63-bit integer v = rint(x 2^(54-pe)); each digit is stored as the bf16 value a_s 2^-9s (exact).
+// of the 63-bit integer v = rint(x 2^(54-pe)); each digit is stored as the bf16 value a_s 2^-9s (exact). Blocks
+// below the normal range keep the exponent of its lower end.
 __device__ __forceinline__ int exp7_of_maxbits(unsigned long long mbits)
 {
     const int ex = (int)((mbits >> 52) & 0x7FF);
-    return ex == 0 ? PE7_ZERO : ex - 1023 + 1 - 8;
+    return mbits == 0 ? PE7_ZERO : max(ex, 1) - 1023 + 1 - 8;
 }
 __device__ __forceinline__ void digits7(unsigned long long bits, int pe, uint16_t (&s)[7])
 {
     const int ex = (int)((bits >> 52) & 0x7FF);
+    const long long mant = (long long)(bits & 0xFFFFFFFFFFFFFull) | (ex ? 1ll << 52 : 0ll);
     long long v = 0;
-    if (ex != 0) {                                   // zero and subnormal values count as 0
-        const long long mant = (long long)((bits & 0xFFFFFFFFFFFFFull) | (1ull << 52));
-        const int r = pe + 1021 - ex;                // >= -9: within 9 binary orders of the largest, exact
+    if (mant != 0) {
+        const int r = pe + 1021 - max(ex, 1);        // >= -9: within 9 binary orders of the largest, exact
         if (r <= 0) v = mant << min(-r, 9);
         else if (r < 62) {
             const long long q = mant >> r, rem = mant & ((1ll << r) - 1), half = 1ll << (r - 1);
