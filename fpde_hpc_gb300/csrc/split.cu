@@ -267,11 +267,12 @@ __global__ void __launch_bounds__(64) k_wgen3(const double *__restrict__ wlag_al
 
 // ---- seven-slice form: x 2^-pe = sum_s a_s 2^-9s, |x| < 2^(pe+8), balanced base-512 digits |a_s| <= 256
 // of the 63-bit integer v = rint(x 2^(54-pe)); each digit is stored as the bf16 value a_s 2^-9s (exact). Blocks
-// below the normal range keep the exponent of its lower end.
+// below the normal range keep the exponent of its lower end; one with an infinity or a NaN has PE7_NONFINITE and
+// zero digits, and every sum of its row is NaN.
 __device__ __forceinline__ int exp7_of_maxbits(unsigned long long mbits)
 {
     const int ex = (int)((mbits >> 52) & 0x7FF);
-    return mbits == 0 ? PE7_ZERO : max(ex, 1) - 1023 + 1 - 8;
+    return mbits == 0 ? PE7_ZERO : ex == 0x7FF ? PE7_NONFINITE : max(ex, 1) - 1023 + 1 - 8;
 }
 __device__ __forceinline__ void digits7(unsigned long long bits, int pe, uint16_t (&s)[7])
 {

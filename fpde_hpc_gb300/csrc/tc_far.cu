@@ -946,9 +946,11 @@ __global__ void __launch_bounds__(F7_THREADS, 1) k_far_tc7(const __grid_constant
                         double d[2];
                         value(j, d);
 #pragma unroll
-                        for (int u = 0; u < 2; ++u)
+                        for (int u = 0; u < 2; ++u) {
+                            const int e = ea + __shfl_sync(0xffffffffu, ew, 2 * j + u);
                             out[(int64_t)(2 * j + u) * p.ldc_col] =
-                                scale_f64(d[u], ea + __shfl_sync(0xffffffffu, ew, 2 * j + u));
+                                eA == PE7_NONFINITE ? __longlong_as_double(0x7FF8000000000000ll) : scale_f64(d[u], e);
+                        }
                     }
                 }
             }

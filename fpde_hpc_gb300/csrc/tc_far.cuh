@@ -64,7 +64,7 @@ struct Hist7 {
     int64_t rows = 0;
     int n_delta = 0, w_tiles = 1;
 };
-constexpr int PE7_ZERO = -4096;                // exponent of an all-zero block
+constexpr int PE7_ZERO = -4096, PE7_NONFINITE = 4096;   // exponents of an all-zero block, of one with Inf or NaN
 struct FarPlan7 {
     alignas(64) unsigned char maps[14 * 128];
     int64_t rows = 0;
