@@ -308,9 +308,10 @@ __global__ void __launch_bounds__(32 * (2 * W + 1), 1) k_rich_step(RichLineArgs 
     }
     const int k = warp * 32 + lane, i = a + k;          // solve warps: this lane's node
     const bool solve = warp < W, in = solve && i < N;
-    double uo = 0.0, kk = 0.0, om = 0.0;
+    double uo = 0.0, lo = 0.0, kk = 0.0, om = 0.0;
     if (in) {
         uo = p.U[i];
+        lo = p.last[i];
         double sv = 0.0;                                // the history partials, four chains of loads
         double s1 = 0.0, s2 = 0.0, s3 = 0.0;
         int q = 0;
@@ -572,9 +573,10 @@ __global__ void __launch_bounds__(32 * (2 * W + 1), 1) k_rich_step(RichLineArgs 
     }
     __syncthreads();
     if (s_abort) return;
-    // ---- the new state, its increment and (split history) the increment as a float pair
-    auto put = [&](int q, double un, double old) {
-        const double d = un - old;
+    // ---- the new state, its increment and (split history) the increment as a float pair. The increment counts
+    // from the last computed state, whatever the caller has written to U since (as k_append's)
+    auto put = [&](int q, double un, double before) {
+        const double d = un - before;
         p.U[q] = un;
         p.last[q] = un;
         p.Drow[q] = d;
@@ -583,11 +585,11 @@ __global__ void __launch_bounds__(32 * (2 * W + 1), 1) k_rich_step(RichLineArgs 
     double u = 0.0;
     if (in) {
         u = fma(Q, sCarry[3], fma(K, sCarry[0], Ub));
-        put(i, u, uo);
-        if (i == N - 1) put(N, sEdge[1], p.U[N]);
+        put(i, u, lo);
+        if (i == N - 1) put(N, sEdge[1], p.last[N]);
     }
     if (c == 0 && tid == 0) {
-        put(0, __dadd_rn(__dmul_rn(sCarry[1], u), sCarry[2]), p.U[0]);   // Al[1] U[1] + Bt[1]
+        put(0, __dadd_rn(__dmul_rn(sCarry[1], u), sCarry[2]), p.last[0]);   // Al[1] U[1] + Bt[1]
         *((volatile unsigned long long *)p.seq) = seq;  // every CTA has read it (it published)
     }
 }
