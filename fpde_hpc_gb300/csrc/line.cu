@@ -391,8 +391,6 @@ struct LineBlockArgs {
     int j0, nsteps, N, G, rkind, chunk;
 };
 
-constexpr unsigned long long SLOT_EMPTY = ~0ull;        // exchange slot not yet written (a NaN pattern)
-
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const double *p)
 {
     unsigned long long v;
@@ -402,8 +400,7 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const double *p)
 
 __device__ __forceinline__ void st_relaxed_f64(double *p, double v)
 {
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((unsigned long long)__double_as_longlong(v))
-                 : "memory");
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(slot_bits(v)) : "memory");
 }
 
 __device__ __forceinline__ void solver_sync() { asm volatile("bar.sync 1, %0;" ::"n"(LTS) : "memory"); }

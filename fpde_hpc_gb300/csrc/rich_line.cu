@@ -249,20 +249,18 @@ __global__ void __launch_bounds__(RT, 1) k_rich_thomas(RichLineArgs p)
 
 // ------------------------------------------------------------------ the step over all SMs
 
-constexpr unsigned long long RSLOT_EMPTY = ~0ull;       // slot not yet written (a NaN no arithmetic makes)
-
 __device__ __forceinline__ double rslot_load(const double *p, bool &got)
 {
     unsigned long long v;
     asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    if (v == RSLOT_EMPTY) got = false;
+    if (v == SLOT_EMPTY) got = false;
     return __longlong_as_double((long long)v);
 }
-__device__ __forceinline__ void rslot_store(double *p, double v)
+__device__ __forceinline__ void rslot_store_bits(double *p, unsigned long long v)
 {
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((unsigned long long)__double_as_longlong(v))
-                 : "memory");
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ void rslot_store(double *p, double v) { rslot_store_bits(p, slot_bits(v)); }
 
 __device__ __forceinline__ Mob shfl_down_mob(const Mob &m, int o)
 {
@@ -331,8 +329,7 @@ __global__ void __launch_bounds__(32 * (2 * W + 1), 1) k_rich_step(RichLineArgs 
     const unsigned long long seq = s_seq;
     double *slots = p.slots + (seq & 1) * (size_t)(16 * G);
     if (warp == 2 * W && lane < 16)                     // empty this chunk's slots for the next launch
-        rslot_store(p.slots + ((seq & 1) ^ 1) * (size_t)(16 * G) + 16 * c + lane,
-                    __longlong_as_double((long long)RSLOT_EMPTY));
+        rslot_store_bits(p.slots + ((seq & 1) ^ 1) * (size_t)(16 * G) + 16 * c + lane, SLOT_EMPTY);
 
     // ---- coefficients (A_/B/R) and the alpha maps; inclusive products over the CTA's nodes
     double cA = 0.0, cB = 1.0, cBl = 1.0;               // A, B, B + l

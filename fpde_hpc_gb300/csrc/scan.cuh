@@ -33,4 +33,13 @@ __device__ __forceinline__ unsigned long long gtimer_ns()
     return t;
 }
 
+// Exchange slots that are polled as values: empty is the NaN of all ones. Arithmetic passes the bits of an
+// input's NaN on, so a value with this pattern travels as another NaN.
+constexpr unsigned long long SLOT_EMPTY = ~0ull;
+__device__ __forceinline__ unsigned long long slot_bits(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return b == SLOT_EMPTY ? 0xFFF8000000000000ull : b;
+}
+
 }  // namespace fpde

@@ -1,11 +1,13 @@
-"""A Richards line whose state the caller writes between runs: the increment of the next step counts from the
-last computed state."""
+"""Lines whose inputs hold a NaN, whatever its bits (a 64-bit pattern of ones marks an empty exchange slot of
+the block solve and of the Richards step): the result is NaN, not an error. A Richards line whose state the
+caller writes between runs: the increment of the next step counts from the last computed state."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
 from conftest import relmax
+from test_gpu_far7 import _problem
 from test_gpu_richards_step import _case
 
 pytestmark = pytest.mark.gpu
@@ -17,6 +19,37 @@ def ctx():
     c = fp.Context(0)
     yield c
     c.close()
+
+
+ONES = np.array([~np.uint64(0)]).view(np.float64)[0]
+
+
+@pytest.mark.parametrize("precision,N", [(0, 100), (0, 1000), (3, 1000)])
+def test_nan_of_all_ones(ctx, precision, N):
+    import fpde_hpc_gb300 as fp
+    A, B, R, u0, alpha, tau, Da, w, rng = _problem(N, 3)
+    u0 = u0.copy()
+    u0.view(np.uint64)[N // 2] = ~np.uint64(0)
+    line = fp.Line(ctx, N, alpha, tau, Da, A, B, R, u0, 3, precision=precision)
+    line.run(3)
+    u = line.state()
+    line.close()
+    assert np.isnan(u[1:N]).all()
+
+
+def test_nan_of_all_ones_richards(ctx):
+    import fpde_hpc_gb300 as fp
+    N, steps = 300, 2
+    c = _case(N, steps, False)
+    u0 = c["u0"].copy()
+    u0.view(np.uint64)[N // 2] = ~np.uint64(0)
+    rich = dict(k_form=1, k_sat=2e-6, Z=c["Z"], dL=c["dL"], evaporation=c["E"])
+    line = fp.Line(ctx, N, c["alpha"], c["tau"], c["Da"], None, None, None, u0, steps, right=(0, c["u0"][-1]),
+                   richards=rich)
+    line.run(steps)
+    u = line.state()
+    line.close()
+    assert np.isnan(u[1:N]).all()
 
 
 def test_richards_state_written_between_runs(ctx):
