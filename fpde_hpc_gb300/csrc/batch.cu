@@ -468,6 +468,7 @@ int fpde_batch_destroy(fpde_batch *b)
         cudaStreamSynchronize(b->ctx->stream);
     }
     b->graphs.clear();
+    if (b->x7) b->ring = b->cfar = nullptr;                            // parts of the slices' allocation
     for (double *p : {b->ga, b->g, b->al, b->lane, b->warp, b->cmap, b->agg, b->uN, b->KF, b->CB, b->U, b->U0, b->Y, b->D,
                       b->part, b->wall, b->ring, b->cfar, b->wlag, b->Sn})
         dev_free(p);
@@ -690,17 +691,31 @@ int fpde_batch_create(fpde_ctx *ctx, const fpde_column_desc *cols, int n_cols, i
                 dev_alloc((void **)&b->cta_col, cta_col.size() * sizeof(int)) ||
                 (any_restrict && dev_alloc((void **)&b->col_lag, (size_t)n_cols * sizeof(int)));
     if (!fail && want7) {
-        b->x7 = hist7_alloc(ctx->stream, &b->h7, &b->plan7, tot, max_steps, n_cols) == FPDE_OK;
-        if (!b->x7) clear_error();                                     // FP64 rows instead (8 bytes against 14)
+        rc = dev_alloc((void **)&b->part, tb);
+        if (!rc) rc = dev_alloc((void **)&b->wlag, hwl.size() * sizeof(double));
+        if (!rc) rc = dev_alloc((void **)&b->wcol, hwcol.size() * sizeof(int));
+        if (!rc) rc = hist7_alloc(ctx->stream, &b->h7, &b->plan7, tot, tot, max_steps, n_cols, 1);
+        if (rc && rc != FPDE_ERR_NOMEM) {
+            std::string keep = fpde_last_error_string();
+            fpde_batch_destroy(b);
+            return set_error(rc, "%s", keep.c_str());
+        }
+        b->x7 = rc == FPDE_OK;
+        b->ring = b->h7.ring;
+        b->cfar = b->h7.far;
+        clear_error();
+        if (!b->x7) {                                                  // FP64 rows instead (8 bytes against 14)
+            dev_free(b->part);
+            dev_free(b->wlag);
+            dev_free(b->wcol);
+            b->part = b->wlag = nullptr;
+            b->wcol = nullptr;
+        }
     }
-    if (!fail && b->x7) {
-        fail = dev_alloc((void **)&b->ring, (size_t)64 * tb) || dev_alloc((void **)&b->cfar, (size_t)64 * tb) ||
-               dev_alloc((void **)&b->part, tb) || dev_alloc((void **)&b->wlag, hwl.size() * sizeof(double)) ||
-               dev_alloc((void **)&b->wcol, hwcol.size() * sizeof(int));
-    } else if (!fail && !split) {
+    if (!fail && !b->x7 && !split) {
         fail = dev_alloc((void **)&b->D, (size_t)max_steps * tb) || dev_alloc((void **)&b->part, (size_t)KS_MAX * tb) ||
                dev_alloc((void **)&b->wall, hw.size() * sizeof(double));
-    } else if (!fail) {
+    } else if (!fail && split) {
         b->ld16 = ((int64_t)max_steps + 63) / 64 * 64;
         b->ldp = b->ld16 / 64;
         const int64_t wrows = (int64_t)n_cols * 64;

@@ -1653,6 +1653,7 @@ int fpde_line_destroy(fpde_line *L)
     }
     L->graphs.clear();
     for (cudaEvent_t e : L->probe_ev) cudaEventDestroy(e);
+    if (L->x7) L->ring = L->cfar = nullptr;    // parts of the slices' allocation
     dev_free(L->cflag);
     dev_free(L->seq);
     dev_free(L->sclane);
@@ -2028,20 +2029,9 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
                 (spec && (dev_alloc((void **)&L->sclane, hsl.size() * sizeof(double)) ||
                            dev_alloc((void **)&L->scwarp, hsw.size() * sizeof(double)))) ||
                 dev_alloc((void **)&L->barrier, 2 * sizeof(unsigned));
-    if (!fail && b64 && L->max_steps > BLK && slices7_hold(wlag.data(), L->max_steps - 1)) {
-        // the far history in bf16 slices on the tensor cores; where they do not fit (14 bytes per node and
-        // step against 8) or the weights rule them out, FP64 rows and k_far64
-        L->x7 = hist7_alloc(ctx->stream, &L->h7, &L->plan7, N + 1, L->max_steps, 1) == FPDE_OK;
-        if (!L->x7) clear_error();
-    }
-    if (!fail && !L->split) {
-        fail = (L->x7 ? dev_alloc((void **)&L->ring, (size_t)BLK * L->P * sizeof(double))
-                      : dev_alloc((void **)&L->D, (size_t)L->max_steps * L->P * sizeof(double))) ||
-               (b64 ? dev_alloc((void **)&L->cfar, (size_t)(L->x7 ? FAR_MAX_SPLITS : 1) * BLK * L->P * sizeof(double)) ||
-                          dev_alloc((void **)&L->wlag, LW * sizeof(double)) || dev_alloc((void **)&L->cub, nb) ||
-                          dev_alloc((void **)&L->cu, nb) || dev_alloc((void **)&L->ccar, 4 * gb)
-                    : dev_alloc((void **)&L->part, (size_t)KS_MAX * L->P * sizeof(double)));
-    }
+    if (!fail && b64)
+        fail = dev_alloc((void **)&L->wlag, LW * sizeof(double)) || dev_alloc((void **)&L->cub, nb) ||
+               dev_alloc((void **)&L->cu, nb) || dev_alloc((void **)&L->ccar, 4 * gb);
     if (!fail && L->x3) {
         L->rows16 = (N + 1 + 127) / 128 * 128;
         L->ld16 = ((int64_t)L->max_steps + 63) / 64 * 64;
@@ -2103,6 +2093,24 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
                dev_alloc((void **)&L->sc3, nb) || dev_alloc((void **)&L->sngf, (size_t)N * sizeof(float2));
     if (!fail && spec && d.theta != 0.0)
         fail = dev_alloc((void **)&L->sxa, nb) || dev_alloc((void **)&L->sxb, nb);
+    if (!fail && b64 && L->max_steps > BLK && slices7_hold(wlag.data(), L->max_steps - 1)) {
+        // the far history in bf16 slices on the tensor cores; where they do not fit (14 bytes per node and
+        // step against 8) or the weights rule them out, FP64 rows and k_far64
+        rc = hist7_alloc(ctx->stream, &L->h7, &L->plan7, N + 1, L->P, L->max_steps, 1, FAR_MAX_SPLITS);
+        if (rc && rc != FPDE_ERR_NOMEM) {
+            std::string keep = fpde_last_error_string();
+            fpde_line_destroy(L);
+            return set_error(rc, "%s", keep.c_str());
+        }
+        L->x7 = rc == FPDE_OK;
+        L->ring = L->h7.ring;
+        L->cfar = L->h7.far;
+        clear_error();
+    }
+    if (!fail && !split && !L->x7)
+        fail = dev_alloc((void **)&L->D, (size_t)L->max_steps * L->P * sizeof(double)) ||
+               (b64 ? dev_alloc((void **)&L->cfar, (size_t)BLK * L->P * sizeof(double))
+                    : dev_alloc((void **)&L->part, (size_t)KS_MAX * L->P * sizeof(double)));
     if (fail) {
         std::string keep = fpde_last_error_string();
         fpde_line_destroy(L);

@@ -1411,6 +1411,7 @@ int fpde_lod3d_destroy(fpde_lod3d *L)
         cudaStreamSynchronize(L->ctx->stream);
     }
     L->graphs.clear();
+    if (L->x7) L->ring = L->cfar = nullptr;    // parts of the slices' allocation
     hist7_free(&L->h7);
     dev_free(L->ringf);
     dev_free(L->wff);
@@ -1566,28 +1567,7 @@ int fpde_lod3d_create(fpde_ctx *ctx, const fpde_lod3d_desc *desc, const double *
     if (!fail && L->series) {                                      // two increment rows and the moments
         fail = dev_alloc((void **)&L->D, 2 * pbytes) || dev_alloc((void **)&L->part, pbytes) ||
                dev_alloc((void **)&L->H, (size_t)L->series * pbytes);
-    } else if (!fail && !L->split) {
-        // blocks of 64 steps, the older history in bf16 slices on the tensor cores, for the passes with
-        // constant coefficients (space-fractional solves stop at a threshold, so their iterates would move
-        // with the sums' rounding); rows of FP64 where the slices do not fit (14 bytes per node and step
-        // against 8) or the weights rule them out
-        const int64_t LW = L->max_steps + 64 + 1;
-        if (!rich && !sfd && !vart && d.max_steps > 64) {
-            wlag.assign(LW, 0.0);
-            for (int64_t j = 1; j < LW; ++j) wlag[j] = wlag_at(j);
-        }
-        if (!wlag.empty() && slices7_hold(wlag.data(), L->max_steps - 1)) {
-            L->x7 = hist7_alloc(ctx->stream, &L->h7, &L->plan7, L->G, d.max_steps, 1) == FPDE_OK;
-            if (!L->x7) clear_error();
-        }
-        if (L->x7) {
-            fail = dev_alloc((void **)&L->ring, 64 * pbytes) || dev_alloc((void **)&L->cfar, 64 * pbytes) ||
-                   dev_alloc((void **)&L->part, pbytes) || dev_alloc((void **)&L->wlag, LW * sizeof(double));
-        } else {
-            fail = dev_alloc((void **)&L->D, (size_t)L->max_steps * pbytes) ||
-                   dev_alloc((void **)&L->part, (size_t)KS_MAX * pbytes);
-        }
-    } else if (!fail) {
+    } else if (!fail && L->split) {
         L->rows16 = (L->G + 127) / 128 * 128;
         L->ld16 = ((int64_t)L->max_steps + 63) / 64 * 64;
         L->ldp = L->ld16 / 64;
@@ -1896,6 +1876,38 @@ int fpde_lod3d_create(fpde_ctx *ctx, const fpde_lod3d_desc *desc, const double *
                 L->segs[pass] = SG;
                 L->segcap[pass] = SL;
             }
+        }
+    }
+    if (!fail && !L->series && !L->split) {
+        // blocks of 64 steps, the older history in bf16 slices on the tensor cores, for the passes with
+        // constant coefficients (space-fractional solves stop at a threshold, so their iterates would move
+        // with the sums' rounding); rows of FP64 where the slices do not fit (14 bytes per node and step
+        // against 8) or the weights rule them out
+        const int64_t LW = L->max_steps + 64 + 1;
+        if (!rich && !sfd && !vart && d.max_steps > 64) {
+            wlag.assign(LW, 0.0);
+            for (int64_t j = 1; j < LW; ++j) wlag[j] = wlag_at(j);
+        }
+        if (!wlag.empty() && slices7_hold(wlag.data(), L->max_steps - 1)) {
+            rc = dev_alloc((void **)&L->part, pbytes);
+            if (!rc) rc = dev_alloc((void **)&L->wlag, LW * sizeof(double));
+            if (!rc) rc = hist7_alloc(st, &L->h7, &L->plan7, L->G, L->P, d.max_steps, 1, 1);
+            if (rc && rc != FPDE_ERR_NOMEM) {
+                std::string keep = fpde_last_error_string();
+                fpde_lod3d_destroy(L);
+                return set_error(rc, "%s", keep.c_str());
+            }
+            L->x7 = rc == FPDE_OK;
+            L->ring = L->h7.ring;
+            L->cfar = L->h7.far;
+            clear_error();
+        }
+        if (!L->x7) {
+            dev_free(L->part);
+            dev_free(L->wlag);
+            L->part = L->wlag = nullptr;
+            fail = dev_alloc((void **)&L->D, (size_t)L->max_steps * pbytes) ||
+                   dev_alloc((void **)&L->part, (size_t)KS_MAX * pbytes);
         }
     }
     if (fail) {

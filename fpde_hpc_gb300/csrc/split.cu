@@ -474,7 +474,7 @@ bool slices7_hold(const double *w, int64_t lags)
     return true;
 }
 
-int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles)
+int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int64_t P, int max_steps, int w_tiles, int far_parts)
 {
     h->rows = (nodes + 127) / 128 * 128;
     h->n_delta = (max_steps - 1) / 64;
@@ -493,8 +493,13 @@ int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_s
         at_w[q] = place(n_w * 128);
     }
     const size_t at_pA = place(n_a * sizeof(int16_t)), at_eA = place((size_t)h->rows * sizeof(int16_t)),
-                 at_eW = place((size_t)w_tiles * 64 * sizeof(int16_t)), at_sW = place(n_w * sizeof(float));
-    int rc = dev_alloc(&h->base, total) ? FPDE_ERR_NOMEM : FPDE_OK;
+                 at_eW = place((size_t)w_tiles * 64 * sizeof(int16_t)), at_sW = place(n_w * sizeof(float)),
+                 at_ring = place((size_t)64 * P * sizeof(double)),
+                 at_far = place((size_t)far_parts * 64 * P * sizeof(double));
+    size_t avail = 0, all = 0;
+    FPDE_CUDA(cudaMemGetInfo(&avail, &all));
+    if (total > avail / 2) return set_error(FPDE_ERR_NOMEM, "digit slices: %zu bytes of %zu free", total, avail);
+    int rc = dev_alloc(&h->base, total);
     if (!rc) {
         char *p0 = (char *)h->base;
         for (int q = 0; q < 7; ++q) {
@@ -505,6 +510,8 @@ int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_s
         h->eA = (int16_t *)(p0 + at_eA);
         h->eW = (int16_t *)(p0 + at_eW);
         h->sW = (float *)(p0 + at_sW);
+        h->ring = (double *)(p0 + at_ring);
+        h->far = (double *)(p0 + at_far);
     }
     if (!rc) {
         const void *a[7], *w[7];
@@ -516,7 +523,7 @@ int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_s
     // first blocks are converted
     if (!rc && (cudaMemsetAsync(h->pA, 0, (size_t)h->rows * h->n_delta * sizeof(int16_t), st) != cudaSuccess ||
                 cudaMemsetAsync(h->eA, 0, (size_t)h->rows * sizeof(int16_t), st) != cudaSuccess))
-        rc = FPDE_ERR_CUDA;
+        rc = set_error(FPDE_ERR_CUDA, "digit slices: clearing the exponents failed");
     if (rc) hist7_free(h);
     return rc;
 }

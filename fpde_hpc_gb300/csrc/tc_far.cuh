@@ -61,6 +61,7 @@ struct Hist7 {
     int16_t *pA = nullptr, *eA = nullptr;      // [n_delta][rows] exponents per (block, node); [rows] largest so far
     int16_t *eW = nullptr;                     // [w_tiles][64] largest exponent of the step's weights
     float *sW = nullptr;                       // [w_tiles][n_delta][64] 2^(exponent - eW)
+    double *ring = nullptr, *far = nullptr;    // the block's FP64 rows [64][P], far sums [far_parts][64][P]
     int64_t rows = 0;
     int n_delta = 0, w_tiles = 1;
 };
@@ -70,8 +71,11 @@ struct FarPlan7 {
     int64_t rows = 0;
     uint32_t idesc = 0;
 };
-// Allocate for `nodes` rows and max_steps columns (FPDE_ERR_NOMEM leaves nothing behind; clears on st), free.
-int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int max_steps, int w_tiles);
+// Allocate for `nodes` rows and max_steps columns, free. One allocation, made last by the creations, so that
+// FPDE_ERR_NOMEM leaves nothing behind and the FP64 rows can take its place (other errors are errors). It is
+// also returned where the slices would take more than half of the free memory: they need 14 bytes per node and
+// step against the rows' 8, and a second object of the size has to fit as it does with rows.
+int hist7_alloc(cudaStream_t st, Hist7 *h, FarPlan7 *p, int64_t nodes, int64_t P, int max_steps, int w_tiles, int far_parts);
 void hist7_free(Hist7 *h);
 // Weight tiles from w[lag] (w_tiles rows of wstride values, lag < 64 n_delta + 64), once.
 int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t wstride);
