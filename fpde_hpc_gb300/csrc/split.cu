@@ -342,14 +342,14 @@ __global__ void __launch_bounds__(256) k_convert7(const double *__restrict__ row
     }
 }
 
-// grid (64 steps j, weight tiles), 64 threads: every distance's tile of step j, two passes (the largest
-// exponent first).
+// grid (weight tiles, 64 steps j), 64 threads: every distance's tile of step j, two passes (the largest
+// exponent first). The tiles, one per column of an ensemble, take the x axis: y ends at 65,535.
 __global__ void __launch_bounds__(64) k_wgen7(const double *__restrict__ wlag_all, int64_t wstride, Slices7 out,
                                               int n_delta, float *__restrict__ sW, int16_t *__restrict__ eW)
 {
     __shared__ unsigned long long red[2];
-    const int j = blockIdx.x, c = threadIdx.x;
-    const double *w = wlag_all + (int64_t)blockIdx.y * wstride;
+    const int j = blockIdx.y, c = threadIdx.x;
+    const double *w = wlag_all + (int64_t)blockIdx.x * wstride;
     auto tile_exp = [&](int d) {
         unsigned long long m = (unsigned long long)__double_as_longlong(fabs(w[64 * d + j - c]));
 #pragma unroll
@@ -364,16 +364,16 @@ __global__ void __launch_bounds__(64) k_wgen7(const double *__restrict__ wlag_al
     };
     int emax = PE7_ZERO;
     for (int d = 1; d <= n_delta; ++d) emax = max(emax, tile_exp(d));
-    if (c == 0) eW[(int64_t)blockIdx.y * 64 + j] = (int16_t)emax;
+    if (c == 0) eW[(int64_t)blockIdx.x * 64 + j] = (int16_t)emax;
     for (int d = 1; d <= n_delta; ++d) {
         const int pe = tile_exp(d);
         if (c == 0) {
             const int e = max(pe - emax, -126);
-            sW[((int64_t)blockIdx.y * n_delta + d - 1) * 64 + j] = __int_as_float((e + 127) << 23);
+            sW[((int64_t)blockIdx.x * n_delta + d - 1) * 64 + j] = __int_as_float((e + 127) << 23);
         }
         uint16_t s[7];
         digits7((unsigned long long)__double_as_longlong(w[64 * d + j - c]), pe, s);
-        const int64_t o = (((int64_t)2 * (d - 1) + c / 32) * (64 * gridDim.y) + 64 * blockIdx.y + j) * 32 + c % 32;
+        const int64_t o = (((int64_t)2 * (d - 1) + c / 32) * (64 * (int64_t)gridDim.x) + 64 * (int64_t)blockIdx.x + j) * 32 + c % 32;
 #pragma unroll
         for (int q = 0; q < 7; ++q) out.p[q][o] = s[q];
     }
@@ -538,7 +538,7 @@ int hist7_weights(cudaStream_t st, const Hist7 &h, const double *wlag, int64_t w
 {
     Slices7 o;
     for (int q = 0; q < 7; ++q) o.p[q] = h.w[q];
-    k_wgen7<<<dim3(64, (unsigned)h.w_tiles), 64, 0, st>>>(wlag, wstride, o, h.n_delta, h.sW, h.eW);
+    k_wgen7<<<dim3((unsigned)h.w_tiles, 64), 64, 0, st>>>(wlag, wstride, o, h.n_delta, h.sW, h.eW);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }
