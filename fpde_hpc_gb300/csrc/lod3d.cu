@@ -190,6 +190,7 @@ struct LodStageArgs {
     const double *al;                     // [tiles][F][GN][32]
     unsigned *flags;
     int wave;                             // CTAs of one resident round over the SMs (role placement)
+    unsigned zero;                        // 0
 };
 
 template <bool TRANS, bool KP, int S>
@@ -216,13 +217,13 @@ __global__ void __launch_bounds__(128, 4) k_lod_pass_st(LodPassArgs p, LodStageA
     double *yb = sh + 2 * GD;                           // [F GN][YP], row q - 1
     const double *AL = sa.al + (size_t)tile * F * GD;
     if (threadIdx.x == 0) {
-        auto init = [](uint64_t *bar) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(st_smem_u32(bar)) : "memory");
+        auto init = [](uint64_t *bar, int n) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(st_smem_u32(bar)), "r"(n) : "memory");
         };
 #pragma unroll
-        for (int s = 0; s < S; ++s) { init(&full[s]); init(&used[s]); }
-        init(&ready[0]);
-        init(&ready[1]);
+        for (int s = 0; s < S; ++s) { init(&full[s], 1); init(&used[s], 32); }
+        init(&ready[0], 1);
+        init(&ready[1], 1);
         s_done = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -352,17 +353,16 @@ __global__ void __launch_bounds__(128, 4) k_lod_pass_st(LodPassArgs p, LodStageA
 #pragma unroll
         for (int t = 0; t < GN; ++t) { A[t] = sg[t * 32]; H[t] = hi[t * 32]; }
     };
-    // Give a group's buffers back. Its operands must be in registers by then: loads that are still
-    // queued behind the helpers' traffic would meet the next bulk copy (seen in the K and sN passes),
-    // so the warp votes on a value formed from all of them.
+    // Give a group's buffers back. Every lane's operands must be in registers by then: loads that are still
+    // queued behind the helpers' traffic would meet the next bulk copy (seen in the K and sN passes). So every
+    // lane arrives for its own loads, at an address that depends on their values (z & 0 with a 0 the compiler
+    // does not know): 128^3, 100 steps, 155.7 us a step on the split path; one arrival for the warp after a vote
+    // on z took 156.9, after a vote and a warp barrier 159.1.
     auto release = [&](int gi, const double (&A)[GN], const double (&H)[GN]) {
         unsigned z = 0;
 #pragma unroll
         for (int t = 0; t < GN; ++t) z ^= (unsigned)(__double2loint(A[t]) ^ __double2loint(H[t]));
-        asm volatile("{\n\t.reg .pred p, q;\n\t"
-                     "setp.eq.u32 p, %0, 1;\n\t"
-                     "vote.sync.any.pred q, p, 0xffffffff;\n\t}\n" ::"r"(z) : "memory");
-        if (lane == 0) st_arrive(&used[gi % S]);
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(st_smem_u32(&used[gi % S]) + (z & sa.zero)) : "memory");
     };
     // forward: y_q = Bt[q+1] = gA y_{q-1} + g (-Om), y_0 = Bt[1] = g0
     double y = g0, A0[GN], H0[GN], A1[GN], H1[GN], R[GN / 2];
@@ -1172,6 +1172,7 @@ static int lod_launch_pass(fpde_lod3d *L, cudaStream_t st, int pass, int64_t n, 
         LodStageArgs sa;
         sa.AG = L->cA[pass]; sa.al = L->cal[pass]; sa.flags = L->ctx->d_flags;
         sa.wave = device_sm_count();
+        sa.zero = 0;
         if (L->sdepth[pass] == 8) st_launch<8>(st, a, sa, pass);
         else st_launch<4>(st, a, sa, pass);
     } else if (L->seglen[pass] > 0) {
