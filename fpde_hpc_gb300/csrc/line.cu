@@ -2256,6 +2256,16 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     return FPDE_OK;
 }
 
+// The Richards line's part of a reset: the previous state (increments) and the step's exchange slots, which a
+// step that gave up waiting leaves with values that a later launch would take for its own.
+static int line_reset_rich(fpde_line *L)
+{
+    cudaStream_t st = L->ctx->stream;
+    FPDE_CUDA(cudaMemcpyAsync(L->last, L->U, (L->N + 1) * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    if (L->rslots) FPDE_CUDA(cudaMemsetAsync(L->rslots, 0xFF, rich_slot_count((int)L->N) * sizeof(double), st));
+    return FPDE_OK;
+}
+
 int fpde_line_reset(fpde_line *L, const double *u0, int on_device)
 {
     clear_error();
@@ -2264,9 +2274,7 @@ int fpde_line_reset(fpde_line *L, const double *u0, int on_device)
     if (rc) return rc;
     FPDE_CUDA(cudaMemcpyAsync(L->U, u0, (L->N + 1) * sizeof(double),
                               on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, L->ctx->stream));
-    if (L->last)                               // the Richards line's previous state (increments)
-        FPDE_CUDA(cudaMemcpyAsync(L->last, L->U, (L->N + 1) * sizeof(double), cudaMemcpyDeviceToDevice,
-                                  L->ctx->stream));
+    if (L->last && (rc = line_reset_rich(L))) return rc;
     if (!on_device) FPDE_CUDA(cudaStreamSynchronize(L->ctx->stream));
     L->n_done = 0;
     return FPDE_OK;
@@ -2334,8 +2342,7 @@ int fpde_line_solve_host(fpde_line *L, const double *u0_host, int steps, double 
     if (rc) return rc;
     cudaStream_t st = L->ctx->stream;
     FPDE_CUDA(cudaMemcpyAsync(L->U, u0_host, (L->N + 1) * sizeof(double), cudaMemcpyHostToDevice, st));
-    if (L->last)
-        FPDE_CUDA(cudaMemcpyAsync(L->last, L->U, (L->N + 1) * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    if (L->last && (rc = line_reset_rich(L))) return rc;
     L->n_done = 0;
     if ((rc = fpde_line_run(L, steps))) return rc;
     FPDE_CUDA(cudaMemcpyAsync(u_out_host, L->U, (L->N + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
