@@ -74,7 +74,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
         : "memory");
     return ok != 0;
 }
-// Bounded wait on the phase with the given parity.
+// Bounded wait on the phase with the given parity. After a timeout (abort_s) no wait of the CTA waits again. The
+// epilogue warps go on with whatever they read, since TMEM loads, shuffles and votes take a warp as a whole and
+// a lane that left alone would keep the others waiting; one vote on abort_s per item drops their results.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned *flags, volatile int *abort_s)
 {
     if (mbar_try_wait(bar, parity)) return true;
@@ -300,11 +302,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         float hi[BN], lo[BN];
 #pragma unroll
         for (int j = 0; j < BN; ++j) { hi[j] = 0.f; lo[j] = 0.f; }
-        bool ok = true;
         for (int c = 0; c < nchunks; ++c) {
             const int buf = c & 1;
             const uint32_t use = (uint32_t)(c >> 1);
-            if (!mbar_wait(&tfull[buf], use & 1u, flags, abort_s)) { ok = false; break; }
+            mbar_wait(&tfull[buf], use & 1u, flags, abort_s);
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
             float v[BN];
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 lo[j] += e;
             }
         }
-        if (ok && row < rows && nchunks > 0) {
+        if (*abort_s == 0 && row < rows && nchunks > 0) {
             if (out_scale_ptr) out_scale *= *out_scale_ptr;
             double *out = C + (int64_t)split * ldc_split + row;
 #pragma unroll
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(Far3Cfg<NG>::THREADS, 1)
 #pragma unroll
                     for (int u = 0; u < NU; ++u) w_nx[u] = __ldg(pWl + 32 * u * ly.pw_row + (kt + 1) * ly.pw_kt);
                 }
-                if (!mbar_wait(&tfull[buf], use & 1u, flags, abort_s)) { ok = false; break; }
+                mbar_wait(&tfull[buf], use & 1u, flags, abort_s);
                 tc_fence_after();
                 // 2^pA * 2^pW: a product of powers of two, exact while it stays normal
                 const float sa1 = pow2f(e_cur);
@@ -651,6 +652,7 @@ __global__ void __launch_bounds__(Far3Cfg<NG>::THREADS, 1)
                     }
                 }
             }
+            ok = __all_sync(0xffffffffu, *abort_s == 0);
             if (ok && row < rows) {                   // float pairs: no FP64 work here
                 // column c of the item is step c % 64 of group NG gi + c / 64, i.e. at
                 // C + (NG gi) ldc_grp + c ldc_col (ldc_grp = 64 ldc_col)
@@ -881,7 +883,7 @@ __global__ void __launch_bounds__(F7_THREADS, 1) k_far_tc7(const __grid_constant
 #pragma unroll
             for (int j = 0; j < NP; ++j) hh[j] = mm[j] = ll[j] = 0ull;
             int e_nx = k0 < k1 ? (int)pAr[k0 * p.rows] : 0;
-            for (int kt = k0; kt < k1 && ok; ++kt, c += F7_LEV) {
+            for (int kt = k0; kt < k1; ++kt, c += F7_LEV) {
                 const float sa1 = pow2f(max(e_nx - eA, -127));
                 const f32x2 sa = pack2(sa1, sa1);
                 if (kt + 1 < k1) e_nx = pAr[(kt + 1) * p.rows];
@@ -891,7 +893,7 @@ __global__ void __launch_bounds__(F7_THREADS, 1) k_far_tc7(const __grid_constant
 #pragma unroll 1
                 for (int l = 0; l < F7_LEV; ++l) {
                     const int sl = (c + l) % F7_SLOTS;
-                    if (!mbar_wait(&sfull[sl], (uint32_t)((c + l) / F7_SLOTS) & 1u, p.flags, abort_s)) { ok = false; break; }
+                    mbar_wait(&sfull[sl], (uint32_t)((c + l) / F7_SLOTS) & 1u, p.flags, abort_s);
                     tc_fence_after();
                     const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(sl * BN + c0);
                     float v[F7_COLS];
@@ -916,6 +918,7 @@ __global__ void __launch_bounds__(F7_THREADS, 1) k_far_tc7(const __grid_constant
                     }
                 }
             }
+            ok = __all_sync(0xffffffffu, *abort_s == 0);
             if (ok) {
                 const int16_t *eW = p.eW + (int64_t)wt * BN + c0;
                 double *out = p.C + (int64_t)ks * p.ldc_split + row + (int64_t)c0 * p.ldc_col;
