@@ -1330,6 +1330,17 @@ static cudaEvent_t *probe_begin(fpde_line *L, int kind, int64_t n, double bytes,
     return &L->probe_ev[2 * k];
 }
 
+// A block's persistent solve of steps j .. j + nst - 1: far fold, near ring and state per step.
+static cudaEvent_t *probe_solve(fpde_line *L, int64_t n, int j, int nst, int splits, int64_t nodes)
+{
+    double bytes = 0.0, flops = 0.0;
+    for (int q = j; q < j + nst; ++q) {
+        bytes += 8.0 * nodes * (splits + q + 2);
+        flops += (double)nodes * (splits + 2.0 * q + 30.0);
+    }
+    return probe_begin(L, 2, n, bytes, flops, nst);
+}
+
 // Opt the speculative kernels in to their dynamic shared memory (the row ring) on this device.
 static cudaError_t spec_smem_attrs()
 {
@@ -1465,6 +1476,12 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
                 ++k;
             }
             if (j == 0 && splits > 0) {
+                // 28 bf16 products of seven slices, or one FP64 multiply-add, per row, step and node
+                const double rn = (double)(nb0 - t0) * nodes_hist;
+                ev = L->probe_every <= 0 ? nullptr
+                     : L->x7             ? probe_begin(L, 1, nb0, 14.0 * rn, 28.0 * 2.0 * BLK * rn)
+                                         : probe_begin(L, 0, nb0, 8.0 * rn, 2.0 * BLK * rn, BLK);
+                PROBE_REC(ev, 0);
                 if (L->x7) {
                     if ((rc = far7_launch(st, &L->plan7, L->h7, (int)nb0, L->cfar, (int64_t)BLK * L->P, L->P, splits,
                                           L->ctx->d_flags)))
@@ -1472,10 +1489,11 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
                 } else if ((rc = launch_far64(st, L->D, L->P, L->N, t0, nb0, L->wlag, L->cfar))) {
                     return rc;
                 }
+                PROBE_REC(ev, 1);
                 ++k;
             }
             const int nst = (int)std::min<int64_t>(BLK - j, n0 + steps - n);
-            ev = L->probe_every > 0 ? probe_begin(L, 2, n, 0.0, 0.0, nst) : nullptr;
+            ev = L->probe_every > 0 ? probe_solve(L, n, j, nst, splits, nodes_hist) : nullptr;
             PROBE_REC(ev, 0);
             if ((rc = line_launch_block(L, st, nb0, j, nst, splits, BLK, 0))) return rc;
             PROBE_REC(ev, 1);
@@ -1609,12 +1627,7 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
                 continue;
             }
             // the rest of this block (or of the requested range) in one persistent launch
-            double bytes = 0.0, flops = 0.0;
-            for (int q = j; q < j + nst; ++q) {                  // far fold + near ring + state
-                bytes += 8.0 * nodes_hist * (splits + q + 2);
-                flops += (double)nodes_hist * (splits + 2.0 * q + 30.0);
-            }
-            ev = L->probe_every > 0 ? probe_begin(L, 2, n, bytes, flops, nst) : nullptr;
+            ev = L->probe_every > 0 ? probe_solve(L, n, j, nst, splits, nodes_hist) : nullptr;
             PROBE_REC(ev, 0);
             if ((rc = line_launch_block(L, st, nb0, j, nst, splits, far_ld, far_row0))) return rc;
             PROBE_REC(ev, 1);

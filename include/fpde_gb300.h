@@ -390,12 +390,15 @@ int fpde_step_block(fpde_line *line, int *steps_run);
  * clock_gettime, opencl_cuda_base.cpp:708-716): with every > 0, later runs record CUDA
  * events inside the captured graph around the history-sum and solve kernels of every
  * `every`-th step and around every far-history contraction. fpde_line_probe_stats returns,
- * for the last run and one kind of kernel (0 FP64 history GEMV, 1 tensor-core far
- * contraction, 2 line solve), the summed event time (ms), the summed algorithmic bytes
- * (GEMV: 8 * rows * (N+1); contraction: 2 bytes per slice * rows * (N+1) of 16-bit history;
- * solve: 8 * (N+1) * (far splits + near rows + 2)), the summed algorithmic flops and the
- * number of time steps the probed launches cover (for the contraction: its launches). On
- * the split paths every block's solve launch is probed; on the FP64 path every `every`-th. */
+ * for the last run and one kind of kernel (0 sum over FP64 rows, 1 tensor-core far
+ * contraction, 2 line solve; 3 three-slice path, the contraction over a super-block's own blocks),
+ * the summed event time (ms), the summed algorithmic bytes (rows: 8 * rows * (N+1); contraction:
+ * 2 bytes per slice * rows * (N+1) of 16-bit history, three slices on the split path and seven on
+ * the FP64 one; block solve: 8 * (N+1) * (far splits + near rows + 2)), the summed algorithmic
+ * flops and the number of time steps the probed launches cover (for the contraction: its
+ * launches). Lines in 64-step blocks (the split paths and the FP64 rule) have every block's far
+ * sum and solve probed: FP64 lines as kind 1 where the history is in slices, else as kind 0, the
+ * block's 64 steps at once. The per-step FP64 form has every `every`-th step probed. */
 int fpde_line_set_probe(fpde_line *line, int every);
 int fpde_line_probe_stats(fpde_line *line, int kind, double *ms, double *bytes, double *flops,
                           int *count);
