@@ -225,6 +225,8 @@ class LineWorkload:
             self.desc = (f"distributed-order line N={self.p.N}, {self.p.steps} steps, w(a)=6a(1-a), 16-node "
                          "Gauss-Legendre, tau 1e-4, lognormal k (seed 3), 8-Gaussian H0 (seed 4) (config 3)")
         self.node_steps = self.p.node_steps
+        windowed = not self.do and self.restrict_eps > 0.0
+        self.rows_kernel = "k_far64 (FP64 rows of a window)" if windowed else "k_l1_partial (FP64 history GEMV)"
 
     def weights(self, n):
         import fpde_hpc_gb300 as fp
@@ -241,15 +243,14 @@ class LineWorkload:
                        restrict_eps=self.restrict_eps)
 
     def autotune(self, ctx, prec):
-        """fpde_line_autotune for this line (partition of the solve, far split depth, GEMV splits)."""
+        """fpde_line_autotune for this line (partition of the solve, far split depth, GEMV splits of the
+        per-step FP64 form)."""
         import fpde_hpc_gb300 as fp
         p = self.p
         A, B, R = p.coefs()
         if self.do:
             return fp.autotune_line(ctx, p.N, 0.5, p.tau, 1.0, A, B, R, p.u0, p.steps, precision=prec,
                                     lag_weights=self.weights(p.steps + 1), theta=1.0)
-        if prec == fp.FPDE_PREC_FP64:       # the plain method (a GEMV per step), not the 64-step blocks
-            return fp.LineTuning(gemv_splits=32)
         return fp.autotune_line(ctx, p.N, p.alpha, p.tau, p.Da, A, B, R, p.u0, p.steps, precision=prec)
 
     @property
@@ -851,8 +852,9 @@ def _timed(obj, u0_dev, steps, reps, stream):
 
 
 def _probe(line, u0_dev, steps, every):
-    """One probed solve: per-kind event sums (0 FP64 GEMV, 1 tensor-core far contraction over the
-    history older than a super-block, 2 solve, 3 contraction over the super-block's own blocks)."""
+    """One probed solve: per-kind event sums (0 sums over FP64 rows, 1 tensor-core far contraction (split:
+    over the history older than a super-block), 2 solve, 3 contraction over the super-block's own
+    blocks)."""
     import torch
     line.set_probe(every)
     line.reset(u0_dev)
@@ -888,6 +890,55 @@ def _kernel_entry(t, name, peak, peak_src, scale=1.0):
     return e
 
 
+def _sustained_tflops():
+    path = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    peaks = json.load(open(path)) if os.path.exists(path) else {}
+    if "bf16_tflops_sustained" in peaks:
+        return peaks["bf16_tflops_sustained"], ("of measured (MEASURED_PEAKS.json bf16_tflops_sustained: the kernel "
+                                                "runs inside a long solve)")
+    return 1700.0, "of fallback 1.7 PFLOP/s sustained"
+
+
+def fp64_line_roofline(tot, steps, hbm, hbm_src, rows_kernel="k_l1_partial (FP64 history GEMV)"):
+    """The FP64 line's far history from one probed solve: k_far_tc7 (28 bf16 products per FP64 one) where the
+    line runs on digit slices, else the sums over FP64 rows (k_far64 per block under restricted summing)."""
+    t = tot[1]
+    if t["count"] > 0 and t["ms"] > 0:
+        peak, src = _sustained_tflops()
+        tf = t["flops"] / (t["ms"] / 1e3) / 1e12
+        return {"kernel": "k_far_tc7 (tcgen05 far history of a 64-step block, seven bf16 slices)", "bound": "tensor",
+                "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak, "peak_source": src,
+                "flops_counted": "28 bf16 products x 2 x rows x K x 64 steps per launch", "traffic": None,
+                "launches": t["count"], "ms_per_launch": t["ms"] / t["count"], "est_ms_per_solve": t["ms"]}
+    e = _kernel_entry(tot[0], rows_kernel, hbm, hbm_src, steps / max(tot[0]["count"], 1))
+    if e:
+        e["fp64_fma_ceiling_gbs"] = 4800.0
+    return e
+
+
+def plain_fp64_line(wl, ctx, u0_dev, steps, stream, hbm, hbm_src):
+    """The plain FP64 method on the same line (one GEMV over all rows per step): its row splits chosen by
+    timing the first steps, then one probed solve."""
+    import fpde_hpc_gb300 as fp
+    head, best = min(steps, 2048), None
+    for ks in (16, 32, 64):
+        line = wl.build(ctx, fp.FPDE_PREC_FP64, fp.LineTuning(gemv_splits=ks))
+        _timed(line, u0_dev, head, 1, stream)
+        t = _timed(line, u0_dev, head, 1, stream)
+        line.close()
+        if best is None or t < best[0]:
+            best = (t, ks)
+    line = wl.build(ctx, fp.FPDE_PREC_FP64, fp.LineTuning(gemv_splits=best[1]))
+    line.set_probe(max(1, steps // 32))
+    _timed(line, u0_dev, steps, 1, stream)
+    ms = _timed(line, u0_dev, steps, 1, stream)
+    tot = {k: line.probe_stats(k) for k in (0, 1)}
+    line.close()
+    return {"value": wl.node_steps / (ms / 1e3), "ms_per_step": ms, "gemv_splits": best[1],
+            "note": "one GEMV over every earlier row per step (gemv_splits set), not the library's default",
+            "roofline": fp64_line_roofline(tot, steps, hbm, hbm_src)}
+
+
 def split_line_rooflines(tot, steps, nodes, rows, sbk, ms_solve, hbm, hbm_src):
     """Kernel records of the split (bf16x3) line from one probed solve.
 
@@ -902,11 +953,7 @@ def split_line_rooflines(tot, steps, nodes, rows, sbk, ms_solve, hbm, hbm_src):
     whole_solve: the benchmark's blocked byte model (history read once per block of B = 64 steps as
     hi+lo bf16 plus the near history and state; and the same at the super-block length) over the
     whole solve time."""
-    peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) if os.path.exists(
-        os.path.join(ROOT, "MEASURED_PEAKS.json")) else {}
-    tflops_peak = peaks.get("bf16_tflops_sustained", 1700.0)
-    tsrc = ("of measured (MEASURED_PEAKS.json bf16_tflops_sustained: the kernel runs inside a long solve)"
-            if "bf16_tflops_sustained" in peaks else "of fallback 1.7 PFLOP/s sustained")
+    tflops_peak, tsrc = _sustained_tflops()
     out = {}
     t1, t3, t2 = tot[1], tot[3], tot[2]
     if t1["count"] > 0 and t1["ms"] > 0:
@@ -1107,9 +1154,8 @@ def run_ours(args):
         tot = _probe(obj, u0_dev, steps, every)
         nodes = wl.p.N + 1
         if prec == 0:
-            k = _kernel_entry(tot[0], "k_l1_partial (FP64 history GEMV)", peak, peak_src,
-                              steps / max(tot[0]["count"], 1))
-            kernels = {"hist_gemv": k} if k else {}
+            k = fp64_line_roofline(tot, steps, peak, peak_src, wl.rows_kernel)
+            kernels = {("far_tc" if tot[1]["count"] else "hist_gemv"): k} if k else {}
         elif prec == fp.FPDE_PREC_SPLIT_BF16X3:
             sbk = tuning.far_super if (tuning is not None and tuning.far_super) else 4
             rows = (nodes + 127) // 128 * 128
@@ -1121,7 +1167,7 @@ def run_ours(args):
         out["kernels"] = kernels
         if "far_tc" in kernels:
             out["roofline"] = dict(kernels["far_tc"])
-            out["roofline_note"] = ("the tensor-core far contraction (the split path's HBM/tensor kernel); the "
+            out["roofline_note"] = ("the tensor-core far contraction (the path's HBM/tensor kernel); the "
                                     "block solve (kernels.solve) takes a comparable share but is bound by the "
                                     "FP64 pipe and its per-step chain, not by HBM or the tensor cores")
         elif "hist_gemv" in kernels:
@@ -1170,7 +1216,8 @@ def run_ours(args):
                            "traffic": None, "note": "algorithmic history bytes / whole solve time"}
 
     if prec != 0 and not args.no_fp64_arm:
-        # the plain FP64 kernel on the same workload: speed-up and accuracy of the split path
+        # the library's FP64 path on the same workload: speed-up and accuracy of the split path; for lines
+        # also the plain method (a GEMV per step)
         t64 = wl.autotune(ctx, fp.FPDE_PREC_FP64) if (is_line and not args.no_autotune) else None
         l64 = wl.build(ctx, fp.FPDE_PREC_FP64, t64) if is_line else wl.build(ctx, fp.FPDE_PREC_FP64)
         # both paths in eight pieces (untimed; the FP64 one is also its warm-up): max and RMS
@@ -1187,12 +1234,11 @@ def run_ours(args):
         out["fp64_kernel"] = {"value": wl.node_steps / (ms64 / 1e3), "ms_per_step": ms64}
         if is_line:
             tot64 = _probe(l64, u0_dev, steps, max(1, steps // 32))
-            r64 = _kernel_entry(tot64[0], "k_l1_partial (FP64 history GEMV)", peak, peak_src,
-                                steps / max(tot64[0]["count"], 1))
-            if r64:
-                r64["fp64_fma_ceiling_gbs"] = 4800.0
-            out["fp64_kernel"]["roofline"] = r64
+            out["fp64_kernel"]["roofline"] = fp64_line_roofline(tot64, steps, peak, peak_src, wl.rows_kernel)
         l64.close()
+        if is_line and not wl.do:            # (the distributed-order line's FP64 path is the plain method)
+            out["fp64_plain"] = plain_fp64_line(wl, ctx, u0_dev, steps, stream, peak, peak_src)
+            out["fp64_plain"]["split_speedup"] = out["fp64_plain"]["ms_per_step"] / ms
         out["split_vs_fp64"] = {"speedup": ms64 / ms, "max_rel_err": max([err] + [e["max_rel_err"] for e in cp_err]),
                                 "final_max_rel_err": err, "final_rms_rel_err": rms, "checkpoints": cp_err,
                                 "bound": 1e-7, "norm": "relative to max |u_fp64| at the same step"}
