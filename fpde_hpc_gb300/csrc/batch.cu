@@ -1,5 +1,5 @@
 // Ensemble of independent 1D Caputo columns (fpde_batch_*): many lines of different length,
-// order and coefficients advanced together, three kernels per time step for the whole ensemble.
+// order and coefficients advanced together, two or three kernels per time step for the whole ensemble.
 //
 // Layout in HBM: the columns' nodes are concatenated, column c occupying
 // [off_c, off_c + P_c) with P_c = N_c + 1 rounded up to 512, so that every CTA of the
@@ -13,7 +13,8 @@
 //                        every chunk of up to 1,024 nodes of a column from zero carries: the chunk's
 //                        solution, its last y and first u; the column's last chunk to finish solves
 //                        the column's chunk-level recurrences for every chunk's carries
-//   3. k_batch_join    : u = u^chunk + c_in KF + c_out CB, writing U and D_n
+//   3. k_batch_join    : u = u^chunk + c_in KF + c_out CB, writing U and D_n (columns of at most 1,024
+//                        intervals, all of them: done by the sweep)
 // FP64 where the digit slices and weight tiles fit and every column's weights allow them: step 1 becomes k_far_tc7 per 64-step block, k_near64_pre
 // per 8 steps and k_near64 per step, as for the 3D grids.
 // Split path (FPDE_PREC_SPLIT_BF16X3): step 1 becomes, per 64-step block, the exact
@@ -117,13 +118,24 @@ struct BatchSweepArgs {
     const double *part;
     int KS;
     int64_t pstride;
-    const double *U;
+    double *U;
     double *Y;                           // the chunk's zero-carry solution
     double *agg;                         // [chunks][2]: last y, first u; then the chunk's carries c_in, c_out
     const double *cmap;                  // [chunks][3]: product of gA, and KF, CB at the chunk's first node
     double *uN;                          // per column: U[N-1] before the step, then U[N] after it
     unsigned *count;                     // per column: chunks done in this step
+    const double *CB;                    // single-chunk columns: as in BatchJoinArgs
+    double *Drow;
+    float2 *Drowf;
 };
+
+// The right end (U1 :4685-4719) from y at node N-1 and the old U[N-1].
+__device__ __forceinline__ double batch_right_end(const ColInfo &c, double yN, double uNm1)
+{
+    if (c.rkind == FPDE_BC_DIRICHLET) return c.gN;
+    if (fabs(yN) > 1e-15) return (fabs(1.0 - c.AlN) > 1e-15) ? (yN + c.gN * c.dLN) / (1.0 - c.AlN) : uNm1;
+    return (fabs(1.0 - c.AlN) > 1e-15) ? 0.0 : uNm1;
+}
 
 // One warp: the chunk-level recurrences of a column (at most 17 chunks up to 16,384 intervals, one per
 // lane). agg[k] (last y, first u of chunk k from zero carries) becomes chunk k's carries.
@@ -152,11 +164,7 @@ __device__ void batch_carries(const ColInfo &c, int col, const BatchSweepArgs &p
         __stcg(ag + 2 * k + 1, v);
         y = fma(__ldg(cm + 3 * k), y, yl);
     }
-    double uN;                                           // right end (U1 :4685-4719) with the old U[N-1]
-    const double uNm1 = __ldcg(p.uN + col);
-    if (c.rkind == FPDE_BC_DIRICHLET) uN = c.gN;
-    else if (fabs(yN) > 1e-15) uN = (fabs(1.0 - c.AlN) > 1e-15) ? (yN + c.gN * c.dLN) / (1.0 - c.AlN) : uNm1;
-    else uN = (fabs(1.0 - c.AlN) > 1e-15) ? 0.0 : uNm1;
+    const double uN = batch_right_end(c, yN, __ldcg(p.uN + col));
     warp_scan_down(Q, V, lane);
     double u = __shfl_down_sync(FULL, fma(Q, uN, V), 1);          // u after this lane's chunks
     if (lane == 31) u = uN;
@@ -170,17 +178,21 @@ __device__ void batch_carries(const ColInfo &c, int col, const BatchSweepArgs &p
 
 // The scans' products are time-invariant and come from tables, so a scan level is one shuffle and one
 // multiply-add; carries enter by a second sweep (the same operation count as adding responses,
-// without their loads).
-__global__ void __launch_bounds__(CT, 6) k_batch_sweep(BatchSweepArgs p)
+// without their loads). ONE: every column is one chunk, which then needs no other's carries and finishes the
+// step itself, to the same bits as the join. Without that, ensembles of short columns took longer than with one
+// CTA per column (split, 400 steps, per step: 8 columns of 70 nodes 16.7 us against 13.9, 64 of 500 19.0
+// against 17.4); with it 12.4 and 12.7.
+template <bool ONE>
+__global__ void __launch_bounds__(CT, ONE ? 4 : 6) k_batch_sweep(BatchSweepArgs p)
 {
-    __shared__ double sX[2][CW];
+    __shared__ double sX[2][CW], s_end[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const ChunkInfo ch = p.chunks[blockIdx.x];
     const ColInfo *c = p.cols + ch.col;
     const int i0 = tid * CQ, cnt = min(max(ch.n - i0, 0), CQ);
     const int64_t q = ch.off + (cnt > 0 ? i0 : 0);
     const int64_t T = (int64_t)blockIdx.x * CT + tid;
-    double h[CQ], ga[CQ], al[CQ];
+    double h[CQ], ga[CQ], al[CQ], uo[ONE ? CQ : 1];
     {
         double u[CQ], g[CQ], s[CQ];
         load8(p.U + q, u);
@@ -200,7 +212,13 @@ __global__ void __launch_bounds__(CT, 6) k_batch_sweep(BatchSweepArgs p)
 #pragma unroll
         for (int k = 0; k < CQ; ++k) h[k] = g[k] * fma(lam, u[k], -s[k]);       // -g Om
         if (ch.idx == 0 && tid == 0) h[0] = c->g0;                             // Bt[1]
-        if (tid == 0 && ch.idx == c->nchunk - 1) p.uN[ch.col] = __ldcg(p.U + ch.off + ch.n - 1);
+        if constexpr (ONE) {
+#pragma unroll
+            for (int k = 0; k < CQ; ++k) uo[k] = u[k];
+            if (tid == 0) s_end[1] = __ldcg(p.U + ch.off + ch.n - 1);
+        } else if (tid == 0 && ch.idx == c->nchunk - 1) {
+            p.uN[ch.col] = __ldcg(p.U + ch.off + ch.n - 1);
+        }
     }
     const double *lp = p.lane + T, *wp = p.warp + (int64_t)blockIdx.x * (2 * CW);
     double pf[6];
@@ -226,7 +244,10 @@ __global__ void __launch_bounds__(CT, 6) k_batch_sweep(BatchSweepArgs p)
 #pragma unroll
     for (int k = 0; k < CQ; ++k)
         if (k < cnt) h[k] = x = fma(ga[k], x, h[k]);                           // y
-    if (cnt > 0 && i0 + cnt == ch.n) p.agg[2 * (int64_t)blockIdx.x] = x;
+    if (cnt > 0 && i0 + cnt == ch.n) {
+        if constexpr (ONE) s_end[0] = x;
+        else p.agg[2 * (int64_t)blockIdx.x] = x;
+    }
 #pragma unroll
     for (int k = 0; k < 6; ++k) pf[k] = __ldg(lp + (6 + k) * p.nlane);
     // backward: u_i = Al u_{i+1} + y_i
@@ -249,6 +270,43 @@ __global__ void __launch_bounds__(CT, 6) k_batch_sweep(BatchSweepArgs p)
 #pragma unroll
     for (int k = CQ - 1; k >= 0; --k)
         if (k < cnt) h[k] = x = fma(al[k], x, h[k]);                           // u^chunk
+    if constexpr (ONE) {
+        const double uN = batch_right_end(*c, s_end[0], s_end[1]);
+        double cb[CQ];
+        load8(p.CB + q, cb);
+#pragma unroll
+        for (int k = 0; k < CQ; ++k) {
+            h[k] = fma(uN, cb[k], h[k]);                                       // the new state, then its increment
+            uo[k] = h[k] - uo[k];
+        }
+        if (cnt == CQ) {
+#pragma unroll
+            for (int k = 0; k < CQ; k += 2) {
+                *reinterpret_cast<double2 *>(p.U + q + k) = make_double2(h[k], h[k + 1]);
+                *reinterpret_cast<double2 *>(p.Drow + q + k) = make_double2(uo[k], uo[k + 1]);
+                if (p.Drowf) {
+                    const float2 f0 = d2ff(uo[k]), f1 = d2ff(uo[k + 1]);
+                    *reinterpret_cast<float4 *>(p.Drowf + q + k) = make_float4(f0.x, f0.y, f1.x, f1.y);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < CQ; ++k)
+                if (k < cnt) {
+                    p.U[q + k] = h[k];
+                    p.Drow[q + k] = uo[k];
+                    if (p.Drowf) p.Drowf[q + k] = d2ff(uo[k]);
+                }
+        }
+        if (tid == 0) {
+            const int64_t e = ch.off + ch.n;
+            const double d = uN - p.U[e];
+            p.U[e] = uN;
+            p.Drow[e] = d;
+            if (p.Drowf) p.Drowf[e] = d2ff(d);
+        }
+        return;
+    }
     if (tid == 0) p.agg[2 * (int64_t)blockIdx.x + 1] = x;
     if (cnt == CQ) {
 #pragma unroll
@@ -443,7 +501,14 @@ static int batch_enqueue(fpde_batch *b, cudaStream_t st, int64_t n0, int steps, 
         sa.lane = b->lane; sa.warp = b->warp; sa.nlane = (int64_t)b->n_chunks * CT;
         sa.part = part; sa.KS = KS; sa.pstride = b->Ptot; sa.U = b->U; sa.Y = b->Y; sa.agg = b->agg; sa.cmap = b->cmap;
         sa.uN = b->uN; sa.count = b->count;
-        k_batch_sweep<<<b->n_chunks, CT, 0, st>>>(sa);
+        sa.CB = b->CB; sa.Drow = Drow; sa.Drowf = Drowf;
+        if (b->n_chunks == b->n_cols) {                              // every column is one chunk
+            k_batch_sweep<true><<<b->n_chunks, CT, 0, st>>>(sa);
+            FPDE_LAUNCHED(1);
+            ++k;
+            continue;
+        }
+        k_batch_sweep<false><<<b->n_chunks, CT, 0, st>>>(sa);
         FPDE_LAUNCHED(1);
         BatchJoinArgs ja;
         ja.cols = b->cols; ja.cta_col = b->cta_col; ja.KF = b->KF; ja.CB = b->CB;
