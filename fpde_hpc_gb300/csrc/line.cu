@@ -389,6 +389,7 @@ struct LineBlockArgs {
     double lam, g0, gN, dLN, AlN;
     int64_t n0;                           // global index of step j0
     int j0, nsteps, N, G, rkind, chunk;
+    int lag;                              // FP64 path: the oldest lag with a weight
 };
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const double *p)
@@ -496,10 +497,10 @@ __device__ __forceinline__ void far_add(const LineBlockArgs &p, int ht, int a, i
     }
 }
 
-// acc += sum_{r < rmax} w[j - r] D_r for this thread's nodes (rows of the row ring in global memory,
+// acc += sum_{r0 <= r < rmax} w[j - r] D_r for this thread's nodes (rows of the row ring in global memory,
 // two batches of rows in flight).
 template <class H, int SP>
-__device__ __forceinline__ void near_rows(const LineBlockArgs &p, int ht, int a, int b, int j, int rmax, H *acc)
+__device__ __forceinline__ void near_rows(const LineBlockArgs &p, int ht, int a, int b, int j, int r0, int rmax, H *acc)
 {
     using Row = typename H::Row;
     constexpr int RB = SP <= 2 ? 8 : (SP == 4 ? 4 : 2);  // rows per batch
@@ -525,8 +526,8 @@ __device__ __forceinline__ void near_rows(const LineBlockArgs &p, int ht, int a,
 #pragma unroll
         for (int q = 0; q < SP; ++q) acc[q].renorm();
     };
-    int r = 0;
-    if (RB <= rmax) load(va, 0);
+    int r = r0;
+    if (r + RB <= rmax) load(va, r);
     while (r + RB <= rmax) {                             // batch r in registers, the next one loading
         const bool more = r + 2 * RB <= rmax;
         if (more) load(vb, r + RB);
@@ -596,14 +597,15 @@ __device__ __forceinline__ void near_rows_smem(const LineBlockArgs &p, const typ
 }
 
 // acc += sum_{r < rmax} w[j - r] D_r: rows below rlo from the global row ring, the rest from the
-// shared-memory row ring.
+// shared-memory row ring. On the FP64 path rows before the step's window (restricted summing) are left out:
+// the row sums, not the chain, set the pace there.
 template <class H, int SP>
 __device__ __forceinline__ void near_rows_split(const LineBlockArgs &p, const typename H::Row *sR, int ht, int a, int b,
                                                 int j, int rmax, int rlo, H *acc)
 {
-    const int rg = min(rlo, rmax);
-    if (rg > 0) near_rows<H, SP>(p, ht, a, b, j, rg, acc);
-    if (rmax > rg) near_rows_smem<H, SP>(p, sR, ht, j, rg, rmax, acc);
+    const int rg = min(rlo, rmax), r0 = std::is_same<H, Near64>::value ? max(j - p.lag, 0) : 0;
+    if (rg > r0) near_rows<H, SP>(p, ht, a, b, j, r0, rg, acc);
+    if (rmax > max(rg, r0)) near_rows_smem<H, SP>(p, sR, ht, j, max(rg, r0), rmax, acc);
 }
 
 // v[n - 1] for a register array and a run-time n (1..SP) without indexing it dynamically,
@@ -653,8 +655,9 @@ __device__ __forceinline__ void history_store_scaled(int ht, int a, int b, const
 // forming the four carry dot products side by side: polled by the history warps, it took 2,400 of their
 // 9,900 cycles a step at 65,536 nodes (SP = 4), and the solver waited for them. With it, and the far
 // partials loaded ahead of the near sums instead of waited for (1,300 cycles), far product included: a
-// split step of 16,384 nodes with an explicit part 3.2 us (3.7 before), of 65,536 nodes 8.1 (8.5); an
-// FP64 step of 1,000 nodes 3.8 (4.2), of 65,536 nodes 15.6 (16.6).
+// split step of 16,384 nodes with an explicit part went from 3.7 to 3.2 us, of 65,536 nodes from 8.5 to 8.1, an
+// FP64 step of 1,000 nodes from 4.2 to 3.8 (since then, through the exchange and the far product: 3.1, 8.0, 3.6
+// and, FP64 at 65,536 nodes, 14.0).
 constexpr int BST = 3 * LTS;             // threads: solver, history and carry warpgroups
 // registers a thread: the solver keeps its nodes' state and coefficients; the shares add up to what the
 // block is launched with
@@ -1152,20 +1155,20 @@ __global__ void __launch_bounds__(BST, 1) k_line_block_spec(LineBlockArgs p)
 }
 
 // Far history of a block in FP64: C[j][i] = sum_{t0 <= t < nb0} w[nb0 + j - t] D_t[i] for the block's 64
-// steps at once, so that a row is read 4 times per 64 steps (once per FJ steps) instead of once per
-// step. CTA: 32 nodes (lanes) x FJ steps; its FW warps take consecutive slices of the rows and their
-// sums are added in order. A thread slides the FJ weights through registers (the next row needs
+// steps at once, t0 the window's start (lags up to `lag`) for the CTA's first step, so that a row is read 4
+// times per 64 steps (once per FJ steps) instead of once per step. CTA: 32 nodes (lanes) x FJ steps; its FW
+// warps take consecutive slices of the rows and their sums are added in order. A thread slides the FJ weights through registers (the next row needs
 // one new weight). Bound by the FP64 pipe: one multiply-add per row, step and node; the row
 // slices give a short line (1,000 nodes: 32 x 4 CTAs) 8 warps per SM, enough to fill it.
 constexpr int FJ = 16, FW = 8;
 
-__global__ void __launch_bounds__(32 * FW) k_far64(const double *__restrict__ D, int64_t P, int N, int t0, int nb0,
+__global__ void __launch_bounds__(32 * FW) k_far64(const double *__restrict__ D, int64_t P, int N, int lag, int nb0,
                                                    const double *__restrict__ wlag, double *__restrict__ C)
 {
     __shared__ double red[FW][FJ][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = (int64_t)blockIdx.x * 32 + lane;
-    const int j0 = blockIdx.y * FJ;
+    const int j0 = blockIdx.y * FJ, t0 = lag < nb0 + j0 ? min(nb0 + j0 - lag, nb0) : 0;
     const int per = (nb0 - t0 + FW - 1) / FW;
     const int ta = t0 + warp * per, tb = min(ta + per, nb0);
     const double *col = D + (i < N ? i : N - 1);
@@ -1202,10 +1205,10 @@ __global__ void __launch_bounds__(32 * FW) k_far64(const double *__restrict__ D,
     }
 }
 
-static int launch_far64(cudaStream_t st, const double *D, int64_t P, int64_t N, int64_t t0, int64_t nb0,
+static int launch_far64(cudaStream_t st, const double *D, int64_t P, int64_t N, int lag, int64_t nb0,
                         const double *wlag, double *C)
 {
-    k_far64<<<dim3((unsigned)((N + 31) / 32), BLK / FJ), 32 * FW, 0, st>>>(D, P, (int)N, (int)t0, (int)nb0, wlag, C);
+    k_far64<<<dim3((unsigned)((N + 31) / 32), BLK / FJ), 32 * FW, 0, st>>>(D, P, (int)N, lag, (int)nb0, wlag, C);
     FPDE_LAUNCHED(1);
     return FPDE_OK;
 }
@@ -1395,6 +1398,7 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     a.lam = L->lam; a.g0 = L->d.left_value; a.gN = L->d.right_value; a.dLN = L->d.dLN; a.AlN = L->AlN;
     a.n0 = nb0 + j0; a.j0 = j0; a.nsteps = nsteps; a.N = (int)L->N; a.G = L->G; a.rkind = L->d.right_kind;
     a.chunk = L->chunk;
+    a.lag = L->max_lag;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(L->G);
     cfg.blockDim = dim3(BST);
@@ -1418,18 +1422,43 @@ static int line_launch_block(fpde_line *L, cudaStream_t st, int64_t nb0, int j0,
     return FPDE_OK;
 }
 
+static double line_lag_weight(const fpde_line_desc &d, double kkk0, int64_t j)
+{
+    return d.lag_weights ? d.lag_weights[j] : d.Da * (kkk0 * l1_lag(d.alpha, j)) / d.tau;
+}
+
+// Restricted summing (time_summing :4117-4131, newest first): the history stops before the first lag whose
+// kb = w tau / Da falls below restrict_eps. The lags kept, INT_MAX for all.
+static int line_window(const fpde_line_desc &d)
+{
+    if (!(d.restrict_eps > 0.0) || d.max_steps <= 0) return INT_MAX;
+    const double kkk0 = d.lag_weights ? 0.0 : l1_interval_weight(d.alpha, 0.0, d.tau);
+    std::vector<double> kbl(d.max_steps);
+    for (int64_t j = 1; j <= d.max_steps; ++j) kbl[j - 1] = line_lag_weight(d, kkk0, j) * d.tau / d.Da;
+    int keep = 0;
+    fpde_restricted_lags(kbl.data(), d.max_steps, d.restrict_eps, &keep);
+    return keep < d.max_steps ? keep : INT_MAX;
+}
+
 // Whether an FP64 line runs in 64-step blocks: every one but
 //   - the Richards problem (its coefficients change with the state);
 //   - lines with an explicit part, whose speculative form rounds 3 to 6 times worse than the
 //     per-step form (20,000 intervals: 1.1e-9 against 1.9e-10);
 //   - a requested number of row splits of the per-step history sum, or a requested partition that
 //     only fits the per-step form's wider CTAs;
-//   - lines of over 1,024 nodes per SM.
-// N = 1,000, 1,000 steps: 24.3 ms per step by step (two launches a step), 4.6 ms in blocks; N = 65,536, 2,048
-// steps: 270 ms (the row sums' FP64 multiply-adds) against 245 ms.
+//   - lines of over 1,024 nodes per SM, and of over 512 under a window of 32 lags or more, where the block's
+//     row sums, whole rows for all of its 64 steps, cost the FP64 pipe more than the window's (150,000
+//     intervals, per step: 40 lags 35.8 us in blocks, 29.3 step by step; 20 lags 21.4 and 24.7; 65,536 intervals,
+//     40 lags 17.2 and 21.0).
+// N = 1,000, 1,000 steps: 24.5 ms step by step (two launches a step), 3.6 ms in blocks; N = 65,536, 2,048 steps:
+// 276 ms (the row sums' FP64 multiply-adds) against 28.6 ms.
 static bool line_blocked64(const fpde_ctx *ctx, const fpde_line_desc &d, const fpde_line_tuning *tu)
 {
     if (d.richards || d.theta != 0.0 || d.N > (int64_t)ctx->sm_count * LTS * LSEG) return false;
+    if (d.N > (int64_t)ctx->sm_count * LTS * (LSEG / 2)) {
+        const int lag = line_window(d);
+        if (lag >= 32 && lag != INT_MAX) return false;
+    }
     if (!tu) return true;
     if (tu->gemv_splits > 0) return false;
     if (tu->solve_sp <= 0 && tu->chunks <= 0) return true;
@@ -1486,7 +1515,7 @@ static int line_enqueue(fpde_line *L, cudaStream_t st, int64_t n0, int steps, in
                     if ((rc = far7_launch(st, &L->plan7, L->h7, (int)nb0, L->cfar, (int64_t)BLK * L->P, L->P, splits,
                                           L->ctx->d_flags)))
                         return rc;
-                } else if ((rc = launch_far64(st, L->D, L->P, L->N, t0, nb0, L->wlag, L->cfar))) {
+                } else if ((rc = launch_far64(st, L->D, L->P, L->N, L->max_lag, nb0, L->wlag, L->cfar))) {
                     return rc;
                 }
                 PROBE_REC(ev, 1);
@@ -1943,20 +1972,9 @@ int fpde_line_create(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A,
     const int64_t LW = L->max_steps + (int64_t)BLK * FAR_MAX_SUPER + 1;
     std::vector<double> wlag(LW, 0.0);
     for (int64_t j = 1; j < LW; ++j)
-        wlag[j] = d.lag_weights ? (j <= L->max_steps ? d.lag_weights[j] : 0.0)
-                                : d.Da * (L->kkk0 * l1_lag(d.alpha, j)) / d.tau;
-    // restricted summing (time_summing :4117-4131, newest first): the history stops before the
-    // first lag whose kb = w tau / Da falls below restrict_eps; later lags get weight 0
-    if (d.restrict_eps > 0.0) {
-        std::vector<double> kbl(L->max_steps);
-        for (int64_t j = 1; j <= L->max_steps; ++j) kbl[j - 1] = wlag[j] * d.tau / d.Da;
-        int keep = 0;
-        fpde_restricted_lags(kbl.data(), L->max_steps, d.restrict_eps, &keep);
-        if (keep < L->max_steps) {
-            L->max_lag = keep;
-            for (int64_t q = keep + 1; q < LW; ++q) wlag[q] = 0.0;
-        }
-    }
+        wlag[j] = j <= L->max_steps || !d.lag_weights ? line_lag_weight(d, L->kkk0, j) : 0.0;
+    L->max_lag = line_window(d);
+    for (int64_t q = (int64_t)L->max_lag + 1; q < LW; ++q) wlag[q] = 0.0;
     std::vector<double> wrev(L->max_steps + 1, 0.0);
     for (int64_t m = 0; m < L->max_steps; ++m) wrev[m] = wlag[L->max_steps - m];
     // Speculative block solve (split path): step n+1's right-hand side is affine in step n's
