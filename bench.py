@@ -872,9 +872,9 @@ def _probe(line, u0_dev, steps, every):
 #   k_far_tc3 (two weight groups per item, a 256-step super-block): reads per row x history
 #     column, writes (the float-pair partials) per launch and row;
 #   k_line_block_spec: bytes per node-step (64 steps x 65,537 nodes per launch).
-NCU_FAR = {"read_per_row_col": 514.54e6 / (65664 * 1280), "write_per_row": 108.04e6 / 65664,
+NCU_FAR = {"read_per_row_col": 514.94e6 / (65664 * 1280), "write_per_row": 108.05e6 / 65664,
            "source": "profiles/k_far_tc3_super_N65536_K1280.md"}
-NCU_SOLVE = {"per_node_step": (43.63e6 + 12.77e6) / (64 * 65537), "fp64_pipe_active": 0.5169,
+NCU_SOLVE = {"per_node_step": (43.63e6 + 12.24e6) / (64 * 65537), "fp64_pipe_active": 0.5179,
              "source": "profiles/k_line_block_spec_N65536_400steps.md"}
 
 

@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(128) k_lod_pass(LodPassArgs p)
 // cycles = 13 us per pass (K pass 17 us), next to 40 bytes per node (13 us at the measured copy
 // rate). Everything that shared the chain's warp held its operations back: forms with one and two
 // warps per tile took 33-37 us per pass with the FP64 pipe 31-35 % busy. Measured at 128^3, per pass:
-// K 32, _M 26, sN 29 us (segmented 66 us each); 61 x 47 x 90: 19, 11, 12 us (25 us each).
+// K 32, _M 26, sN 28 us (segmented 66 us each); 61 x 47 x 90: 19, 11, 12 us (25 us each).
 // The sN pass (TRANS) walks along the contiguous axis: a helper's consecutive loads share sectors
 // through L1, and its results go out 4 nodes x 8 lines per store instruction.
 constexpr int GN = 8;                     // nodes per group

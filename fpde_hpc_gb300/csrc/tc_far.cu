@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(Far3Cfg<NG>::THREADS, 1)
 // that read 6 KB each next to 168 KB of TMA writes: 6,600 cycles of shared memory at 128 B per cycle; the
 // tensor cores' own time is 3,600, the fold's 4,000 on the FP32 pipes and 3,000 of TMEM reads, HBM's 5,000.
 // Measured 10,600: the FP64 pipe would take 320,000. At 65,536 rows the product over one k-tile takes 50 us,
-// over ten 227 us. On the way: 8 epilogue warps of 32 columns, their conversions to FP64 with branches, and
+// over ten 231 us. On the way: 8 epilogue warps of 32 columns, their conversions to FP64 with branches, and
 // two stages of node-major slices took 102 and 302 us; the conversions alone 58 of each.
 // Operands come as 32-column half tiles (64-byte swizzle), contiguous in memory: three stages of the history
 // (it comes from HBM), two of the weights (they come from L2). 16-column stages of 32-byte swizzle let more

@@ -42,7 +42,18 @@ enum fpde_status {
 
 /* History storage / arithmetic of the L1 sum. */
 enum fpde_precision {
-    FPDE_PREC_FP64 = 0,        /* FP64 increments, FP64 FMA sum (the plain method) */
+    FPDE_PREC_FP64 = 0,        /* FP64 accuracy. Lines without an explicit part, 3D grids and ensembles run in
+                                  64-step blocks: the block's own increments in FP64 multiply-adds, the older
+                                  ones as seven bf16 digits each (62 bits from the largest of a node's 64
+                                  increments down, likewise the weights of 64 lags), 28 exact products on the
+                                  tensor cores and error-free sums. Against exact sums the rms error is that of
+                                  an FP64 multiply-add chain (1.01 times); an increment more than 2^10 below its
+                                  block's largest keeps fewer than 53 bits. 14 bytes per node and step, 8 as
+                                  FP64 rows. Rows (FP64 multiply-adds throughout) are kept where the digits
+                                  would take more than half of the free memory, where a weight is 0 (restricted
+                                  summing) or 64 neighbouring lag weights differ by more than 2^8 or any two by
+                                  2^40, and for Richards, space-fractional and variable-step runs; a line's
+                                  tuning.gemv_splits asks for them (the plain method, one sum per step) */
     FPDE_PREC_SPLIT_BF16 = 1,  /* far history as bf16 hi+lo on tensor cores, FP64 fold */
     FPDE_PREC_SPLIT_F16 = 2,   /* same with fp16 hi+lo (per-block power-of-two scaling) */
     FPDE_PREC_SPLIT_BF16X3 = 3 /* far history as three exact bf16 slices (8-bit integers with
@@ -346,7 +357,7 @@ typedef struct fpde_line_desc {
                              restrict_eps (time_summing :4117-4131): newest first, the history
                              stops before the first lag l whose kb = w[l]*tau/Da is below it;
                              0 keeps every lag. FPDE_PREC_FP64 and FPDE_PREC_SPLIT_BF16X3: the
-                             GEMV reads only the window's rows, the far contraction only the
+                             FP64 sums read only the window's rows, the far contraction only the
                              64-step blocks the window reaches. */
     const fpde_richards *richards; /* optional: the Richards problem - A, B, Rlap formed from the state
                              every step (those arguments of fpde_line_create may be NULL);
@@ -407,8 +418,8 @@ int fpde_line_probe_stats(fpde_line *line, int kind, double *ms, double *bytes, 
  * time candidate launch parameters on short runs and on the far contraction / FP64 history
  * sum at a history of min(max_steps, 2048) steps, and return the fastest in *out (pass it as
  * desc->tuning to fpde_line_create). Candidates: solve_sp x chunks (solve time per step of the
- * second 64-step block), far_splits 1..4, gemv_splits {k/2, k, 2k} around the built-in rule k,
- * and on the three-slice path far_super 1, 2, 4 (a whole run of min(max_steps, 4096) steps each).
+ * second 64-step block), far_splits 1..4, gemv_splits {k/2, k, 2k} around the built-in rule k where
+ * an FP64 line runs step by step (0 otherwise: 64-step blocks), and on the three-slice path far_super 1, 2, 4 (a whole run of min(max_steps, 4096) steps each).
  * Allocates and frees temporary device buffers; takes a fraction of a second to seconds. */
 int fpde_line_autotune(fpde_ctx *ctx, const fpde_line_desc *desc, const double *A, const double *B,
                        const double *Rlap, const double *u0, fpde_line_tuning *out);
