@@ -202,6 +202,22 @@ __global__ void k_append_ff(const double *__restrict__ u, double *__restrict__ l
     rowf[i] = d2ff(d);
 }
 
+__global__ void k_sum_partials(double *part, int64_t P, int KS)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P) return;
+    double s = part[i];
+    for (int q = 1; q < KS; ++q) s += part[(int64_t)q * P + i];
+    part[i] = s;
+}
+
+int launch_sum_partials(cudaStream_t st, double *part, int64_t P, int KS)
+{
+    k_sum_partials<<<(unsigned)((P + 127) / 128), 128, 0, st>>>(part, P, KS);
+    FPDE_LAUNCHED(1);
+    return FPDE_OK;
+}
+
 int launch_append_ff(cudaStream_t st, const double *u, double *last, double *row, float2 *rowf, int64_t nodes,
                      int64_t P)
 {

@@ -14,6 +14,8 @@ double l1_lag(double alpha, int64_t j);
 int launch_l1_partial(cudaStream_t st, const double *D, int64_t P, int n, const double *wt,
                       double *part, int KS);
 int choose_splits(int n, int64_t P);
+// part[0][i] += part[1][i] + ... in order, P doubles per row.
+int launch_sum_partials(cudaStream_t st, double *part, int64_t P, int KS);
 // row[i] = u[i] - last[i], last[i] = u[i] for i < nodes; row[i] = 0 up to P.
 int launch_append(cudaStream_t st, const double *u, double *last, double *row, int64_t nodes, int64_t P);
 // The same, also writing the increment row as float pairs (rowf, for the float-float near history).

@@ -159,7 +159,10 @@ __global__ void __launch_bounds__(128) k_lod_pass(LodPassArgs p)
 // The sN pass (TRANS) walks along the contiguous axis: a helper's consecutive loads share sectors
 // through L1, and its results go out 4 nodes x 8 lines per store instruction.
 constexpr int GN = 8;                     // nodes per group
-constexpr int ST_KS_MAX = 2;              // history partial rows of a staged K pass
+// History partial rows of a staged K pass; more are added by a launch of their own. Held to 2 instead, small grids
+// under long windows were slower than segmented passes (20^3, 1,000 lags: 71.8 us per step; segmented 61.6, now
+// 36.4; 300 lags 37.1, 49.8 and 28.5).
+constexpr int ST_KS_MAX = 2;
 constexpr int ST_PD = 8;                  // groups asked into L2 ahead of their copy
 
 __device__ __forceinline__ uint32_t st_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -1324,12 +1327,16 @@ static int lod_enqueue(fpde_lod3d *L, cudaStream_t st, int64_t n0, int steps, in
             const int64_t t0 = n > L->max_lag ? n - L->max_lag : 0;    // oldest row of the window
             if (n - t0 >= 1) {
                 KS = choose_splits((int)(n - t0), L->P);
-                if (L->sdepth[2] > 0) KS = std::min(KS, ST_KS_MAX);
                 const double *wt = L->vart ? L->wrows + n * L->wld     // variable steps: row n
                                            : L->wrev + (L->max_steps - n);     // wt[t] = w[n - t]
                 if ((rc = launch_l1_partial(st, L->D + t0 * L->P, L->P, (int)(n - t0), wt + t0, L->part, KS)))
                     return rc;
                 ++k;
+                if (L->sdepth[2] > 0 && KS > ST_KS_MAX) {
+                    if ((rc = launch_sum_partials(st, L->part, L->P, KS))) return rc;
+                    KS = 1;
+                    ++k;
+                }
                 if (L->salt) {                                           // C's own history, same weights
                     if ((rc = launch_l1_partial(st, L->DC + t0 * L->P, L->P, (int)(n - t0), wt + t0, L->partC, KS)))
                         return rc;

@@ -84,11 +84,12 @@ def test_windowed_ensemble(ctx):
 
 
 def test_windowed_grid(ctx):
-    """Also the per-step FP64 sum over more than 64 rows under the staged K pass."""
+    """Also the per-step FP64 sum over more than 64 rows under the staged K pass: two partial rows, which the pass
+    adds (100 lags), and three, which are added before it (150)."""
     import fpde_hpc_gb300 as fp
     import oracle
     from fpde_hpc_gb300 import problems
-    for tau, lags, steps in ((0.05, 5, 260), (0.5, 100, 200)):
+    for tau, lags, steps in ((0.05, 5, 260), (0.5, 100, 200), (0.5, 150, 220)):
         base = problems.config4(n=9, steps=steps)
         cA, cB, cR = base.coefs()
         Da, alpha = base.Da, base.alpha
